@@ -60,7 +60,7 @@ def listed():
              walkers=4096, burn=1),
         # many hierarchical models advanced together (bench.py's family, the shape its tuner
         # picks), means and final states read back
-        dict(name="hier_batch", kind="batch", members=128, burn=8, run=16, most=4096, rpt=512,
+        dict(name="hier_batch", kind="batch", members=48, burn=16, run=32, most=4096, rpt=512,
              wpi=64, chunk=8192, wpt=4),
         # moments and histograms of a large data matrix that already lies on the device
         dict(name="data_estimates", kind="data", n=(1 << 22) + 11, dim=6, bins=256),
@@ -111,8 +111,8 @@ def draw(rng):
         return dict(kind="robust", rows=_log(rng, 20000, min(1 << 20, 5.4e11 / (f * w))), features=f,
                     walkers=w, burn=1)
     if kind == "batch":
-        return dict(kind="batch", members=_log(rng, 2, 96), burn=rng.randint(1, 8),
-                    run=rng.randint(1, 12), most=rng.choice([256, 1024, 4096]),
+        return dict(kind="batch", members=_log(rng, 2, 48), burn=rng.randint(4, 16),
+                    run=rng.randint(4, 32), most=rng.choice([256, 1024, 4096]),
                     **rng.choice([dict(rpt=512, wpi=64, chunk=8192, wpt=4),
                                   dict(rpt=128, wpi=64, chunk=4096, wpt=1),
                                   dict(rpt=256, wpi=32, chunk=4096, wpt=4)]))
