@@ -203,6 +203,25 @@ struct bay_ctx {
         cudaFree(p);
     }
     void use() { cuda_check(cudaSetDevice(device), "cudaSetDevice"); }
+
+    // Workspace of the estimate kernels, kept between calls (at most 2.5 MB up to
+    // 155,648 dimensions, 16 bytes a dimension past that).  Every user runs on this context's
+    // stream under its lock; growing frees the old one, which waits for the device.
+    void* est_ws = nullptr;
+    size_t est_ws_bytes = 0;
+    void* est_workspace(uint32_t D, uint64_t W) {
+        const size_t need = bay::est_workspace(D, W);
+        if (need > est_ws_bytes) {
+            release(est_ws);
+            est_ws = nullptr;
+            est_ws_bytes = 0;
+            est_ws = alloc(need);
+            est_ws_bytes = need;
+            cuda_check(cudaMemsetAsync(est_ws, 0, bay::kEstTickets * sizeof(uint32_t), stream),
+                       "memset(tickets)");
+        }
+        return est_ws;
+    }
 };
 
 // ============================================================================ model
@@ -395,7 +414,6 @@ struct bay_sampler {
     unsigned int* t_ticket = nullptr;  // tiled form, row slices: [grid()] slice tickets
     float* means = nullptr;
     uint64_t means_cap = 0;
-    float* stage = nullptr;  // W*D floats: AoS staging
     double* stats = nullptr;  // 2*D doubles
     float* hist = nullptr;    // limits + pdf + ranks scratch
     uint32_t* counts = nullptr;
@@ -415,14 +433,6 @@ struct bay_sampler {
     uint32_t gemm_np = 0;                   // rows padded to a multiple of 64
     float* gemm_lay = nullptr;              // the kernel's layout of A and the aux values
     size_t smem = 0;                        // dynamic shared memory per CTA
-
-    // Dimension-major copy of the walker state (stage[d * W + w]) for the per-dimension
-    // estimate kernels (moments, limits, histogram), which read one dimension per CTA.
-    const float* dim_major() {
-        if (!stage) stage = (float*)ctx->alloc(sizeof(float) * (size_t)D * W);
-        cuda_check(bay::launch_aos_to_soa(xs, D, W, stage, ctx->stream), "transpose");
-        return stage;
-    }
 
     // A device-detected failure (a bounded wait that gave up) sets ctl->status.
     void check_status() {
@@ -1407,7 +1417,6 @@ int bay_sampler_release(bay_sampler* s) {
         c->release(s->part);
         c->release(s->stats);
         c->release(s->means);
-        c->release(s->stage);
         c->release(s->hist);
         c->release(s->counts);
         c->release(s->mix);
@@ -1625,15 +1634,15 @@ uint64_t read_accepted(bay_sampler* s) {
     return v;
 }
 
-// Bin counts of dimension-major values (dm[d * W + w]) into counts[d * bins + b]: the
+// Bin counts of point-major values (x[w * D + d]) into counts[d * bins + b]: the
 // IEEE-division kernel, or with BAY_HIST_COMPAT_FASTDIV the reference's expression under
 // -use_fast_math (device/bay_hist_fastdiv.cuh; one NVRTC module per bin count and
 // context, compiled on first use).
-void hist_count(bay_ctx* c, uint32_t flags, const float* dm, uint32_t D, uint64_t W,
+void hist_count(bay_ctx* c, uint32_t flags, const float* x, uint32_t D, uint64_t W,
                 uint32_t bins, const float* lim, uint32_t* counts) {
     if (D > 65535) fail(BAY_ERR_ARG, "histograms of at most 65535 dimensions");
     if (!(flags & BAY_HIST_COMPAT_FASTDIV)) {
-        cuda_check(bay::launch_hist_count(dm, D, W, bins, lim, counts, c->stream), "histogram");
+        cuda_check(bay::launch_hist_count(x, D, W, bins, lim, counts, c->stream), "histogram");
         return;
     }
     CUkernel k = nullptr;
@@ -1657,15 +1666,16 @@ void hist_count(bay_ctx* c, uint32_t flags, const float* dm, uint32_t D, uint64_
         }
         c->hist_fastdiv[bins] = std::make_pair(lib, k);
     }
-    const float* xp = dm;
+    const float* xp = x;
     unsigned int dd = D;
     unsigned long long ww = W;
     const float* lp = lim;
     unsigned int* cp = counts;
-    void* args[] = {&xp, &dd, &ww, &lp, &cp};
-    const unsigned gx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(64, (W + 255) / 256));
-    cu_check(g_cu.LaunchKernel((CUfunction)k, gx, D, 1, 256, 1, 1, 0, (CUstream)c->stream, args,
-                               nullptr),
+    bay::est_plan pl = bay::hist_plan_of(D, W, bins);
+    void* args[] = {&xp, &dd, &ww, &pl.gx, &pl.tile, &lp, &cp};
+    cu_check(g_cu.LaunchKernel((CUfunction)k, pl.gx * pl.gy, 1, 1, 256, 1, 1,
+                               (unsigned)(sizeof(uint32_t) * pl.tile * bins), (CUstream)c->stream,
+                               args, nullptr),
              "cuLaunchKernel(histogram, fast division)");
     bay::count_launches(1);
 }
@@ -1876,8 +1886,8 @@ static int moments_out(bay_sampler* s, double* out, int which) {
         std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
         s->ctx->use();
         s->require_positions();
-        cuda_check(bay::launch_moments(s->dim_major(), s->D, s->W, s->stats, s->stats + s->D,
-                                       s->ctx->stream),
+        cuda_check(bay::launch_moments(s->xs, s->D, s->W, s->stats, which ? s->stats + s->D : nullptr,
+                                       s->ctx->est_workspace(s->D, s->W), s->ctx->stream),
                    "moments");
         cuda_check(cudaMemcpyAsync(out, s->stats + (which ? s->D : 0), sizeof(double) * s->D,
                                    cudaMemcpyDefault, s->ctx->stream),
@@ -1944,17 +1954,17 @@ int bay_histogram(bay_sampler* s, uint32_t cycles, uint32_t bins, uint32_t flags
                 cnt = (cnt + B - 1) / B;
             } while (cnt > 1);
         }
-        const float* dm = s->dim_major();
-        cuda_check(bay::launch_minmax(dm, s->D, s->W, zero, d_lim, c->stream), "minmax");
-        cuda_check(bay::launch_fill_u32(s->counts, (flags & BAY_HIST_COMPAT_START1) ? 1u : 0u,
-                                        (uint64_t)bins * s->D, c->stream),
-                   "fill");
-        hist_count(c, flags, dm, s->D, s->W, bins, d_lim, s->counts);
+        cuda_check(bay::launch_limits(s->xs, s->D, s->W, zero, d_lim, s->counts,
+                                      (uint64_t)bins * s->D,
+                                      (flags & BAY_HIST_COMPAT_START1) ? 1u : 0u,
+                                      c->est_workspace(s->D, s->W), c->stream),
+                   "limits");
+        hist_count(c, flags, s->xs, s->D, s->W, bins, d_lim, s->counts);
         if (cycles > 1) {
             s->set_a_beta(s->a, 1.0f);
             for (uint32_t i = 1; i < cycles; ++i) {
                 s->steps(false, 1);
-                hist_count(c, flags, s->dim_major(), s->D, s->W, bins, d_lim, s->counts);
+                hist_count(c, flags, s->xs, s->D, s->W, bins, d_lim, s->counts);
             }
             s->iteration_counter += cycles - 1;
         }

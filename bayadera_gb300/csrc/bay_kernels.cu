@@ -1,7 +1,7 @@
-// bay_kernels.cu -- nvcc-compiled kernels of the stretch-move engine: walker init,
-// SoA<->AoS layout changes, FP64 moments, the integer histogram with its bitonic
-// ranks, acor, and the device-resident control block.  The per-model fused stretch
-// kernels are in device/bay_stretch.cuh (NVRTC).
+// bay_kernels.cu -- nvcc-compiled kernels of the stretch-move engine: walker init, the GEMM
+// forms' matrix layouts, per-step means, acor, and the device-resident control block.  The
+// estimates are in bay_estimates.cu, the per-model fused stretch kernels in
+// device/bay_stretch.cuh (NVRTC).
 #include <atomic>
 
 #include "bay_kernels.cuh"
@@ -129,150 +129,6 @@ __global__ void init_normal(float* xs, uint32_t D, uint64_t W, uint32_t seed, fl
     }
 }
 
-// 32x32 tiled transposes between SoA (D rows of W) and AoS (W rows of D).
-__global__ void soa_to_aos(const float* xs, uint32_t D, uint64_t W, uint64_t w0, uint64_t nw,
-                           float* out) {
-    __shared__ float tile[32][33];
-    const uint64_t wb = w0 + (uint64_t)blockIdx.x * 32;
-    const uint32_t db = blockIdx.y * 32;
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const uint32_t d = db + r;
-        const uint64_t w = wb + threadIdx.x;
-        if (d < D && w < w0 + nw) tile[r][threadIdx.x] = xs[(uint64_t)d * W + w];
-    }
-    __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const uint64_t w = wb + r;
-        const uint32_t d = db + threadIdx.x;
-        if (d < D && w < w0 + nw) out[(w - w0) * D + d] = tile[threadIdx.x][r];
-    }
-}
-
-__global__ void aos_to_soa(const float* in, uint32_t D, uint64_t W, float* xs) {
-    __shared__ float tile[32][33];
-    const uint64_t wb = (uint64_t)blockIdx.x * 32;
-    const uint32_t db = blockIdx.y * 32;
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const uint64_t w = wb + r;
-        const uint32_t d = db + threadIdx.x;
-        if (d < D && w < W) tile[r][threadIdx.x] = in[w * D + d];
-    }
-    __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const uint32_t d = db + r;
-        const uint64_t w = wb + threadIdx.x;
-        if (d < D && w < W) xs[(uint64_t)d * W + w] = tile[threadIdx.x][r];
-    }
-}
-
-// One CTA per dim: FP64 mean, then FP64 sum of squared deviations (population variance).
-__global__ void moments(const float* xs, uint32_t D, uint64_t W, double* mean, double* var) {
-    __shared__ double red[33];
-    const uint32_t d = blockIdx.x;
-    const float* row = xs + (uint64_t)d * W;
-    double s = 0.0;
-    for (uint64_t w = threadIdx.x; w < W; w += blockDim.x) s += (double)row[w];
-    const double mu = block_sum_d(s, red) / (double)W;
-    double q = 0.0;
-    for (uint64_t w = threadIdx.x; w < W; w += blockDim.x) {
-        const double t = (double)row[w] - mu;
-        q += t * t;
-    }
-    const double v = block_sum_d(q, red) / (double)W;
-    if (threadIdx.x == 0) {
-        if (mean) mean[d] = mu;
-        if (var) var[d] = v;
-    }
-}
-
-__global__ void minmax(const float* xs, uint32_t D, uint64_t W, int zero_fold, float* limits) {
-    __shared__ float smn[32], smx[32];
-    const uint32_t d = blockIdx.x;
-    const float* row = xs + (uint64_t)d * W;
-    float mn = row[0], mx = row[0];
-    for (uint64_t w = threadIdx.x; w < W; w += blockDim.x) {
-        mn = fminf(mn, row[w]);
-        mx = fmaxf(mx, row[w]);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        mn = fminf(mn, __shfl_down_sync(FULL, mn, o));
-        mx = fmaxf(mx, __shfl_down_sync(FULL, mx, o));
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-        smn[warp] = mn;
-        smx[warp] = mx;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-            mn = fminf(mn, smn[w]);
-            mx = fmaxf(mx, smx[w]);
-        }
-        if (zero_fold) {
-            mn = fminf(mn, 0.0f);
-            mx = fmaxf(mx, 0.0f);
-        }
-        limits[2 * d] = mn;
-        limits[2 * d + 1] = mx;
-    }
-}
-
-// histogram (nvidia-gtx-estimate.cu:5-32): bin = (uint)((x - lo)/(hi - lo) * bins) with
-// IEEE division and the saturating float->uint conversion, clamped to bins - 1.
-// Shared-memory counts per CTA, one global atomic per non-empty bin.
-__global__ void hist_count(const float* xs, uint32_t D, uint64_t W, uint32_t bins,
-                           const float* limits, uint32_t* counts) {
-    extern __shared__ uint32_t h[];
-    const uint32_t d = blockIdx.y;
-    for (uint32_t b = threadIdx.x; b < bins; b += blockDim.x) h[b] = 0;
-    __syncthreads();
-    const float lo = limits[2 * d], hi = limits[2 * d + 1];
-    const float range = __fsub_rn(hi, lo);
-    const float fb = (float)bins;
-    const float* row = xs + (uint64_t)d * W;
-    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < W;
-         w += (uint64_t)gridDim.x * blockDim.x) {
-        const float v = __fmul_rn(__fdiv_rn(__fsub_rn(row[w], lo), range), fb);
-        uint32_t b = __float2uint_rz(v);
-        b = b < bins ? b : bins - 1;
-        atomicAdd(&h[b], 1u);
-    }
-    __syncthreads();
-    for (uint32_t b = threadIdx.x; b < bins; b += blockDim.x)
-        if (h[b]) atomicAdd(&counts[(uint64_t)d * bins + b], h[b]);
-}
-
-// uint_to_real (nvidia-gtx-estimate.cu:34-44) and bitonic_local (:117-147): the
-// reference's compare-exchange network over (bin, pdf) pairs, decreasing pdf; equal
-// pdfs count as "smaller" when the partner position j is below lid.
-__global__ void hist_finish(const uint32_t* counts, const float* limits, uint32_t bins,
-                            float alpha, float* pdf, float* ranks) {
-    extern __shared__ float2 aux[];
-    const uint32_t d = blockIdx.x, lid = threadIdx.x;
-    const float c = __fdiv_rn(alpha, __fsub_rn(limits[2 * d + 1], limits[2 * d]));
-    const float p = __fmul_rn(c, (float)counts[(uint64_t)d * bins + lid]);
-    pdf[(uint64_t)d * bins + lid] = p;
-    float2 v = make_float2((float)lid, p);
-    aux[lid] = v;
-    __syncthreads();
-    for (uint32_t length = 1; length < bins; length <<= 1) {
-        const bool direction = (lid & (length << 1)) != 0;
-        for (uint32_t inc = length; inc > 0; inc >>= 1) {
-            const uint32_t j = lid ^ inc;
-            const float2 o = aux[j];
-            const bool smaller = (v.y < o.y) || (o.y == v.y && j < lid);
-            const bool swap = smaller ^ (j < lid) ^ direction;
-            v = swap ? o : v;
-            __syncthreads();
-            aux[lid] = v;
-            __syncthreads();
-        }
-    }
-    ranks[(uint64_t)d * bins + lid] = v.x;
-}
-
 // One CTA per (step, dim): the 2 x G per-CTA sums part[((t*2 + h)*D + d)*G + b] read
 // coalesced along b, summed in FP64 in a fixed order.
 __global__ void reduce_means(const bay_ctl* ctl, const float* part, float* means,
@@ -376,12 +232,6 @@ __global__ void gemm_tc_image(const float* A, uint64_t ld, uint32_t rows, uint32
             aux[e] = (r < rows && cc < aux_len) ? A[r * ld + aux_col + cc] : 0.0f;
         }
     }
-}
-
-__global__ void fill_u32(uint32_t* p, uint32_t v, uint64_t n) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        p[i] = v;
 }
 
 __global__ void fill_bytes(uint4* p, uint64_t n16, unsigned int v) {
@@ -513,54 +363,6 @@ cudaError_t launch_init_normal(float* xs, uint32_t D, uint64_t W, uint32_t seed,
     return cudaGetLastError();
 }
 
-cudaError_t launch_soa_to_aos(const float* xs, uint32_t D, uint64_t W, uint64_t w0, uint64_t n,
-                              float* out, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    dim3 grid((unsigned)((n + 31) / 32), (D + 31) / 32), block(32, 8);
-    soa_to_aos<<<grid, block, 0, s>>>(xs, D, W, w0, n, out);
-    g_launches++;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_aos_to_soa(const float* in, uint32_t D, uint64_t W, float* xs, cudaStream_t s) {
-    dim3 grid((unsigned)((W + 31) / 32), (D + 31) / 32), block(32, 8);
-    aos_to_soa<<<grid, block, 0, s>>>(in, D, W, xs);
-    g_launches++;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_moments(const float* xs, uint32_t D, uint64_t W, double* mean, double* var,
-                           cudaStream_t s) {
-    moments<<<D, 512, 0, s>>>(xs, D, W, mean, var);
-    g_launches++;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_minmax(const float* xs, uint32_t D, uint64_t W, int zero_fold, float* limits,
-                          cudaStream_t s) {
-    minmax<<<D, 512, 0, s>>>(xs, D, W, zero_fold, limits);
-    g_launches++;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_hist_count(const float* xs, uint32_t D, uint64_t W, uint32_t bins,
-                              const float* limits, uint32_t* counts, cudaStream_t s) {
-    unsigned gx = grid_for(W, 256, 64);
-    dim3 grid(gx, D);
-    hist_count<<<grid, 256, bins * sizeof(uint32_t), s>>>(xs, D, W, bins, limits, counts);
-    g_launches++;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_hist_finish(const uint32_t* counts, const float* limits, uint32_t D,
-                               uint32_t bins, uint64_t n, float* pdf, float* ranks,
-                               cudaStream_t s) {
-    const float alpha = (float)((double)bins / (double)n);
-    hist_finish<<<D, bins, bins * sizeof(float2), s>>>(counts, limits, bins, alpha, pdf, ranks);
-    g_launches++;
-    return cudaGetLastError();
-}
-
 cudaError_t launch_reduce_means(const bay_ctl* ctl, const float* part, float* means,
                                 uint32_t means_cap, uint32_t G, uint32_t D, uint32_t nsteps,
                                 double inv_W, cudaStream_t s) {
@@ -596,13 +398,6 @@ cudaError_t launch_gemm_tc_image(const float* A, uint64_t ld, uint32_t rows, uin
     const uint64_t n = (uint64_t)KC * NP * 8 + (uint64_t)NP * auxs;
     gemm_tc_image<<<grid_for(n, 256), 256, 0, s>>>(A, ld, rows, F, KC, NP, aux_col, aux_len, auxs,
                                                     static_cast<unsigned char*>(img));
-    g_launches++;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fill_u32(uint32_t* p, uint32_t v, uint64_t n, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    fill_u32<<<grid_for(n, 256), 256, 0, s>>>(p, v, n);
     g_launches++;
     return cudaGetLastError();
 }

@@ -101,24 +101,34 @@ cudaError_t launch_init_uniform(float* xs, uint32_t D, uint64_t W, uint32_t seed
                                 const float* limits, cudaStream_t s);
 cudaError_t launch_init_normal(float* xs, uint32_t D, uint64_t W, uint32_t seed, float mean,
                                float sd, cudaStream_t s);
-// SoA xs[d*W + w] <-> AoS out[w*D + d] (dim x W column-major), for walkers [w0, w0+n).
-cudaError_t launch_soa_to_aos(const float* xs, uint32_t D, uint64_t W, uint64_t w0, uint64_t n,
-                              float* out, cudaStream_t s);
-cudaError_t launch_aos_to_soa(const float* in, uint32_t D, uint64_t W, float* xs, cudaStream_t s);
-// FP64 per-dim mean and population variance over W walkers (two passes per dim).
-cudaError_t launch_moments(const float* xs, uint32_t D, uint64_t W, double* mean, double* var,
-                           cudaStream_t s);
-// Per-dim [min, max] into limits[2*d], [2*d+1]; zero_fold folds 0.0 in (reference Q7).
-cudaError_t launch_minmax(const float* xs, uint32_t D, uint64_t W, int zero_fold, float* limits,
+// How an estimate kernel is spread: equal tiles of at most 256 dimensions, gx CTAs a tile
+// (kEstCtas CTAs at most unless the tiles alone are more).
+constexpr uint32_t kEstCtas = 608;        // 4 CTAs of 256 threads an SM
+constexpr uint32_t kEstTickets = 1024;    // one a tile wherever gx > 1
+constexpr uint32_t kHistCounts = 12288;   // shared-memory counts of a histogram CTA (48 KB)
+struct est_plan {
+    uint32_t tile = 1, gy = 1, gx = 1, copies = 1;
+};
+est_plan est_plan_of(uint32_t D, uint64_t W, uint32_t tile_max, uint64_t rows_min);
+est_plan hist_plan_of(uint32_t D, uint64_t W, uint32_t bins);
+// Bytes of the estimate kernels' workspace: kEstTickets words, zero before the first use
+// and after every launch, then the CTAs' partial results.
+size_t est_workspace(uint32_t D, uint64_t W);
+// Per-dim FP64 mean and (var not NULL) population variance of x[w * D + d] over W points.
+cudaError_t launch_moments(const float* x, uint32_t D, uint64_t W, double* mean, double* var,
+                           void* ws, cudaStream_t s);
+// Per-dim [min, max] into limits[2*d], [2*d+1]; zero_fold folds 0.0 in (reference Q7).  Also
+// sets counts[0, n_counts) to `start`.
+cudaError_t launch_limits(const float* x, uint32_t D, uint64_t W, int zero_fold, float* limits,
+                          uint32_t* counts, uint64_t n_counts, uint32_t start, void* ws,
                           cudaStream_t s);
-// counts[d*bins + b] += bin counts of the walkers (bins <= 4096).
-cudaError_t launch_hist_count(const float* xs, uint32_t D, uint64_t W, uint32_t bins,
+// counts[d*bins + b] += bin counts of the points (bins <= 1024).
+cudaError_t launch_hist_count(const float* x, uint32_t D, uint64_t W, uint32_t bins,
                               const float* limits, uint32_t* counts, cudaStream_t s);
 // pdf = (bins/n)/(hi-lo) * count, then bitonic ranks (bins a power of two <= 1024).
 cudaError_t launch_hist_finish(const uint32_t* counts, const float* limits, uint32_t D,
                                uint32_t bins, uint64_t n, float* pdf, float* ranks,
                                cudaStream_t s);
-cudaError_t launch_fill_u32(uint32_t* p, uint32_t v, uint64_t n, cudaStream_t s);
 // The GEMM form's matrix (rows x F at A, row stride ld, aux values at column aux_col)
 // laid out feature-major with rows zero-padded to NP, then the aux values [NP][auxs].
 cudaError_t launch_gemm_layout(const float* A, uint64_t ld, uint32_t rows, uint32_t F, uint32_t NP,

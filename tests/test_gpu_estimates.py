@@ -1,0 +1,93 @@
+"""The estimate kernels (moments, limits, histograms) at the sizes where their split changes:
+one and several dimension tiles, one and several CTAs a tile, ragged rows, and values that
+leave the fp32 batches' range."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def factory():
+    from bayadera_gb300.engine import GB300BayaderaFactory
+    f = GB300BayaderaFactory()
+    yield f
+    f.release()
+
+
+def matrix(n, dim, kind):
+    rng = np.random.default_rng(1000 * dim + n)
+    x = rng.standard_normal((n, dim))
+    if kind == "offset":
+        x = x + 1e4 * (1 + np.arange(dim))
+    elif kind == "huge":
+        x = x * 1e30
+    elif kind == "tiny":
+        x = x * 1e-30
+    elif kind == "mixed":
+        x[:: max(1, n // 7)] *= 1e18
+    return x.astype(np.float32)
+
+
+SHAPES = [(1, 1), (5, 3), (16, 256), (17, 257), (255, 1), (4095, 1), (4097, 2), (40001, 7),
+          (3001, 50), (700, 300), (33, 1000), (300007, 1), (60013, 6)]
+
+
+# A mean's error: FP64 additions over a tree (below 2^-49 of the mean absolute value at
+# these sizes) and 2^-47 for a batch's fp32 error words; a variance's the same of itself (the
+# deviations are exact): 1e-12 covers every case by a factor above 50.
+@pytest.mark.parametrize("kind", ["normal", "offset", "huge", "tiny", "mixed"])
+@pytest.mark.parametrize("n,dim", SHAPES)
+def test_moments_match_long_double(factory, n, dim, kind):
+    x = matrix(n, dim, kind)
+    mean, var = factory.data_moments(x)
+    v = x.astype(np.longdouble)
+    mu = v.sum(axis=0) / n
+    want = ((v - mu) ** 2).sum(axis=0) / n
+    assert np.all(np.abs(mean - mu) <= 1e-12 * np.abs(v).mean(axis=0))
+    assert np.all(np.abs(var - want) <= 1e-12 * want)
+
+
+def test_moments_of_constants_and_non_finite_columns(factory):
+    x = matrix(5000, 6, "normal")
+    x[:, 0] = 3.7
+    x[17, 1] = np.inf
+    x[18, 2] = np.nan
+    x[19, 3] = -np.inf
+    x[20, 3] = np.inf
+    x[:, 4] = 3e38
+    mean, var = factory.data_moments(x)
+    assert mean[0] == np.float32(3.7) and 0.0 <= var[0] < 1e-28
+    assert mean[1] == np.inf and np.isnan(var[1])
+    assert np.isnan(mean[2]) and np.isnan(var[2]) and np.isnan(mean[3])
+    assert abs(mean[4] / np.float64(np.float32(3e38)) - 1) < 1e-14
+    assert abs(var[5] / x[:, 5].astype(np.float64).var() - 1) < 1e-12
+
+
+@pytest.mark.parametrize("flags", [0, 1])
+@pytest.mark.parametrize("bins", [2, 64, 1024])
+@pytest.mark.parametrize("n,dim", SHAPES[1:])
+def test_histogram_matches_float32_binning(factory, n, dim, bins, flags):
+    x = matrix(n, dim, "normal")
+    h = factory.data_histogram(x, bins, flags)
+    lo, hi = x.min(axis=0), x.max(axis=0)
+    assert np.array_equal(h.limits, np.stack([lo, hi]))
+    b = ((x - lo) / (hi - lo) * np.float32(bins)).astype(np.uint32)
+    b = np.minimum(b, bins - 1)
+    counts = np.stack([np.bincount(c, minlength=bins) for c in b.T], axis=1) + flags
+    scale = np.float32(bins / n) / (hi - lo)
+    assert np.array_equal(h.pdf, scale * counts.astype(np.float32))
+    order = np.take_along_axis(h.pdf, h.bin_ranks.astype(np.int64), axis=0)
+    assert np.all(np.diff(order, axis=0) <= 0)
+    assert np.array_equal(np.sort(h.bin_ranks, axis=0),
+                          np.repeat(np.arange(bins, dtype=np.float32)[:, None], dim, axis=1))
+
+
+def test_limits_pass_over_nan(factory):
+    x = matrix(3000, 3, "normal")
+    x[0, 0] = np.nan
+    x[2999, 1] = np.nan
+    x[:, 2] = np.nan
+    h = factory.data_histogram(x, 16)
+    assert h.limits[0, 0] == np.nanmin(x[:, 0]) and h.limits[1, 1] == np.nanmax(x[:, 1])
+    assert np.all(np.isnan(h.limits[:, 2]))
