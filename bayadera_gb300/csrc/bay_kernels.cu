@@ -2,6 +2,8 @@
 // forms' matrix layouts, per-step means, acor, and the device-resident control block.  The
 // estimates are in bay_estimates.cu, the per-model fused stretch kernels in
 // device/bay_stretch.cuh (NVRTC).
+#include <cooperative_groups.h>
+
 #include <atomic>
 
 #include "bay_kernels.cuh"
@@ -241,67 +243,216 @@ __global__ void fill_bytes(uint4* p, uint64_t n16, unsigned int v) {
         p[i] = q;
 }
 
-// One acor pass (nvidia-gtx-acor.cu:40-103) in FP64: x_t = m[t*stride] for t + lag < n;
-// the lag window of t reads x (zeroed past n - lag) inside t's block of B = min(wgs, n)
-// entries and raw m across the block edge, as the reference's shared-memory window does.
-__device__ void acor_pass(const double* m, uint64_t stride, uint32_t n, uint32_t wgs,
-                          uint32_t lag, double* red, double* c0_out, double* d_out) {
-    const uint32_t B = wgs < n ? wgs : n;
-    double c0 = 0.0, dd = 0.0;
-    for (uint32_t t = threadIdx.x; t + lag < n; t += blockDim.x) {
-        const double x = m[(uint64_t)t * stride];
-        const uint32_t blk_end = (t / B + 1) * B;
-        double acc = 0.0;
-        for (uint32_t s = 1; s <= lag; ++s) {
-            const uint32_t u = t + s;
-            double v;
-            if (u < blk_end) v = (u + lag < n) ? m[(uint64_t)u * stride] : 0.0;
-            else v = m[(uint64_t)u * stride];
-            acc += v;
-        }
-        c0 += x * x;
-        dd += x * (x + 2.0 * acc);
-    }
-    const double C0 = block_sum_d(c0, red);
-    const double DD = block_sum_d(dd, red);
-    *c0_out = C0;
-    *d_out = DD;
+// acor (nvidia-gtx-acor.cu:116-168 + nvidia_gtx.clj:240-278), a cluster of C CTAs a
+// dimension, no dynamic parallelism: mean, centring, the first pass, then pairwise halving
+// while 10 < lag2 and lag2 < 5 tau; tau = D (n - lag) / (stride (n2 - lag2) C0_first),
+// sigma = sqrt(D / (stride (n2 - lag2) n)).
+// FP64 issue bounds it (1.9 operations a clock an SM).  A pass needs, for every t with
+// t + lag < n, x_t^2 and x_t times the sum of the lag entries after t: adding those up for
+// each t is n lag additions.  A thread here takes a run of R consecutive t from a tile in
+// shared memory, puts the first window together from the runs' sums and slides it: about
+// 1.3 + 2 additions a t at R = 16, lag = 64.  C grows with the series to 16 CTAs (a cluster of that size is opt-in; 8 otherwise),
+// whose partial sums meet in distributed shared memory: a barrier of a cluster costs some
+// hundred ns, a grid's over a us, and the decision to halve needs two for every level.
+// 8 x 200,003 values: 191 us; 7,975 us with one 256-thread CTA a dimension and full windows.
+constexpr uint32_t kAcorThreads = 256;
+constexpr uint32_t kAcorRun = 16;                          // longest run of a thread
+constexpr uint32_t kAcorMaxLag = 64;
+constexpr uint32_t kAcorTile = kAcorThreads * kAcorRun + kAcorMaxLag;
+constexpr uint32_t kAcorCluster = 16;
+
+// a padded slot an entry: runs of 16 start in different banks
+__device__ __forceinline__ uint32_t acor_slot(uint32_t i) { return i + (i >> 4); }
+
+struct acor_shared {
+    double tile[kAcorTile + kAcorTile / 16 + 1];
+    double runs[kAcorThreads + kAcorMaxLag / kAcorRun];   // sums of the tile's runs of 16
+    double tail[2 * kAcorMaxLag];                          // the series' last entries
+    double red[2][kAcorThreads];
+    double got[2][kAcorCluster];       // the CTAs' partial sums, written by each of them
+};
+
+__device__ __forceinline__ void cluster_sync(cooperative_groups::cluster_group& cl) {
+    if (cl.num_blocks() == 1) __syncthreads();
+    else cl.sync();
 }
 
-// acor (nvidia-gtx-acor.cu:116-168 + nvidia_gtx.clj:240-278) for one dim per CTA, with
-// no dynamic parallelism: mean, centring, the first pass, then pairwise halving while
-// 10 < lag2 and lag2 < 5 tau; tau = D (n - lag) / (stride (n2 - lag2) C0_first),
-// sigma = sqrt(D / (stride (n2 - lag2) n)).
-__global__ void acor_kernel(const float* series, uint32_t D, uint32_t n, uint32_t wgs,
-                            uint32_t lag, double* work, double* tau_out, double* mean_out,
-                            double* sigma_out) {
-    __shared__ double red[33];
-    const uint32_t d = blockIdx.x;
-    double* m = work + (uint64_t)d * n;
-    double s = 0.0;
-    for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) s += (double)series[(uint64_t)t * D + d];
-    const double mu = block_sum_d(s, red) / (double)n;
-    for (uint32_t t = threadIdx.x; t < n; t += blockDim.x)
-        m[t] = (double)series[(uint64_t)t * D + d] - mu;
+// The cluster's sums of the N values, in lane, warp and CTA order; a barrier of the cluster.
+// (An FP64 instruction takes a warp 17 clocks of the SM here, however many lanes it has: the
+// first levels go over shared memory, where a warp adds up four warps' values.)
+template <int N>
+__device__ __forceinline__ void cluster_sum(cooperative_groups::cluster_group& cl, acor_shared& sh,
+                                            double (&v)[N]) {
+    const uint32_t C = cl.num_blocks(), me = cl.block_rank(), tid = threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < N; ++k) sh.red[k][tid] = v[k];
     __syncthreads();
+    if (tid < 32) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            double a = sh.red[k][tid];
+#pragma unroll
+            for (uint32_t w = 1; w < kAcorThreads / 32; ++w) a += sh.red[k][tid + 32 * w];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(FULL, a, o);
+            if (tid < C) {
+                if (C == 1) sh.got[k][0] = a;
+                else *cl.map_shared_rank(&sh.got[k][me], tid) = a;
+            }
+        }
+    }
+    cluster_sync(cl);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        double a = sh.got[k][0];
+        for (uint32_t r = 1; r < C; ++r) a += sh.got[k][r];
+        v[k] = a;
+    }
+}
+
+// One pass (nvidia-gtx-acor.cu:40-103) in FP64: x_t = m[t*stride] for t + lag < n; the lag
+// window of t reads x (zeroed past n - lag) inside t's block of B = min(wgs, n) entries and
+// raw m across the block edge, as the reference's shared-memory window does.  So only the
+// windows of the last lag t's that reach past n - lag differ from raw ones; those are
+// added up one by one, on the last CTA.
+__device__ void acor_pass(cooperative_groups::cluster_group& cl, acor_shared& sh, const double* m,
+                          uint64_t stride, uint32_t n, uint32_t wgs, uint32_t lag, uint32_t R,
+                          double* c0_out, double* d_out) {
+    const uint32_t C = cl.num_blocks(), me = cl.block_rank(), tid = threadIdx.x;
+    const uint32_t plain = n > 2u * lag ? n - 2u * lag : 0u;      // t below: raw windows
+    const uint32_t per = kAcorThreads * R;
+    double c0 = 0.0, dd = 0.0;
+    if (me == C - 1 && plain + tid < n && tid < 2u * lag)
+        sh.tail[tid] = __ldcg(&m[(uint64_t)(plain + tid) * stride]);
+    for (uint64_t t0 = (uint64_t)me * per; t0 < plain; t0 += (uint64_t)C * per) {
+        const uint32_t have = (uint32_t)(n - t0 < per + lag ? n - t0 : per + lag);
+        __syncthreads();
+        for (uint32_t i = tid; i < have; i += kAcorThreads)
+            sh.tile[acor_slot(i)] = __ldcg(&m[(t0 + i) * stride]);
+        __syncthreads();
+        const uint32_t i0 = tid * R;
+        const bool by_runs = R == kAcorRun && lag + 1 >= kAcorRun;
+        if (by_runs) {      // entries past `have` are read (not used by any window): in the tile
+            for (uint32_t j = tid; j < kAcorThreads + kAcorMaxLag / kAcorRun; j += kAcorThreads) {
+                double q = 0.0;
+#pragma unroll
+                for (uint32_t i = 0; i < kAcorRun; ++i) q += sh.tile[acor_slot(j * kAcorRun + i)];
+                sh.runs[j] = q;
+            }
+            __syncthreads();
+        }
+        if (t0 + i0 < plain) {
+            const uint32_t i1 = plain - t0 < i0 + R ? (uint32_t)(plain - t0) : i0 + R;
+            double acc = 0.0;
+            uint32_t s = 1;
+            if (by_runs) {
+#pragma unroll
+                for (; s < kAcorRun; ++s) acc += sh.tile[acor_slot(i0 + s)];
+                for (; s + kAcorRun <= lag + 1; s += kAcorRun) acc += sh.runs[tid + s / kAcorRun];
+            }
+            double part[4] = {};                        // (shorter chains of additions)
+            for (; s + 3 <= lag; s += 4)
+#pragma unroll
+                for (uint32_t q = 0; q < 4; ++q) part[q] += sh.tile[acor_slot(i0 + s + q)];
+            for (; s <= lag; ++s) acc += sh.tile[acor_slot(i0 + s)];
+            acc += (part[0] + part[1]) + (part[2] + part[3]);
+            double x = sh.tile[acor_slot(i0)];
+            for (uint32_t i = i0;;) {
+                c0 += x * x;
+                dd += x * (x + 2.0 * acc);
+                if (++i >= i1) break;
+                x = sh.tile[acor_slot(i)];
+                acc += sh.tile[acor_slot(i + lag)] - x;
+            }
+        }
+    }
+    if (me == C - 1) {
+        // t in [plain, n - lag), the last threads first: in a short series those have no run,
+        // so both parts go on at once
+        const uint32_t B = wgs < n ? wgs : n;
+        if ((uint64_t)me * per >= plain) __syncthreads();   // no tile: the staged entries' barrier
+        const uint64_t t = (uint64_t)plain + (kAcorThreads - 1u - tid);
+        if (t + lag < n) {                              // fewer than 2 lag <= 128 of them
+            const double x = sh.tail[t - plain];
+            const uint64_t blk_end = (t / B + 1) * B;
+            double part[4] = {};
+            for (uint64_t u = t + 1; u <= t + lag; u += 4)
+#pragma unroll
+                for (uint32_t q = 0; q < 4; ++q)
+                    if (u + q <= t + lag && (u + q >= blk_end || u + q + lag < n))
+                        part[q] += sh.tail[u + q - plain];
+            const double acc = (part[0] + part[1]) + (part[2] + part[3]);
+            c0 += x * x;
+            dd += x * (x + 2.0 * acc);
+        }
+    }
+    double both[2] = {c0, dd};
+    cluster_sum(cl, sh, both);
+    *c0_out = both[0];
+    *d_out = both[1];
+}
+
+__global__ void __launch_bounds__(kAcorThreads)
+acor_kernel(const float* series, uint32_t D, uint32_t n, uint32_t wgs, uint32_t lag, double* work,
+            double* tau_out, double* mean_out, double* sigma_out) {
+    __shared__ acor_shared sh;
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const uint32_t C = cl.num_blocks(), me = cl.block_rank();
+    const uint32_t d = blockIdx.x / C;
+    double* m = work + (uint64_t)d * n;
+    cluster_sync(cl);                                 // every CTA's shared memory is there
+    const uint64_t step = (uint64_t)C * kAcorThreads, first = (uint64_t)me * kAcorThreads + threadIdx.x;
+    constexpr uint32_t U = 8;                         // loads in flight
+    double sum[1] = {};
+    for (uint64_t t = first; t < n; t += U * step) {
+        float v[U];
+#pragma unroll
+        for (uint32_t i = 0; i < U; ++i) v[i] = t + i * step < n ? __ldg(&series[(t + i * step) * D + d]) : 0.0f;
+#pragma unroll
+        for (uint32_t i = 0; i < U; ++i)
+            if (t + i * step < n) sum[0] += (double)v[i];
+    }
+    cluster_sum(cl, sh, sum);
+    const double mu = sum[0] / (double)n;
+    for (uint64_t t = first; t < n; t += U * step) {
+        float v[U];
+#pragma unroll
+        for (uint32_t i = 0; i < U; ++i) v[i] = t + i * step < n ? __ldg(&series[(t + i * step) * D + d]) : 0.0f;
+#pragma unroll
+        for (uint32_t i = 0; i < U; ++i)
+            if (t + i * step < n) m[t + i * step] = (double)v[i] - mu;
+    }
+    cluster_sync(cl);
+    // shorter runs while the threads outnumber the entries
+    const uint32_t R = n / (C * kAcorThreads) >= 8u ? kAcorRun : 4u;
     double c0a, da;
-    acor_pass(m, 1, n, wgs, lag, red, &c0a, &da);
+    acor_pass(cl, sh, m, 1, n, wgs, lag, R, &c0a, &da);
     const double c0 = c0a;
     double tau = da / c0;
-    uint32_t lag2 = lag, n2 = n, stride = 1;
+    uint32_t lag2 = lag, n2 = n;
+    uint64_t stride = 1;
     while (10u < lag2 && (double)lag2 < tau * 5.0) {
         n2 /= 2;
         lag2 = (lag * 5u < n2) ? lag : ((n2 / 5u) > 10u ? n2 / 5u : 10u);
         const double c0prev = c0a;
-        __syncthreads();
-        for (uint32_t g = threadIdx.x; g < n2; g += blockDim.x)
-            m[(uint64_t)2 * g * stride] += m[(uint64_t)(2 * g + 1) * stride];
-        __syncthreads();
+        for (uint64_t g = first; g < n2; g += U * step) {
+            double v[U], w[U];
+#pragma unroll
+            for (uint32_t i = 0; i < U; ++i) {
+                const uint64_t h = g + i * step < n2 ? g + i * step : g;
+                v[i] = __ldcg(&m[2 * h * stride]);
+                w[i] = __ldcg(&m[(2 * h + 1) * stride]);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < U; ++i)
+                if (g + i * step < n2) m[2 * (g + i * step) * stride] = v[i] + w[i];
+        }
+        cluster_sync(cl);
         stride *= 2;
-        acor_pass(m, stride, n2, wgs, lag2, red, &c0a, &da);
+        acor_pass(cl, sh, m, stride, n2, wgs, lag2, R, &c0a, &da);
         tau = da / c0prev;
     }
-    if (threadIdx.x == 0) {
+    if (me == 0 && threadIdx.x == 0) {
         const double scale = (double)stride * (double)(n2 - lag2);
         tau_out[d] = da * (double)(n - lag) / (scale * c0);
         mean_out[d] = mu;
@@ -404,7 +555,36 @@ cudaError_t launch_gemm_tc_image(const float* A, uint64_t ld, uint32_t rows, uin
 
 cudaError_t launch_acor(const float* series, uint32_t D, uint32_t n, uint32_t wgs, uint32_t lag,
                         double* work, double* tau, double* mean, double* sigma, cudaStream_t s) {
-    acor_kernel<<<D, 256, 0, s>>>(series, D, n, wgs, lag, work, tau, mean, sigma);
+    // a CTA of the cluster for every 1,024 entries, a power of two up to 16 (8 where the
+    // device takes no cluster of 16)
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(kAcorThreads);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    uint32_t C = 1;
+    while (C < kAcorCluster && (uint64_t)C * 1024u < n) C *= 2;
+    if (C > 8) {
+        cudaError_t e = cudaFuncSetAttribute(acor_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
+        at[0].val.clusterDim.x = C;
+        cfg.gridDim = dim3(C);
+        int fit = 0;
+        e = cudaOccupancyMaxActiveClusters(&fit, acor_kernel, &cfg);
+        if (e != cudaSuccess || fit < 1) {
+            cudaGetLastError();
+            C = 8;
+        }
+    }
+    at[0].val.clusterDim.x = C;
+    cfg.gridDim = dim3(D * C);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, acor_kernel, series, D, n, wgs, lag, work, tau, mean,
+                                             sigma);
+    if (e != cudaSuccess) return e;
     g_launches++;
     return cudaGetLastError();
 }

@@ -91,3 +91,24 @@ def test_limits_pass_over_nan(factory):
     h = factory.data_histogram(x, 16)
     assert h.limits[0, 0] == np.nanmin(x[:, 0]) and h.limits[1, 1] == np.nanmax(x[:, 1])
     assert np.all(np.isnan(h.limits[:, 2]))
+
+
+# FP64 sums of n lag terms in another order than the oracle's: n lag 2^-53 is 3e-10 at the
+# longest series, and a random walk of the roundings some 1e-13.
+@pytest.mark.parametrize("rho", [0.0, 0.97])
+@pytest.mark.parametrize("wgs", [64, 1024])
+@pytest.mark.parametrize("n", [50, 51, 127, 320, 1024, 1025, 2049, 4224, 16385, 40003])
+def test_acor_matches_oracle_at_the_split_edges(oracle, n, wgs, rho):
+    from bayadera_gb300.engine import GB300BayaderaFactory
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((3, n))
+    for t in range(1, n):
+        x[:, t] += rho * x[:, t - 1]
+    x = x.astype(np.float32)
+    with GB300BayaderaFactory(wgs=wgs) as f:
+        got = f.acor(x)
+    tau, mean, sigma, lag = oracle.acor64(x, wgs)
+    assert got.lag == lag
+    assert np.allclose(got.tau, tau, rtol=1e-11, atol=0)
+    assert np.allclose(got.sigma, sigma, rtol=1e-11, atol=0, equal_nan=True)
+    assert np.allclose(got.mean, mean, rtol=0, atol=1e-13 * np.abs(x).max())
