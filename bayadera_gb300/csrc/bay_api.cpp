@@ -270,6 +270,10 @@ size_t gemm_smem_bytes(const bay_model* m, uint64_t rows) {
                             kGemmWalkers * dpad + np * auxs);
 }
 
+// Streamed GEMM form: walkers per CTA of the propose kernel (BAY_PW), their rows in at most
+// 48 KB of shared memory (8 rows up to 1,535 coordinates, 2 up to the largest dim of 4,096).
+uint32_t gemm_propose_walkers(uint32_t dim) { return (dim | 1u) * 8 * sizeof(float) <= 49152 ? 8u : 2u; }
+
 // Tiled form: the data rows are staged in chunks of kTileChunk floats (BAY_TILE_CHUNK of
 // the kernel), rounded down to whole rows, a multiple of 4; two chunk buffers when the
 // data span more than one chunk, else one buffer of the data's size.
@@ -492,8 +496,10 @@ struct bay_sampler {
     void launch_streaming(int mode, uint32_t half, uint32_t step_off, cudaStream_t st) {
         bay_stretch_params p = make_params(half, step_off);
         const uint64_t nk = mode == 2 ? W : K;
+        const uint32_t pw = gemm_propose_walkers(D);
         const unsigned g1 = (unsigned)((nk + 255) / 256), gt = (unsigned)((nk + 127) / 128);
-        launch(model->k_gp[mode], g1, 1, 0, p, st, "cuLaunchKernel(gemm propose)");
+        launch(model->k_gp[mode], (unsigned)((nk + pw - 1) / pw), 1, 0, p, st,
+               "cuLaunchKernel(gemm propose)");
         if (tc) {
             const uint64_t per = 128ull * model->tc_g;
             void* args[] = {&p, &tc_maps};
@@ -506,7 +512,8 @@ struct bay_sampler {
             launch(model->k_gr[mode == 2 ? 1 : 0], gt, s_nsb, smem_rows, p, st,
                    "cuLaunchKernel(gemm rows)");
         }
-        launch(model->k_ga[mode], g1, 1, 0, p, st, "cuLaunchKernel(gemm accept)");
+        launch(model->k_ga[mode], g1, mode == 2 ? 1u : (D + 63) / 64, 0, p, st,
+               "cuLaunchKernel(gemm accept)");
         if (st == ctx->stream) bay::count_launches(3);
     }
 
@@ -931,6 +938,7 @@ Codegen codegen(const bay_model_desc* d, uint32_t wgs) {
         const uint32_t pl = d->prep_len ? d->prep_len : 1u;
         if (pl > 64) fail(BAY_ERR_ARG, "prep_len must be <= 64");
         opts.push_back("-DBAY_GEMM=1");
+        opts.push_back("-DBAY_PW=" + std::to_string(gemm_propose_walkers(d->dim)) + "u");
         opts.push_back("-DBAY_GEMM_F=" + std::to_string(d->gemm_features));
         opts.push_back("-DBAY_GEMM_COEF=" + std::to_string(d->gemm_coef));
         opts.push_back("-DBAY_GEMM_AUX=" + std::to_string(d->gemm_aux_len));
@@ -1298,7 +1306,7 @@ static int sampler_create(bay_model* m, uint32_t seed, uint64_t walkers, const f
                 s->s_b = (float*)c->alloc(sizeof(float) * Wn * m->gemm_features);
                 s->s_prep = (float*)c->alloc(sizeof(float) * Wn * m->prep_len);
                 s->s_w = (float*)c->alloc(sizeof(float) * Wn);
-                s->s_zu = (float*)c->alloc(sizeof(float) * Wn * 2);
+                s->s_zu = (float*)c->alloc(sizeof(float) * Wn * 3);
                 s->s_part = (float*)c->alloc(sizeof(float) * Wn * 2 * s->s_nsb);
                 if (s->tc) {
                     const uint32_t auxs = m->gemm_aux_len ? m->gemm_aux_len : 1u;

@@ -99,7 +99,7 @@ struct bay_stretch_params {
     float* s_b;                     // [nk][F] coefficient block
     float* s_prep;                  // [nk][BAY_PREP_LEN]
     float* s_w;                     // [nk] terms outside the row sum
-    float* s_zu;                    // [nk][2] stretch factor and accept uniform
+    float* s_zu;                    // [nk][3] stretch factor, accept uniform, log density
     float* s_part;                  // [nsb][nk] compensated (hi, lo) partial row sums
     unsigned int s_nsb;             // row super-blocks
     unsigned int s_sbrows;          // rows per super-block (a multiple of 128)
@@ -516,7 +516,7 @@ extern "C" __global__ void __launch_bounds__(256) bay_logfn_all(bay_stretch_para
 
 // ---------------------------------------------------------------- GEMM form, streaming
 // For matrices too large for shared memory.  A half-step is three launches:
-//   propose: one thread per walker -- Philox, stretch, partner, proposal row, prep and the
+//   propose: a warp per walker -- Philox, stretch, partner, proposal row, prep and the
 //            terms outside the row sum into per-walker scratch;
 //   rows:    CTA (128-walker tile, row super-block): the tile's coefficient block stays in
 //            shared memory (feature-major); for each 128-row sub-block the matrix is
@@ -525,8 +525,7 @@ extern "C" __global__ void __launch_bounds__(256) bay_logfn_all(bay_stretch_para
 //            lanes of a walker combine as compensated fp32 pairs -> s_part[sb][walker];
 //            blockIdx.x runs over walker tiles so that the tiles sharing a row block run
 //            together and the block is read from HBM once;
-//   accept:  one thread per walker -- partials summed in super-block order, accept,
-//            write-back, statistics.
+//   accept:  partials summed in super-block order, accept, write-back, statistics.
 #define BAY_SW 128
 #define BAY_SR 128
 #define BAY_SF 32
@@ -551,54 +550,85 @@ __device__ __forceinline__ void bay_split_bf16x2(float a, float b, unsigned int&
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(__fsub_rn(b, hb)), "f"(__fsub_rn(a, ha)));
 }
 
+// Propose: BAY_PW walkers per CTA, a warp per walker with its lanes over the coordinates, so
+// that the walker's row, its partner's and the outputs are read and written in whole
+// sectors; the proposals also stay in shared memory (odd stride), from which one thread per
+// walker evaluates the model's prep and walker terms in the model's own order.  2,048 walkers
+// of 257 coordinates: 5.1 us, 268 us with one thread per walker for the rows too (a sector
+// per float read or written); 8 walkers per CTA are 256 CTAs there.  BAY_PW is the host's (kernel grid), 8 while the rows fit in 48 KB.
 template <int MODE>  // 0 bare, 1 accu, 2 log density of the current positions
 __device__ __forceinline__ void bay_gemm_propose_impl(const bay_stretch_params& P) {
+    __shared__ float sY[BAY_PW][DIM | 1];
     const unsigned int kind = MODE == 1 ? 1u : 0u;
     const unsigned int nk = MODE == 2 ? P.W : P.K;
-    const unsigned int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nk) return;
-    float* y = P.s_y + (size_t)k * DIM;
-    if (MODE == 2) {
-        const float* x = P.xs + (size_t)k * DIM;
-        for (int d = 0; d < DIM; ++d) y[d] = x[d];
-    } else {
-        const float* X = P.xs + (size_t)P.half * P.K * DIM + (size_t)k * DIM;
-        const unsigned int stream = MODE == 1 ? (P.half ? 2222u : 1111u) : (P.half ? 4444u : 3333u);
-        bay_u4 c;
-        c.x = k;
-        c.y = P.ctl->step[kind] + P.step_off;
-        c.z = stream;
-        c.w = 0xbeeff00du;
-        const bay_u4 r = bay_philox4x32_10(c, P.ctl->seed[kind] + P.half, 0xdecafbadu);
-        const float z = bay_stretch_z(P.ctl->a, bay_u01(r.y));
-        const unsigned int j = bay_partner(bay_u01(r.x), P.K);
-        const float* S = P.xs + (size_t)(1u - P.half) * P.K * DIM + (size_t)j * DIM;
-        for (int d = 0; d < DIM; ++d) {
-            const float s = S[d];
-            y[d] = __fmaf_rn(z, __fsub_rn(X[d], s), s);
+    const unsigned int k0 = blockIdx.x * BAY_PW;
+    const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    for (unsigned int i = warp; i < BAY_PW; i += 8u) {
+        const unsigned int k = k0 + i;
+        if (k >= nk) break;
+        float* y = P.s_y + (size_t)k * DIM;
+        const float* X = P.xs + (MODE == 2 ? (size_t)0 : (size_t)P.half * P.K * DIM) + (size_t)k * DIM;
+        const float* S = X;
+        float z = 0.0f;
+        if (MODE != 2) {
+            const unsigned int stream = MODE == 1 ? (P.half ? 2222u : 1111u) : (P.half ? 4444u : 3333u);
+            bay_u4 c;
+            c.x = k;
+            c.y = P.ctl->step[kind] + P.step_off;
+            c.z = stream;
+            c.w = 0xbeeff00du;
+            const bay_u4 r = bay_philox4x32_10(c, P.ctl->seed[kind] + P.half, 0xdecafbadu);
+            z = bay_stretch_z(P.ctl->a, bay_u01(r.y));
+            const unsigned int j = bay_partner(bay_u01(r.x), P.K);
+            S = P.xs + (size_t)(1u - P.half) * P.K * DIM + (size_t)j * DIM;
+            if (lane == 0u) {
+                P.s_zu[3 * (size_t)k] = z;
+                P.s_zu[3 * (size_t)k + 1] = bay_u01(r.z);
+                P.s_zu[3 * (size_t)k + 2] = P.logfn[(size_t)P.half * P.K + k];
+            }
         }
-        P.s_zu[2 * (size_t)k] = z;
-        P.s_zu[2 * (size_t)k + 1] = bay_u01(r.z);
-    }
-    if (!P.s_bh) {
-        for (int f = 0; f < BAY_GEMM_F; ++f) P.s_b[(size_t)k * BAY_GEMM_F + f] = y[BAY_GEMM_COEF + f];
-    } else {
-        // the tensor-core form's operand: coefficient = hi + lo, both bf16
-        for (int f = 0; f < BAY_GEMM_F; ++f) {
-            const float v = y[BAY_GEMM_COEF + f];
-            const unsigned short h = bay_bf16_rn(v);
-            P.s_bh[(size_t)k * P.tc_fp + f] = h;
-            P.s_bl[(size_t)k * P.tc_fp + f] = bay_bf16_rn(__fsub_rn(v, bay_bf16_float(h)));
+        // 8 coordinates per lane per pass, their loads all in flight
+        for (unsigned int d0 = lane; d0 < DIM; d0 += 256u) {
+            float xv[8], sv[8];
+#pragma unroll
+            for (unsigned int q = 0; q < 8u; ++q) {
+                const unsigned int d = d0 + 32u * q;
+                xv[q] = d < DIM ? X[d] : 0.0f;
+                sv[q] = MODE != 2 && d < DIM ? S[d] : 0.0f;
+            }
+#pragma unroll
+            for (unsigned int q = 0; q < 8u; ++q) {
+                const unsigned int d = d0 + 32u * q;
+                if (d >= DIM) continue;
+                const float v = MODE == 2 ? xv[q] : __fmaf_rn(z, __fsub_rn(xv[q], sv[q]), sv[q]);
+                y[d] = v;
+                sY[i][d] = v;
+                const unsigned int f = d - BAY_GEMM_COEF;
+                if (d < BAY_GEMM_COEF || f >= BAY_GEMM_F) continue;
+                if (!P.s_bh) {
+                    P.s_b[(size_t)k * BAY_GEMM_F + f] = v;
+                } else {
+                    // the tensor-core form's operand: coefficient = hi + lo, both bf16
+                    const unsigned short h = bay_bf16_rn(v);
+                    P.s_bh[(size_t)k * P.tc_fp + f] = h;
+                    P.s_bl[(size_t)k * P.tc_fp + f] = bay_bf16_rn(__fsub_rn(v, bay_bf16_float(h)));
+                }
+            }
         }
     }
-    const float* hyper = P.params + P.data_len;
-    float pr[BAY_PREP_LEN];
+    __syncthreads();
+    const unsigned int k = k0 + threadIdx.x;
+    if (threadIdx.x < BAY_PW && k < nk) {
+        const float* y = sY[threadIdx.x];
+        const float* hyper = P.params + P.data_len;
+        float pr[BAY_PREP_LEN];
 #pragma unroll
-    for (int i = 0; i < BAY_PREP_LEN; ++i) pr[i] = 0.0f;
-    BAY_GEMM_PREP(hyper, P.params_len, DIM, y, pr);
+        for (int i = 0; i < BAY_PREP_LEN; ++i) pr[i] = 0.0f;
+        BAY_GEMM_PREP(hyper, P.params_len, DIM, y, pr);
 #pragma unroll
-    for (int i = 0; i < BAY_PREP_LEN; ++i) P.s_prep[(size_t)k * BAY_PREP_LEN + i] = pr[i];
-    P.s_w[k] = BAY_GEMM_WALKER(P.gemm_rows, hyper, P.params_len, DIM, y);
+        for (int i = 0; i < BAY_PREP_LEN; ++i) P.s_prep[(size_t)k * BAY_PREP_LEN + i] = pr[i];
+        P.s_w[k] = BAY_GEMM_WALKER(P.gemm_rows, hyper, P.params_len, DIM, y);
+    }
 }
 
 template <int MODE>
@@ -700,10 +730,18 @@ __device__ __forceinline__ void bay_gemm_rows_impl(const bay_stretch_params& P) 
     }
 }
 
+// Accept: CTA (256 walkers, a slice of BAY_AD coordinates).  Every slice's CTA decides for
+// its walkers (the current log density is read from the proposal's scratch, so that the
+// first slice's CTA may store the new one) and then moves its coordinates, the 256 rows'
+// segments in whole sectors.  2,048 walkers of 257 coordinates: 11.7 us on 40 CTAs, 86 us
+// with one thread copying its walker's row on 8.
+#define BAY_AD 64u
 template <int MODE>
 __device__ __forceinline__ void bay_gemm_accept_impl(const bay_stretch_params& P) {
+    __shared__ unsigned char sAcc[256];
     const unsigned int nk = MODE == 2 ? P.W : P.K;
-    const unsigned int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned int k0 = blockIdx.x * 256u, k = k0 + threadIdx.x;
+    const unsigned int d0 = blockIdx.y * BAY_AD;
     const bool valid = k < nk;
     bool accepted = false;
     if (valid) {
@@ -720,27 +758,44 @@ __device__ __forceinline__ void bay_gemm_accept_impl(const bay_stretch_params& P
         if (MODE == 2) {
             P.logfn[k] = ly;
         } else {
-            const float lx = P.logfn[(size_t)P.half * P.K + k];
-            accepted = bay_accept(P.s_zu[2 * (size_t)k + 1], P.s_zu[2 * (size_t)k], ly, lx,
-                                  MODE == 1 ? 1.0f : P.ctl->beta);
-            if (accepted) {
-                float* X = P.xs + (size_t)P.half * P.K * DIM + (size_t)k * DIM;
-                const float* y = P.s_y + (size_t)k * DIM;
-                for (int d = 0; d < DIM; ++d) X[d] = y[d];
-                P.logfn[(size_t)P.half * P.K + k] = ly;
+            const float* zu = P.s_zu + 3 * (size_t)k;      // stretch factor, uniform, log density
+            accepted = bay_accept(zu[1], zu[0], ly, zu[2], MODE == 1 ? 1.0f : P.ctl->beta);
+            if (accepted && blockIdx.y == 0u) P.logfn[(size_t)P.half * P.K + k] = ly;
+        }
+    }
+    if (MODE == 2) return;
+    sAcc[threadIdx.x] = accepted ? 1 : 0;
+    const int n_acc = __syncthreads_count(accepted);
+    const unsigned int nv = nk - k0 < 256u ? nk - k0 : 256u;
+    const unsigned int nd = DIM - d0 < BAY_AD ? DIM - d0 : BAY_AD;
+    float* Xc = P.xs + (size_t)P.half * P.K * DIM + (size_t)k0 * DIM + d0;
+    const float* Yc = P.s_y + (size_t)k0 * DIM + d0;
+    {
+        // thread: coordinate tid % 64 of every 4th walker, 8 loads in flight
+        const unsigned int d = threadIdx.x % BAY_AD;
+        for (unsigned int w0 = threadIdx.x / BAY_AD; w0 < nv; w0 += 32u) {
+            float v[8];
+#pragma unroll
+            for (unsigned int i = 0; i < 8u; ++i) {
+                const unsigned int w = w0 + 4u * i;
+                v[i] = w < nv && d < nd && sAcc[w] ? Yc[(size_t)w * DIM + d] : 0.0f;
+            }
+#pragma unroll
+            for (unsigned int i = 0; i < 8u; ++i) {
+                const unsigned int w = w0 + 4u * i;
+                if (w < nv && d < nd && sAcc[w]) Xc[(size_t)w * DIM + d] = v[i];
             }
         }
     }
     if (MODE != 1) return;
     // accu: acceptance count and the per-dim sums of this CTA's walkers (new positions)
-    const int n_acc = __syncthreads_count(accepted);
-    if (threadIdx.x == 0 && n_acc) atomicAdd(&P.ctl->accepted, (unsigned long long)n_acc);
+    if (threadIdx.x == 0 && blockIdx.y == 0u && n_acc)
+        atomicAdd(&P.ctl->accepted, (unsigned long long)n_acc);
     if (P.means_cap == 0) return;
-    const unsigned int k0 = blockIdx.x * blockDim.x;
-    const unsigned int nv = nk - k0 < blockDim.x ? nk - k0 : blockDim.x;
-    const float* Xc = P.xs + (size_t)P.half * P.K * DIM + (size_t)k0 * DIM;
+    __syncthreads();
     float* out = P.part + ((size_t)P.step_off * 2 + P.half) * DIM * gridDim.x + blockIdx.x;
-    for (unsigned int d = threadIdx.x; d < DIM; d += blockDim.x) {
+    if (threadIdx.x < nd) {
+        const unsigned int d = threadIdx.x;
         bay_cf s;
         s.hi = 0.0f;
         s.lo = 0.0f;
@@ -752,7 +807,7 @@ __device__ __forceinline__ void bay_gemm_accept_impl(const bay_stretch_params& P
             y.lo = 0.0f;
             s = bay_cadd(s, y);
         }
-        out[(size_t)d * gridDim.x] = __fadd_rn(s.hi, s.lo);
+        out[(size_t)(d0 + d) * gridDim.x] = __fadd_rn(s.hi, s.lo);
     }
 }
 
