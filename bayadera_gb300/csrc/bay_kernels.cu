@@ -112,23 +112,33 @@ __global__ void init_uniform(float* xs, uint32_t D, uint64_t W, uint32_t seed,
 }
 
 // N(mean, sd^2) init: element e = w*D + d uses pair p = e/2, Philox(ctr {p, 0x6e6f726d,
-// 0x77616c6b, 0xbeeff00d}, key {seed, 0x9a55a9e5}); Box-Muller in FP64 on words 0, 1.
-__global__ void init_normal(float* xs, uint32_t D, uint64_t W, uint32_t seed, float mean,
-                            float sd) {
-    const uint64_t n = (uint64_t)D * W;
-    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < n;
-         e += (uint64_t)gridDim.x * blockDim.x) {
+// 0x77616c6b, 0xbeeff00d}, key {seed, 0x9a55a9e5}); Box-Muller in FP64 on words 0, 1, the
+// even element the cosine's.  FP64 issue bounds it, so a thread makes a pair: one element
+// per thread evaluated the pair's logarithm and both functions twice (3,276,800 elements:
+// 500 us).  Members (n, off, count, seeds): blockIdx.y's block of count values at off, so
+// that a batch of samplers is one launch.
+__device__ __forceinline__ void normal_pairs(float* xs, uint64_t n, uint32_t seed, float mean,
+                                             float sd) {
+    for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; 2 * p < n;
+         p += (uint64_t)gridDim.x * blockDim.x) {
         bay_u4 c;
-        c.x = (unsigned)(e >> 1);
+        c.x = (unsigned)p;
         c.y = 0x6e6f726du;
         c.z = 0x77616c6bu;
         c.w = 0xbeeff00du;
         const bay_u4 r = bay_philox4x32_10(c, seed, 0x9a55a9e5u);
         const double rr = sqrt(-2.0 * log((double)bay_u01(r.y)));
         const double t = 6.283185307179586 * (double)bay_u01(r.x);
-        const double z = (e & 1) ? rr * sin(t) : rr * cos(t);
-        xs[e] = (float)((double)mean + (double)sd * z);
+        xs[2 * p] = (float)((double)mean + (double)sd * (rr * cos(t)));
+        if (2 * p + 1 < n) xs[2 * p + 1] = (float)((double)mean + (double)sd * (rr * sin(t)));
     }
+}
+__global__ void init_normal(float* xs, uint64_t n, uint32_t seed, float mean, float sd) {
+    normal_pairs(xs, n, seed, mean, sd);
+}
+__global__ void init_normal_members(float* xs, const bay_init_member* mem, float mean, float sd) {
+    const bay_init_member m = mem[blockIdx.y];
+    normal_pairs(xs + m.off, m.count, m.seed, mean, sd);
 }
 
 // One CTA per (step, dim): the 2 x G per-CTA sums part[((t*2 + h)*D + d)*G + b] read
@@ -509,8 +519,24 @@ cudaError_t launch_init_uniform(float* xs, uint32_t D, uint64_t W, uint32_t seed
 
 cudaError_t launch_init_normal(float* xs, uint32_t D, uint64_t W, uint32_t seed, float mean,
                                float sd, cudaStream_t s) {
-    init_normal<<<grid_for((uint64_t)D * W, 256), 256, 0, s>>>(xs, D, W, seed, mean, sd);
+    const uint64_t n = (uint64_t)D * W;
+    init_normal<<<grid_for((n + 1) / 2, 256), 256, 0, s>>>(xs, n, seed, mean, sd);
     g_launches++;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_init_normal_members(float* xs, const bay_init_member* mem, uint32_t n,
+                                       uint64_t count_max, float mean, float sd, cudaStream_t s) {
+    // two pairs a thread of the largest member, up to some 32,768 CTAs over the members: with
+    // equal shares of 50 CTAs the largest of 48 members held the launch (479 us against 263)
+    const uint64_t want = (count_max / 2 + 511) / 512 + 1;
+    for (uint32_t m0 = 0; m0 < n; m0 += 32768u) {
+        const uint32_t nm = n - m0 < 32768u ? n - m0 : 32768u;
+        const uint32_t most = 32768u / nm < 4u ? 4u : 32768u / nm;
+        init_normal_members<<<dim3(want < most ? (uint32_t)want : most, nm), 256, 0, s>>>(xs, mem + m0,
+                                                                                       mean, sd);
+        g_launches++;
+    }
     return cudaGetLastError();
 }
 

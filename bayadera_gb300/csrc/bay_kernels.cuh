@@ -94,6 +94,12 @@ struct bay_mix_state {
     unsigned int pad;
 };
 
+// A batch member's positions: count floats at off, drawn with seed.
+struct bay_init_member {
+    unsigned long long off, count;
+    unsigned int seed, pad;
+};
+
 namespace bay {
 
 cudaError_t launch_ctl_apply(bay_ctl* ctl, const bay_ctl_op& op, cudaStream_t s);
@@ -101,6 +107,10 @@ cudaError_t launch_init_uniform(float* xs, uint32_t D, uint64_t W, uint32_t seed
                                 const float* limits, cudaStream_t s);
 cudaError_t launch_init_normal(float* xs, uint32_t D, uint64_t W, uint32_t seed, float mean,
                                float sd, cudaStream_t s);
+// The same for n blocks of xs, of count_max values at most, with a seed each (mem on the
+// device).
+cudaError_t launch_init_normal_members(float* xs, const bay_init_member* mem, uint32_t n,
+                                       uint64_t count_max, float mean, float sd, cudaStream_t s);
 // How an estimate kernel is spread: equal tiles of at most 256 dimensions, gx CTAs a tile
 // (kEstCtas CTAs at most unless the tiles alone are more).
 constexpr uint32_t kEstCtas = 608;        // 4 CTAs of 256 threads an SM

@@ -4,10 +4,11 @@
 // the model source in front.
 //
 // A half-step of every member is three launches over work lists the host builds once:
-//   propose: CTA = (member, 256-walker tile): Philox draw with the member's seed and the
+//   propose: CTA = (member, tile of at most 32 walkers): Philox draw with the member's seed and the
 //            single-sampler counter {k, step, stream, 0xbeeff00d}, stretch factor, partner
 //            from the member's other half, the proposal y -> scratch (coalesced over the
-//            tile's contiguous block), per-walker prep and the terms outside the row sum;
+//            tile's contiguous block) and shared memory, from which a thread per walker
+//            takes prep and the terms outside the row sum;
 //   rows:    CTA = (member, tile of wpc walkers, chunk of rows): the chunk of rows and the
 //            walkers' proposals are staged in shared memory, then each of 256 / wpc lanes
 //            per walker sums the row terms of its rows (walkers fastest, so a warp reads
@@ -16,8 +17,9 @@
 //            chunk).  wpc and the chunk size are chosen per member so that every item
 //            carries about the same work, which balances members whose data differ by
 //            orders of magnitude;
-//   accept:  CTA = (member, 256-walker tile): partials summed in chunk order, log-space
-//            accept (bay_accept_log), write-back; accu: accepted count per member, per-CTA per-dim sums.
+//   accept:  CTA = (member, 256-walker tile, slice of 32 coordinates): partials summed in
+//            chunk order, log-space accept (bay_accept_log), the slice's write-back; accu:
+//            accepted count per member, the tile's sums of the slice's coordinates.
 // Counter and key words per member are those of a single sampler with the member's seed,
 // so a member's trajectory is the trajectory that sampler would take (up to the order of
 // the log-density sums).
@@ -63,17 +65,20 @@ struct bay_bmember {
     unsigned int dim, W, K, hyper_len;
     unsigned int walker0;         // first walker of the member in the per-walker arrays
     unsigned int chunks, chunk_rows;
-    unsigned int tile0;           // first move tile (accept CTA) of the member
-    unsigned int ntiles;          // move tiles of the member
-    unsigned int pad[3];
+    unsigned int ntiles;          // 256-walker move tiles of the member
+    unsigned int pad[4];
 };
 struct bay_bitem { unsigned int m, k0, c, wpc; };   // rows work item
-struct bay_btile { unsigned int m, k0; };           // propose / accept CTA
+// propose CTA: n walkers from k0; accept CTA: 256 walkers from k0, 32 coordinates from n
+struct bay_btile { unsigned int m, k0, n, pad; };
+#define BAY_BT_W 256u             // walkers of an accept tile (and of its dim sums)
+#define BAY_BT_D 32u              // coordinates of an accept slice
 
 struct bay_batch_params {
     const bay_bmember* mem;
     const bay_bitem* items;
-    const bay_btile* tiles;
+    const bay_btile* ptiles;      // propose
+    const bay_btile* atiles;      // accept
     const unsigned int* seeds;    // [member][2]: bare, accu
     const float* params;
     float* xs;
@@ -81,7 +86,7 @@ struct bay_batch_params {
     float* logfn;                 // [walker0 + w]
     float* prep;                  // [walker0 + k][BAY_PREP_LEN]
     float* wterm;                 // [walker0 + k]
-    float* zu;                    // [walker0 + k][2]
+    float* zu;                    // [walker0 + k][3]: stretch factor, uniform, log density
     float* part;
     unsigned long long* accepted; // [member]
     float* dsum;                  // [step_off * 2 + half][dsum_stride]
@@ -89,10 +94,9 @@ struct bay_batch_params {
     bay_ctl* ctl;
     unsigned long long dsum_stride;
     unsigned int half, step_off, means_cap, n_members;
-    unsigned int n_tiles, n_items;  // move tiles and rows work items (the persistent launch)
+    unsigned int n_ptiles, n_items, n_atiles;   // work of each phase (the persistent launch)
     unsigned int gbar_extra;        // persistent launch: extra arrivals its barriers wait for
                                     // (0; 1 makes them run out, for tests)
-    unsigned int pad;
 };
 
 // log u <= (dim - 1) log z + beta (ly - lx) in fp32 with bay_log_det (bay_accept_log); a
@@ -146,17 +150,21 @@ __device__ __forceinline__ unsigned int bay_div_dim(unsigned int e, unsigned int
     return q;
 }
 
+// The tile's proposals in shared memory serve the model's walker terms, which read a whole
+// row per thread; from global memory, in 256-walker tiles, that chain of loads and the 130
+// elements per thread took 25 us for 48 members of up to 130 dimensions, now 7.9 us.
 template <int MODE>  // 0 bare, 1 accu, 2 log density of the current positions (all W)
 __device__ __forceinline__ void bay_batch_propose_impl(const bay_batch_params& P, unsigned int idx) {
-    __shared__ float sZ[256];
-    __shared__ unsigned int sJ[256];
-    const bay_btile T = P.tiles[idx];
+    extern __shared__ __align__(16) float bay_bsm[];
+    __shared__ float sZ[32];
+    __shared__ unsigned int sJ[32];
+    const bay_btile T = P.ptiles[idx];
     const bay_bmember& M = P.mem[T.m];
     const unsigned int nk = MODE == 2 ? M.W : M.K;
-    const unsigned int dim = M.dim;
+    const unsigned int dim = M.dim, dpad = dim | 1u;   // odd: the threads' rows in distinct banks
     const unsigned int tid = threadIdx.x;
     const unsigned int k = T.k0 + tid;
-    const unsigned int nt = nk - T.k0 < 256u ? nk - T.k0 : 256u;   // walkers of the tile
+    const unsigned int nt = nk - T.k0 < T.n ? nk - T.k0 : T.n;   // walkers of the tile
     const unsigned int kind = MODE == 1 ? 1u : 0u;
     if (MODE != 2 && tid < nt) {
         const unsigned int stream = MODE == 1 ? (P.half ? 2222u : 1111u) : (P.half ? 4444u : 3333u);
@@ -169,8 +177,10 @@ __device__ __forceinline__ void bay_batch_propose_impl(const bay_batch_params& P
         const float z = bay_stretch_z(P.ctl->a, bay_u01(r.y));
         sZ[tid] = z;
         sJ[tid] = bay_partner(bay_u01(r.x), M.K);
-        P.zu[2 * ((size_t)M.walker0 + k)] = z;
-        P.zu[2 * ((size_t)M.walker0 + k) + 1] = bay_u01(r.z);
+        float* zu = P.zu + 3 * ((size_t)M.walker0 + k);
+        zu[0] = z;
+        zu[1] = bay_u01(r.z);
+        zu[2] = P.logfn[(size_t)M.walker0 + (size_t)P.half * M.K + k];
     }
     __syncthreads();
     // the tile's proposals: one contiguous block of nt * dim floats, element-wise
@@ -184,16 +194,19 @@ __device__ __forceinline__ void bay_batch_propose_impl(const bay_batch_params& P
     // 8 elements per thread per pass, all their loads issued before any is used
     for (unsigned int e0 = tid; e0 < ne; e0 += 8u * blockDim.x) {
         float xv[8], sv[8], zv[8];
+        unsigned int at[8];
 #pragma unroll
         for (unsigned int i = 0; i < 8u; ++i) {
             const unsigned int e = e0 + i * blockDim.x;
             xv[i] = 0.0f;
             sv[i] = 0.0f;
             zv[i] = 0.0f;
+            at[i] = 0u;
             if (e < ne) {
+                const unsigned int w = bay_div_dim(e, dim, inv_dim), d = e - w * dim;
+                at[i] = w * dpad + d;
                 xv[i] = X[e];
                 if (MODE != 2) {
-                    const unsigned int w = bay_div_dim(e, dim, inv_dim), d = e - w * dim;
                     sv[i] = S[(size_t)sJ[w] * dim + d];
                     zv[i] = sZ[w];
                 }
@@ -202,12 +215,16 @@ __device__ __forceinline__ void bay_batch_propose_impl(const bay_batch_params& P
 #pragma unroll
         for (unsigned int i = 0; i < 8u; ++i) {
             const unsigned int e = e0 + i * blockDim.x;
-            if (e < ne) Y[e] = MODE == 2 ? xv[i] : __fmaf_rn(zv[i], __fsub_rn(xv[i], sv[i]), sv[i]);
+            if (e < ne) {
+                const float v = MODE == 2 ? xv[i] : __fmaf_rn(zv[i], __fsub_rn(xv[i], sv[i]), sv[i]);
+                Y[e] = v;
+                bay_bsm[at[i]] = v;
+            }
         }
     }
     __syncthreads();
     if (tid < nt) {
-        const float* y = Y + (size_t)tid * dim;
+        const float* y = bay_bsm + tid * dpad;
         const float* hyper = P.params + M.params + M.rows * BAY_ROW_LEN;
         float pr[BAY_PREP_LEN];
 #pragma unroll
@@ -217,6 +234,7 @@ __device__ __forceinline__ void bay_batch_propose_impl(const bay_batch_params& P
         for (int i = 0; i < BAY_PREP_LEN; ++i) P.prep[((size_t)M.walker0 + k) * BAY_PREP_LEN + i] = pr[i];
         P.wterm[(size_t)M.walker0 + k] = BAY_TILE_WALKER(M.rows, hyper, M.hyper_len, dim, y);
     }
+    __syncthreads();    // the persistent launch's next tile rewrites the shared rows
 }
 
 // WPT walkers per thread (1, 2 or 4): thread t serves walkers tw, tw + TPR, ..., tw + (WPT -
@@ -435,9 +453,16 @@ __device__ __forceinline__ void bay_batch_rows_impl(const bay_batch_params& P, u
     }
 }
 
+// Every slice's CTA decides for the tile's walkers (the current log density comes from the
+// proposal's scratch, so that the first slice's CTA may store the new one) and moves 32
+// coordinates of them: 32 elements per thread, all 256 rows' segments in whole sectors.  A
+// CTA per tile moved up to 130 elements per thread and, for the sums, walked 256 rows per
+// thread: 22 us bare, 35 us accu for 48 members, now 6.2 and 8.5 us.  The accu sums go over a staged copy: thread (coordinate,
+// group of 32 walkers), compensated in walker order, the eight groups combined in order.
 template <int MODE>  // 0 bare, 1 accu, 2 log density of the current positions
 __device__ __forceinline__ void bay_batch_accept_impl(const bay_batch_params& P, unsigned int idx) {
-    const bay_btile T = P.tiles[idx];
+    extern __shared__ __align__(16) float bay_bsm[];   // accu: [256][33] new positions
+    const bay_btile T = P.atiles[idx];
     const bay_bmember& M = P.mem[T.m];
     const unsigned int nk = MODE == 2 ? M.W : M.K;
     const unsigned int dim = M.dim, tid = threadIdx.x;
@@ -463,52 +488,76 @@ __device__ __forceinline__ void bay_batch_accept_impl(const bay_batch_params& P,
         if (MODE == 2) {
             P.logfn[wk] = ly;
         } else {
-            const size_t lk = (size_t)M.walker0 + (size_t)P.half * M.K + k;
-            accepted = bay_batch_accept(P.zu[2 * wk + 1], P.zu[2 * wk], ly, P.logfn[lk],
-                                        MODE == 1 ? 1.0f : P.ctl->beta, dim);
-            if (accepted) P.logfn[lk] = ly;
+            const float* zu = P.zu + 3 * wk;
+            accepted = bay_batch_accept(zu[1], zu[0], ly, zu[2], MODE == 1 ? 1.0f : P.ctl->beta, dim);
+            if (accepted && T.n == 0u)
+                P.logfn[(size_t)M.walker0 + (size_t)P.half * M.K + k] = ly;
         }
     }
     if (MODE == 2) return;
-    // the accepted walkers' rows, element-wise over the tile (coalesced, many in flight)
-    __shared__ unsigned char sAcc[256];
+    __shared__ unsigned char sAcc[BAY_BT_W];
     sAcc[tid] = accepted ? 1 : 0;
-    __syncthreads();
+    const int n_acc = __syncthreads_count(accepted);
+    const unsigned int nt = nk - T.k0 < BAY_BT_W ? nk - T.k0 : BAY_BT_W;
+    const unsigned int nd = dim - T.n < BAY_BT_D ? dim - T.n : BAY_BT_D;
+    const bool stats = MODE == 1 && P.means_cap != 0;
     {
-        const unsigned int nt = nk - T.k0 < blockDim.x ? nk - T.k0 : blockDim.x;
-        float* __restrict__ Xt = P.xs + M.xs + ((size_t)P.half * M.K + T.k0) * dim;
-        const float* __restrict__ Yt = P.y + M.xs + (size_t)T.k0 * dim;
-        const float inv_dim = __frcp_rn((float)dim);
-#pragma unroll 4
-        for (unsigned int e = tid; e < nt * dim; e += blockDim.x)
-            if (sAcc[bay_div_dim(e, dim, inv_dim)]) Xt[e] = Yt[e];
+        // lane: coordinate, warp: every 8th walker, 8 loads in flight
+        float* __restrict__ Xt = P.xs + M.xs + ((size_t)P.half * M.K + T.k0) * dim + T.n;
+        const float* __restrict__ Yt = P.y + M.xs + (size_t)T.k0 * dim + T.n;
+        const unsigned int d = tid & 31u;
+        for (unsigned int w0 = tid >> 5; w0 < nt; w0 += 64u) {
+            float v[8];
+            bool a[8];
+#pragma unroll
+            for (unsigned int i = 0; i < 8u; ++i) {
+                const unsigned int w = w0 + 8u * i;
+                a[i] = w < nt && sAcc[w];
+                v[i] = 0.0f;
+                if (w < nt && d < nd) {
+                    if (a[i]) v[i] = Yt[(size_t)w * dim + d];
+                    else if (stats) v[i] = Xt[(size_t)w * dim + d];
+                }
+            }
+#pragma unroll
+            for (unsigned int i = 0; i < 8u; ++i) {
+                const unsigned int w = w0 + 8u * i;
+                if (a[i] && d < nd) Xt[(size_t)w * dim + d] = v[i];
+                if (stats && w < nt) bay_bsm[w * 33u + d] = v[i];
+            }
+        }
     }
-    // the persistent launch runs the next tile's accept in this CTA: sAcc is rewritten
-    // there only after every thread has read it here
+    // (also: the persistent launch's next tile rewrites sAcc and the staged positions only
+    // after every thread has read them)
     __syncthreads();
     if (MODE != 1) return;
-    // accu: the member's accepted count and this CTA's per-dim sums of the moved walkers
-    const int n_acc = __syncthreads_count(accepted);
-    if (tid == 0 && n_acc) atomicAdd(&P.accepted[T.m], (unsigned long long)n_acc);
-    if (P.means_cap == 0) return;
-    const unsigned int nt = nk - T.k0 < blockDim.x ? nk - T.k0 : blockDim.x;
-    const float* Xc = P.xs + M.xs + ((size_t)P.half * M.K + T.k0) * dim;
-    float* out = P.dsum + ((size_t)P.step_off * 2 + P.half) * P.dsum_stride + M.dsum
-        + (size_t)(idx - M.tile0) * dim;
-    for (unsigned int d = tid; d < dim; d += blockDim.x) {
+    // accu: the member's accepted count and the tile's sums of the slice's coordinates
+    if (tid == 0 && T.n == 0u && n_acc) atomicAdd(&P.accepted[T.m], (unsigned long long)n_acc);
+    if (!stats) return;
+    __shared__ bay_bcf sGrp[8][32];
+    {
+        const unsigned int d = tid & 31u, g = tid >> 5;
         bay_bcf s;
         s.hi = 0.0f;
         s.lo = 0.0f;
-        // in walker order; unrolled so that several rows' loads are in flight
 #pragma unroll 8
-        for (unsigned int w = 0; w < nt; ++w) {
+        for (unsigned int w = 32u * g; w < nt && w < 32u * g + 32u; ++w) {
             bay_bcf y;
-            y.hi = Xc[(size_t)w * dim + d];
+            y.hi = bay_bsm[w * 33u + d];
             y.lo = 0.0f;
             s = bay_bcadd(s, y);
         }
-        out[d] = __fadd_rn(s.hi, s.lo);
+        sGrp[g][d] = s;
     }
+    __syncthreads();
+    if (tid < nd) {
+        bay_bcf s = sGrp[0][tid];
+#pragma unroll
+        for (unsigned int g = 1; g < 8u; ++g) s = bay_bcadd(s, sGrp[g][tid]);
+        P.dsum[((size_t)P.step_off * 2 + P.half) * P.dsum_stride + M.dsum
+               + (size_t)(T.k0 / BAY_BT_W) * dim + T.n + tid] = __fadd_rn(s.hi, s.lo);
+    }
+    __syncthreads();
 }
 
 // Per-step ensemble means of each member from the accu launches' per-CTA sums:
@@ -585,7 +634,7 @@ __device__ __forceinline__ void bay_batch_run_impl(bay_batch_params P, unsigned 
                 !bay_grid_sync(&P.ctl->gbar_count, &P.ctl->abort, &P.ctl->status, gridDim.x, ++k,
                                P.gbar_extra))
                 return;
-            for (unsigned int t = blockIdx.x; t < P.n_tiles; t += gridDim.x)
+            for (unsigned int t = blockIdx.x; t < P.n_ptiles; t += gridDim.x)
                 bay_batch_propose_impl<MODE>(P, t);
             if (!bay_grid_sync(&P.ctl->gbar_count, &P.ctl->abort, &P.ctl->status, gridDim.x, ++k,
                                P.gbar_extra))
@@ -595,7 +644,7 @@ __device__ __forceinline__ void bay_batch_run_impl(bay_batch_params P, unsigned 
             if (!bay_grid_sync(&P.ctl->gbar_count, &P.ctl->abort, &P.ctl->status, gridDim.x, ++k,
                                P.gbar_extra))
                 return;
-            for (unsigned int t = blockIdx.x; t < P.n_tiles; t += gridDim.x)
+            for (unsigned int t = blockIdx.x; t < P.n_atiles; t += gridDim.x)
                 bay_batch_accept_impl<MODE>(P, t);
         }
     }
