@@ -183,15 +183,80 @@ struct bay_ctx {
 
     void* alloc(size_t bytes) {
         if (bytes == 0) bytes = 16;
-        if (mem_limit && allocated + bytes > mem_limit)
+        if (over_limit(bytes)) give_back();
+        if (over_limit(bytes))
             fail(BAY_ERR_ALLOC, "device memory limit of the context exceeded (" +
                                     std::to_string(allocated + bytes) + " > " +
                                     std::to_string(mem_limit) + " bytes)");
         void* p = nullptr;
-        cuda_check(cudaMalloc(&p, bytes), "cudaMalloc");
+        if (cudaMalloc(&p, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            give_back();
+            cuda_check(cudaMalloc(&p, bytes), "cudaMalloc");
+        }
         allocated += bytes;
         sizes[p] = bytes;
         return p;
+    }
+    bool over_limit(size_t bytes) const { return mem_limit && allocated + bytes > mem_limit; }
+
+    // Device memory for the length of one call (arguments staged from the host, work copies):
+    // a cudaMalloc and a cudaFree, which waits for the device, cost some tens of us each, so
+    // up to kScratchMax bytes of it are kept with the context, as much as a call has needed
+    // before.  Blocks are cut off in order and the whole is free again when the last is
+    // returned.  Calls hold the context's lock and finish on its stream before they return a
+    // block.  What does not fit, or not under mem_limit, is allocated for the call alone; an
+    // allocation that finds no room takes the idle scratch back.
+    static constexpr size_t kScratchMax = 64u << 20;
+    char* sc_base = nullptr;
+    size_t sc_cap = 0, sc_used = 0, sc_want = 0, sc_total = 0;
+    uint32_t sc_live = 0;
+    void* scratch(size_t bytes) {
+        bytes = (bytes + 255) & ~(size_t)255;
+        if (bytes == 0) bytes = 256;
+        if (sc_live == 0) sc_total = 0;
+        sc_total += bytes;
+        if (sc_live == 0 && sc_want > sc_cap) {
+            give_back();
+            if (!over_limit(sc_want)) {
+                void* p = nullptr;
+                if (cudaMalloc(&p, sc_want) == cudaSuccess) {
+                    sc_base = (char*)p;
+                    sc_cap = sc_want;
+                    allocated += sc_cap;
+                } else {
+                    cudaGetLastError();
+                }
+            }
+        }
+        if (sc_total <= kScratchMax) sc_want = std::max(sc_want, sc_total);
+        if (sc_used + bytes <= sc_cap) {
+            void* p = sc_base + sc_used;
+            sc_used += bytes;
+            ++sc_live;
+            return p;
+        }
+        return alloc(bytes);
+    }
+    void unscratch(void* p) {
+        if (!p) return;
+        if ((char*)p >= sc_base && (char*)p < sc_base + sc_cap) {
+            if (--sc_live == 0) sc_used = 0;
+        } else {
+            release(p);
+        }
+    }
+    // the kept memory that no call is using, back to the device
+    void give_back() {
+        if (sc_live == 0 && sc_base) {
+            cudaFree(sc_base);
+            allocated -= sc_cap;
+            sc_base = nullptr;
+            sc_cap = sc_used = 0;
+        }
+        release(est_ws);
+        est_ws = nullptr;
+        est_ws_bytes = 0;
     }
     void release(void* p) {
         if (!p) return;
@@ -823,6 +888,7 @@ int bay_ctx_release(bay_ctx* c) {
         c->use();
         cudaStreamSynchronize(c->stream);
         for (auto& kv : c->sizes) cudaFree(kv.first);
+        if (c->sc_base) cudaFree(c->sc_base);
         if (c->direct_lib) g_cu.LibraryUnload(c->direct_lib);
         for (auto& kv : c->hist_fastdiv) g_cu.LibraryUnload(kv.second.first);
         if (c->own_stream) cudaStreamDestroy(c->stream);
@@ -1518,7 +1584,7 @@ int bay_init_position_limits(bay_sampler* s, uint32_t seed, const float* limits)
         if (!s || !limits) fail(BAY_ERR_ARG, "NULL argument");
         std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
         s->ctx->use();
-        float* dl = (float*)s->ctx->alloc(sizeof(float) * 2 * s->D);
+        float* dl = (float*)s->ctx->scratch(sizeof(float) * 2 * s->D);
         try {
             cuda_check(cudaMemcpyAsync(dl, limits, sizeof(float) * 2 * s->D, cudaMemcpyDefault,
                                        s->ctx->stream),
@@ -1528,10 +1594,11 @@ int bay_init_position_limits(bay_sampler* s, uint32_t seed, const float* limits)
             s->launch_logfn_all();
             cuda_check(cudaStreamSynchronize(s->ctx->stream), "sync");
         } catch (...) {
-            s->ctx->release(dl);
+            cudaStreamSynchronize(s->ctx->stream);
+            s->ctx->unscratch(dl);
             throw;
         }
-        s->ctx->release(dl);
+        s->ctx->unscratch(dl);
         s->positioned = true;
         s->iteration_counter = 0;
     });
@@ -1695,8 +1762,9 @@ uint32_t acor_lag(uint64_t n, uint32_t wgs) {
     return (uint32_t)(l < 10 ? 10 : l);
 }
 
-// acor of a device-resident series; results to host or device arrays.
-int acor_device(bay_ctx* c, const float* d_series, uint32_t D, uint64_t n, double* tau,
+// acor of a device-resident series -- value t of dimension d at t * D + d, or with rows at
+// d * n + t -- results to host or device arrays.
+int acor_device(bay_ctx* c, const float* d_series, uint32_t D, uint64_t n, bool rows, double* tau,
                 double* mean, double* sigma, uint32_t* lag_out) {
     const uint32_t lag = acor_lag(n, c->wgs);
     if (lag_out) *lag_out = lag;
@@ -1706,21 +1774,22 @@ int acor_device(bay_ctx* c, const float* d_series, uint32_t D, uint64_t n, doubl
         return BAY_ERR_ARG;
     }
     if (n > 0xffffffffull) fail(BAY_ERR_ARG, "series too long");
-    double* work = (double*)c->alloc(sizeof(double) * ((size_t)D * n + 3 * D));
+    double* work = (double*)c->scratch(sizeof(double) * ((size_t)D * n + 3 * D));
     try {
         double* res = work + (size_t)D * n;
-        cuda_check(bay::launch_acor(d_series, D, (uint32_t)n, c->wgs, lag, work, res, res + D,
-                                    res + 2 * D, c->stream),
+        cuda_check(bay::launch_acor(d_series, D, (uint32_t)n, rows ? 1 : D, rows ? n : 1, c->wgs, lag,
+                                    work, res, res + D, res + 2 * D, c->stream),
                    "acor");
         if (tau) cuda_check(cudaMemcpyAsync(tau, res, sizeof(double) * D, cudaMemcpyDefault, c->stream), "copy");
         if (mean) cuda_check(cudaMemcpyAsync(mean, res + D, sizeof(double) * D, cudaMemcpyDefault, c->stream), "copy");
         if (sigma) cuda_check(cudaMemcpyAsync(sigma, res + 2 * D, sizeof(double) * D, cudaMemcpyDefault, c->stream), "copy");
         cuda_check(cudaStreamSynchronize(c->stream), "sync");
     } catch (...) {
-        c->release(work);
+        cudaStreamSynchronize(c->stream);
+        c->unscratch(work);
         throw;
     }
-    c->release(work);
+    c->unscratch(work);
     return BAY_OK;
 }
 }  // namespace
@@ -1857,7 +1926,7 @@ int bay_run_sampler(bay_sampler* s, uint64_t n, float a, bay_run_result* res, do
                        "cudaMemcpy(means)");
         uint32_t lag = 0;
         const std::string keep = g_err;
-        res->acor_status = acor_device(s->ctx, s->means, s->D, n, tau, mean, sigma, &lag);
+        res->acor_status = acor_device(s->ctx, s->means, s->D, n, false, tau, mean, sigma, &lag);
         if (res->acor_status == BAY_OK) g_err = keep;
         res->lag = lag;
         cuda_check(cudaStreamSynchronize(s->ctx->stream), "sync");
@@ -1986,8 +2055,8 @@ int bay_histogram(bay_sampler* s, uint32_t cycles, uint32_t bins, uint32_t flags
     });
 }
 
-int bay_acor(bay_ctx* c, const float* series, uint32_t D, uint64_t n, double* tau, double* mean,
-             double* sigma, uint32_t* lag) {
+static int acor_any(bay_ctx* c, const float* series, uint32_t D, uint64_t n, bool rows, double* tau,
+                    double* mean, double* sigma, uint32_t* lag) {
     NvtxRange trace_("bay_acor");
     int rc = BAY_OK;
     const int g = guarded([&] {
@@ -1996,22 +2065,34 @@ int bay_acor(bay_ctx* c, const float* series, uint32_t D, uint64_t n, double* ta
         std::lock_guard<std::recursive_mutex> lk(c->mu);
         c->use();
         if (is_device_ptr(series, c->device)) {
-            rc = acor_device(c, series, D, n, tau, mean, sigma, lag);
+            rc = acor_device(c, series, D, n, rows, tau, mean, sigma, lag);
             return;
         }
-        float* d = (float*)c->alloc(sizeof(float) * (size_t)D * std::max<uint64_t>(n, 1));
+        float* d = (float*)c->scratch(sizeof(float) * (size_t)D * std::max<uint64_t>(n, 1));
         try {
             cuda_check(cudaMemcpyAsync(d, series, sizeof(float) * (size_t)D * n,
                                        cudaMemcpyHostToDevice, c->stream),
                        "cudaMemcpy(series)");
-            rc = acor_device(c, d, D, n, tau, mean, sigma, lag);
+            rc = acor_device(c, d, D, n, rows, tau, mean, sigma, lag);
         } catch (...) {
-            c->release(d);
+            cudaStreamSynchronize(c->stream);
+            c->unscratch(d);
             throw;
         }
-        c->release(d);
+        if (rc != BAY_OK) cudaStreamSynchronize(c->stream);   // the copy, nothing waited for it
+        c->unscratch(d);
     });
     return g != BAY_OK ? g : rc;
+}
+
+int bay_acor(bay_ctx* c, const float* series, uint32_t D, uint64_t n, double* tau, double* mean,
+             double* sigma, uint32_t* lag) {
+    return acor_any(c, series, D, n, false, tau, mean, sigma, lag);
+}
+
+int bay_acor_rows(bay_ctx* c, const float* series, uint32_t D, uint64_t n, double* tau, double* mean,
+                  double* sigma, uint32_t* lag) {
+    return acor_any(c, series, D, n, true, tau, mean, sigma, lag);
 }
 
 // Allocation-free acor for callers that cannot allocate device memory at call time:
@@ -2039,7 +2120,7 @@ int bay_acor_noalloc(bay_ctx* c, const float* d_series, uint32_t D, uint64_t n, 
         c->use();
         double* work = c->acor_scratch;
         double* res = work + (size_t)D * n;
-        cuda_check(bay::launch_acor(d_series, D, (uint32_t)n, c->wgs, lag, work, res, res + D,
+        cuda_check(bay::launch_acor(d_series, D, (uint32_t)n, D, 1, c->wgs, lag, work, res, res + D,
                                     res + 2 * D, c->stream),
                    "acor");
         if (tau) cuda_check(cudaMemcpyAsync(tau, res, sizeof(double) * D, cudaMemcpyDefault, c->stream), "copy");

@@ -403,8 +403,8 @@ __device__ void acor_pass(cooperative_groups::cluster_group& cl, acor_shared& sh
 }
 
 __global__ void __launch_bounds__(kAcorThreads)
-acor_kernel(const float* series, uint32_t D, uint32_t n, uint32_t wgs, uint32_t lag, double* work,
-            double* tau_out, double* mean_out, double* sigma_out) {
+acor_kernel(const float* series, uint32_t n, uint64_t st, uint64_t sd, uint32_t wgs, uint32_t lag,
+            double* work, double* tau_out, double* mean_out, double* sigma_out) {
     __shared__ acor_shared sh;
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     const uint32_t C = cl.num_blocks(), me = cl.block_rank();
@@ -417,7 +417,7 @@ acor_kernel(const float* series, uint32_t D, uint32_t n, uint32_t wgs, uint32_t 
     for (uint64_t t = first; t < n; t += U * step) {
         float v[U];
 #pragma unroll
-        for (uint32_t i = 0; i < U; ++i) v[i] = t + i * step < n ? __ldg(&series[(t + i * step) * D + d]) : 0.0f;
+        for (uint32_t i = 0; i < U; ++i) v[i] = t + i * step < n ? __ldg(&series[(t + i * step) * st + d * sd]) : 0.0f;
 #pragma unroll
         for (uint32_t i = 0; i < U; ++i)
             if (t + i * step < n) sum[0] += (double)v[i];
@@ -427,7 +427,7 @@ acor_kernel(const float* series, uint32_t D, uint32_t n, uint32_t wgs, uint32_t 
     for (uint64_t t = first; t < n; t += U * step) {
         float v[U];
 #pragma unroll
-        for (uint32_t i = 0; i < U; ++i) v[i] = t + i * step < n ? __ldg(&series[(t + i * step) * D + d]) : 0.0f;
+        for (uint32_t i = 0; i < U; ++i) v[i] = t + i * step < n ? __ldg(&series[(t + i * step) * st + d * sd]) : 0.0f;
 #pragma unroll
         for (uint32_t i = 0; i < U; ++i)
             if (t + i * step < n) m[t + i * step] = (double)v[i] - mu;
@@ -579,8 +579,9 @@ cudaError_t launch_gemm_tc_image(const float* A, uint64_t ld, uint32_t rows, uin
     return cudaGetLastError();
 }
 
-cudaError_t launch_acor(const float* series, uint32_t D, uint32_t n, uint32_t wgs, uint32_t lag,
-                        double* work, double* tau, double* mean, double* sigma, cudaStream_t s) {
+cudaError_t launch_acor(const float* series, uint32_t D, uint32_t n, uint64_t st, uint64_t sd,
+                        uint32_t wgs, uint32_t lag, double* work, double* tau, double* mean,
+                        double* sigma, cudaStream_t s) {
     // a CTA of the cluster for every 1,024 entries, a power of two up to 16 (8 where the
     // device takes no cluster of 16)
     cudaLaunchAttribute at[1];
@@ -608,8 +609,8 @@ cudaError_t launch_acor(const float* series, uint32_t D, uint32_t n, uint32_t wg
     }
     at[0].val.clusterDim.x = C;
     cfg.gridDim = dim3(D * C);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, acor_kernel, series, D, n, wgs, lag, work, tau, mean,
-                                             sigma);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, acor_kernel, series, n, st, sd, wgs, lag, work, tau,
+                                             mean, sigma);
     if (e != cudaSuccess) return e;
     g_launches++;
     return cudaGetLastError();

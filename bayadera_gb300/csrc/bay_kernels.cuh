@@ -161,9 +161,11 @@ cudaError_t launch_gemm_tc_image(const float* A, uint64_t ld, uint32_t rows, uin
 cudaError_t launch_reduce_means(const bay_ctl* ctl, const float* part, float* means,
                                 uint32_t means_cap, uint32_t G, uint32_t D, uint32_t nsteps,
                                 double inv_W, cudaStream_t s);
-// acor of a D x n column-major series (series[t*D + d]); work holds D*n doubles.
-cudaError_t launch_acor(const float* series, uint32_t D, uint32_t n, uint32_t wgs, uint32_t lag,
-                        double* work, double* tau, double* mean, double* sigma, cudaStream_t s);
+// acor of D series of n values, value t of series d at series[t * st + d * sd]; work holds
+// D * n doubles.
+cudaError_t launch_acor(const float* series, uint32_t D, uint32_t n, uint64_t st, uint64_t sd,
+                        uint32_t wgs, uint32_t lag, double* work, double* tau, double* mean,
+                        double* sigma, cudaStream_t s);
 // Fixed scratch of bay_acor_noalloc: dim * n + 3 * dim doubles at most (8 MiB).
 #define BAY_ACOR_NOALLOC_MAX_DOUBLES (1u << 20)
 // Device address of that scratch on the current device (cudaGetSymbolAddress; loads the

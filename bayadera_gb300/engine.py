@@ -41,12 +41,13 @@ class GB300AcorEngine:
         if m.ndim == 1:
             m = m[None, :]
         dim, n = m.shape
-        series = np.ascontiguousarray(m.T)  # column-major dim x n
+        by_dim = m.flags.c_contiguous       # either order goes to the device as it lies
+        series = m if by_dim else np.ascontiguousarray(m.T)
         tau = np.zeros(dim)
         mean = np.zeros(dim)
         sigma = np.zeros(dim)
         lag = C.c_uint32(0)
-        N.call("bay_acor", self.factory.ctx, _ptr(series), dim, n, _ptr(tau), _ptr(mean),
+        N.call("bay_acor_rows" if by_dim else "bay_acor", self.factory.ctx, _ptr(series), dim, n, _ptr(tau), _ptr(mean),
                _ptr(sigma), C.byref(lag))
         return Autocorrelation(tau, mean, sigma, n, lag.value)
 

@@ -64,7 +64,8 @@ int bay_ctx_release(bay_ctx* ctx);
 int bay_ctx_processing_elements(bay_ctx* ctx, uint64_t* out);
 int bay_ctx_stream(bay_ctx* ctx, void** stream);
 int bay_ctx_synchronize(bay_ctx* ctx);
-/* Bytes currently allocated by this context. */
+/* Bytes currently allocated by this context (with the workspaces it keeps between calls: at
+ * most 64 MiB and the estimates' partial results, given back when an allocation needs room). */
 int bay_ctx_allocated(bay_ctx* ctx, uint64_t* out);
 /* Kernels this library has enqueued in this process, all contexts (each replayed graph
  * counts its kernel nodes).  No reference counterpart: an instrumentation counter. */
@@ -295,6 +296,10 @@ int bay_histogram(bay_sampler* s, uint32_t cycles, uint32_t bins, uint32_t flags
  * BAY_ERR_ARG if n < 5 lag. */
 int bay_acor(bay_ctx* ctx, const float* series, uint32_t dim, uint64_t n, double* tau,
              double* mean, double* sigma, uint32_t* lag);
+/* The same for a series stored by dimension (dim rows of n values: a dim x n row-major
+ * matrix), read where it lies. */
+int bay_acor_rows(bay_ctx* ctx, const float* series, uint32_t dim, uint64_t n, double* tau,
+                  double* mean, double* sigma, uint32_t* lag);
 
 /* acor that allocates nothing.  No counterpart in the reference: it is for callers
  * that may not allocate device memory when they call -- for instance a host that runs

@@ -112,3 +112,31 @@ def test_acor_matches_oracle_at_the_split_edges(oracle, n, wgs, rho):
     assert np.allclose(got.tau, tau, rtol=1e-11, atol=0)
     assert np.allclose(got.sigma, sigma, rtol=1e-11, atol=0, equal_nan=True)
     assert np.allclose(got.mean, mean, rtol=0, atol=1e-13 * np.abs(x).max())
+
+
+def test_scratch_is_kept_bounded_and_given_back(oracle):
+    """The kept call scratch: repeated calls of mixed sizes give the same results, it stays
+    below its bound, and a context at its memory limit gets it back for a sampler."""
+    from bayadera_gb300 import models as M
+    from bayadera_gb300.engine import GB300BayaderaFactory
+    rng = np.random.default_rng(3)
+    small = rng.standard_normal((2, 500)).astype(np.float32)
+    large = rng.standard_normal((2, 4_000_000)).astype(np.float32)      # 96 MB of work
+    with GB300BayaderaFactory() as f:
+        first = [f.acor(m).tau for m in (small, large, small)]
+        for _ in range(2):
+            for m, t in zip((small, large, small), first):
+                assert np.array_equal(f.acor(m).tau, t)
+                assert np.array_equal(f.acor(np.asfortranarray(m)).tau, t)
+        assert f.allocated() <= (64 << 20) + (3 << 20)
+    limit = 24 << 20
+    with GB300BayaderaFactory(mem_limit=limit) as f:
+        mid = rng.standard_normal((2, 500_000)).astype(np.float32)      # 4 MB + 8 MB
+        for _ in range(3):
+            f.acor(mid)
+        assert f.allocated() > 8 << 20
+        sf = f.mcmc_factory(M.mvn_precision_model(40), form="plain")
+        s = sf.create_sampler(1, 131072, np.eye(40, dtype=np.float32).reshape(-1))   # 21 MB
+        assert f.allocated() <= limit
+        s.release()
+        sf.release()
