@@ -359,6 +359,9 @@ constexpr size_t kTcSmemMax = 232448;  // opt-in dynamic shared memory per CTA, 
 constexpr size_t kBatchSmemMax = 160 * 1024;   // batched rows kernels: dynamic shared memory, at most
 constexpr uint32_t kTrWalkers = 64;  // walkers per tile of the resident tensor-core form
 constexpr uint32_t kTrGroups = 4;    // tile groups (256 threads each) per persistent CTA
+// With one sub-tile and at most 256 features the kernel holds the walker operand in tensor
+// memory (BAY_TC_ATM), which leaves its shared memory to more stages: the free choice is up to
+// 6 there too; which shapes may be asked for stays as if it were in shared memory.
 // want_g / want_s (0 = free) ask for a shape; false when no shape fits (or the asked one
 // does not).
 bool tc_plan(uint32_t features, uint32_t aux_len, uint32_t* G, uint32_t* S, size_t* smem,
@@ -366,16 +369,16 @@ bool tc_plan(uint32_t features, uint32_t aux_len, uint32_t* G, uint32_t* S, size
     const size_t kc = (features + 63) / 64, auxs = aux_len ? aux_len : 1;
     for (uint32_t g = 2; g >= 1; --g) {
         if (want_g && g != want_g) continue;
-        const size_t fixed = (size_t)g * kc * 32768 + 2 * 128 * auxs * sizeof(float) + 1024 + 256;
+        const size_t rest = 2 * 128 * auxs * sizeof(float) + 1024 + 256;
+        const size_t fixed = (size_t)g * kc * 32768 + rest;
         if (fixed + 2 * 32768 > kTcSmemMax) continue;
         size_t st = std::min<size_t>(6, (kTcSmemMax - fixed) / 32768);
-        if (want_s) {
-            if (want_s < 2 || want_s > st) return false;
-            st = want_s;
-        }
+        if (want_s && (want_s < 2 || want_s > st)) return false;
+        const size_t held = g == 1 && kc <= 4 ? rest : fixed;
+        st = want_s ? want_s : std::min<size_t>(6, (kTcSmemMax - held) / 32768);
         *G = g;
         *S = (uint32_t)st;
-        *smem = fixed + st * 32768;
+        *smem = held + st * 32768;
         return true;
     }
     return false;

@@ -158,4 +158,38 @@ __device__ __forceinline__ bay_v4 bay_v4_sub_rn(bay_v4 a, bay_v4 b) {
     return {__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z), __fsub_rn(a.w, b.w)};
 }
 
+// Two floats in a 64-bit register pair: one instruction for both (the same fp32 rate as two,
+// half the issue slots).  Lane-wise IEEE operations, flushing like the module's scalar ones.
+typedef unsigned long long bay_f2;
+__device__ __forceinline__ bay_f2 bay_f2_of(float x, float y) {
+    bay_f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float bay_f2_x(bay_f2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+    return x;
+}
+__device__ __forceinline__ float bay_f2_y(bay_f2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+    return y;
+}
+__device__ __forceinline__ bay_f2 bay_f2_add(bay_f2 a, bay_f2 b) {
+    bay_f2 r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ bay_f2 bay_f2_mul(bay_f2 a, bay_f2 b) {
+    bay_f2 r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ bay_f2 bay_f2_fma(bay_f2 a, bay_f2 b, bay_f2 c) {
+    bay_f2 r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 #endif

@@ -843,13 +843,17 @@ extern "C" __global__ void __launch_bounds__(256) bay_gemm_accept_logfn(bay_stre
 // and three products (hi.hi + hi.lo + lo.hi) accumulated in fp32 in tensor memory; the
 // dropped lo.lo product is below 2^-16 of each term.  tcgen05.mma kind::f16 with
 // M = 128 walkers (TMEM lanes), N = 128 rows (TMEM columns), K = 16 per instruction,
-// both operands K-major in shared memory with the 128-byte swizzle TMA writes.
+// the rows K-major in shared memory with the 128-byte swizzle TMA writes, the walkers the
+// same or in tensor memory (BAY_TC_ATM).
 // CTA roles: warp 0 -- TMA producer (the CTA's walker operand once, then each 128-row
 // tile in 64-feature chunks through a ring of BAY_TC_STAGES stages); warp 1 -- TMEM
 // allocation and the MMA issue (one thread); warps 2 .. 17 -- epilogue, a thread per
 // walker and share of a tile's rows: tcgen05.ld of its TMEM lane, the model's row terms,
-// a compensated sum over the super-block's rows.  Two accumulator buffers in TMEM let the MMAs of
-// tile t + 1 run under the epilogue of tile t.  Every wait is bounded in time; a wait
+// a compensated sum over the super-block's rows.  A model may give the terms of 16 rows at
+// once (BAY_GEMM_TERMS16: their sum, and BAY_GEMM_CARRY_LEN values that a thread carries over
+// its rows, whose contribution BAY_GEMM_CARRY_END adds at the end as hi + lo); rows past the
+// last whole batch of 16 take the term by itself.  Two accumulator buffers in TMEM let the
+// MMAs of tile t + 1 run under the epilogue of tile t.  Every wait is bounded in time; a wait
 // that gives up sets the sampler's status word and the CTA's abort flag, and the CTA
 // drains its own copies and MMAs, frees its TMEM and exits.
 #ifndef BAY_TC_G
@@ -861,12 +865,32 @@ extern "C" __global__ void __launch_bounds__(256) bay_gemm_accept_logfn(bay_stre
 #define BAY_TC_FP ((BAY_GEMM_F + 63) / 64 * 64)
 #define BAY_TC_KC (BAY_TC_FP / 64)
 #define BAY_TC_TILE 16384u                      // one 128 x 64 bf16 operand chunk
-#define BAY_TC_WBYTES ((unsigned int)BAY_TC_G * BAY_TC_KC * 2u * BAY_TC_TILE)
+// With one sub-tile and up to 256 features the walker operand lies in tensor memory (hi and
+// lo of a 64-feature chunk in 32 columns each, after the two accumulator buffers; 512 columns
+// in all).  From shared memory an M = N = 128 MMA reads 4 KB of each operand per 64 clocks,
+// the 128 bytes a clock that shared memory delivers, and the copies of the next rows come on
+// top: the tensor pipe could be busy 75 % of the time, and was (1.13 ms for 2,048 walkers x
+// 524,589 rows x 256 features).  Two sub-tiles leave no columns for it (and share the rows).
+#define BAY_TC_ATM (BAY_TC_G == 1 && BAY_TC_KC <= 4)
+#define BAY_TC_WBYTES (BAY_TC_ATM ? 0u : (unsigned int)BAY_TC_G * BAY_TC_KC * 2u * BAY_TC_TILE)
 #define BAY_TC_SBYTES (2u * BAY_TC_TILE)        // a stage: rows hi + lo chunk
 #define BAY_TC_AUXF (128u * BAY_AUXS)
 #define BAY_TC_NEPI 512u                        // epilogue threads (16 warps)
 #define BAY_TC_THREADS 576
-#define BAY_TC_COLS (BAY_TC_G == 2 ? 512u : 256u)
+// Order of a 64-feature chunk's products in the accumulator.  The tensor core cuts sums off
+// (toward zero), so that every product added to the large sum takes some 2^-25 of it: with a
+// model that sums its rows' terms exactly enough to show it, the small products come first.
+#ifdef BAY_GEMM_TERMS16
+#define BAY_TC_LO_FIRST 1
+#else
+#define BAY_TC_LO_FIRST 0
+#endif
+#ifdef BAY_GEMM_TERMS16
+#define BAY_TC_EPI_UNROLL 2     // its arithmetic bounds the launch: logistic 2.79 -> 2.52 ms
+#else
+#define BAY_TC_EPI_UNROLL 1     // (tensor-bound: robust_t 0.96 ms a launch, 0.975 unrolled)
+#endif
+#define BAY_TC_COLS (BAY_TC_G == 2 || BAY_TC_ATM ? 512u : 256u)
 #define BAY_TC_WAIT_NS 2000000000ull
 // instruction descriptor: fp32 accumulator, bf16 A and B, both K-major, N = 128, M = 128
 #define BAY_TC_IDESC ((1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24))
@@ -942,6 +966,26 @@ __device__ __forceinline__ void bay_mma(unsigned int d, unsigned long long a, un
         " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
         ::"r"(d), "l"(a), "l"(b), "r"(BAY_TC_IDESC), "r"(acc) : "memory");
 }
+// the A operand in tensor memory: lane = row, two consecutive K elements per column
+__device__ __forceinline__ void bay_mma_ta(unsigned int d, unsigned int a, unsigned long long b,
+                                           unsigned int acc) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+        ::"r"(d), "r"(a), "l"(b), "r"(BAY_TC_IDESC), "r"(acc) : "memory");
+}
+// 128 bytes -> 32 consecutive TMEM columns of this thread's lane
+__device__ __forceinline__ void bay_tmem_st32(unsigned int ta, const uint4 (&v)[8]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+        "%11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, "
+        "%29, %30, %31, %32};"
+        ::"r"(ta), "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"(v[1].x), "r"(v[1].y),
+        "r"(v[1].z), "r"(v[1].w), "r"(v[2].x), "r"(v[2].y), "r"(v[2].z), "r"(v[2].w), "r"(v[3].x),
+        "r"(v[3].y), "r"(v[3].z), "r"(v[3].w), "r"(v[4].x), "r"(v[4].y), "r"(v[4].z), "r"(v[4].w),
+        "r"(v[5].x), "r"(v[5].y), "r"(v[5].z), "r"(v[5].w), "r"(v[6].x), "r"(v[6].y), "r"(v[6].z),
+        "r"(v[6].w), "r"(v[7].x), "r"(v[7].y), "r"(v[7].z), "r"(v[7].w) : "memory");
+}
 __device__ __forceinline__ void bay_mma_commit(unsigned int bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                  ::"r"(bar) : "memory");
@@ -984,7 +1028,7 @@ __device__ __forceinline__ void bay_gemm_rows_tc_impl(const bay_stretch_params& 
     const unsigned int b_full = bar0, b_empty = bar0 + 8u * BAY_TC_STAGES;
     const unsigned int b_tfull = bar0 + 16u * BAY_TC_STAGES, b_tempty = b_tfull + 16u;
     const unsigned int b_wop = b_tempty + 16u, b_drain = b_wop + 8u;
-    // flags: [0] TMEM base, [1] abort, [2], [3] epilogue go flags of the two buffers
+    // flags: [0] TMEM base, [1] abort, [2 + 2 set + buffer] epilogue go flags
     volatile unsigned int* abort = flags + 1;
     unsigned int* status = &P.ctl->status;
 
@@ -1006,7 +1050,7 @@ __device__ __forceinline__ void bay_gemm_rows_tc_impl(const bay_stretch_params& 
             bay_mbar_init(b_tfull + 8u * b, 1u);
             bay_mbar_init(b_tempty + 8u * b, BAY_TC_NEPI / 32u);
         }
-        bay_mbar_init(b_wop, 1u);
+        bay_mbar_init(b_wop, BAY_TC_ATM ? BAY_TC_NEPI / 32u : 1u);
         bay_mbar_init(b_drain, 1u);
         flags[1] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1026,8 +1070,8 @@ __device__ __forceinline__ void bay_gemm_rows_tc_impl(const bay_stretch_params& 
     if (warp == 0) {
         if (lane == 0) {
             // ---- TMA producer
-            bay_expect_tx(b_wop, BAY_TC_WBYTES);
-            for (unsigned int g = 0; g < BAY_TC_G; ++g)
+            if (!BAY_TC_ATM) bay_expect_tx(b_wop, BAY_TC_WBYTES);
+            for (unsigned int g = 0; g < (BAY_TC_ATM ? 0u : BAY_TC_G); ++g)
                 for (unsigned int c = 0; c < BAY_TC_KC; ++c) {
                     const unsigned int dst = s_wop + ((g * BAY_TC_KC + c) * 2u) * BAY_TC_TILE;
                     bay_tma2d(dst, T.bh, (int)(c * 64u), (int)(k0 + g * 128u), b_wop);
@@ -1075,17 +1119,33 @@ __device__ __forceinline__ void bay_gemm_rows_tc_impl(const bay_stretch_params& 
 #pragma unroll
                     for (unsigned int g = 0; g < BAY_TC_G; ++g) {
                         const unsigned int wa = s_wop + ((g * BAY_TC_KC + c) * 2u) * BAY_TC_TILE;
+                        const unsigned int d = d0 + g * 128u;
+                        // the three products of K step ks
+                        auto product = [&](unsigned int ks, unsigned int which, unsigned int acc) {
+                            const unsigned long long x =
+                                bay_sdesc(xs + (which == 1u ? BAY_TC_TILE : 0u) + 32u * ks);   // hi.lo: rows' lo
+#if BAY_TC_ATM
+                            bay_mma_ta(d, tmem + 256u + 64u * c + (which == 2u ? 32u : 0u) + 8u * ks, x, acc);
+#else
+                            bay_mma(d, bay_sdesc(wa + (which == 2u ? BAY_TC_TILE : 0u) + 32u * ks), x, acc);
+#endif
+                        };
+#if BAY_TC_LO_FIRST
 #pragma unroll
                         for (unsigned int ks = 0; ks < 4u; ++ks) {
-                            const unsigned long long ah = bay_sdesc(wa + 32u * ks);
-                            const unsigned long long al = bay_sdesc(wa + BAY_TC_TILE + 32u * ks);
-                            const unsigned long long xh = bay_sdesc(xs + 32u * ks);
-                            const unsigned long long xl = bay_sdesc(xs + BAY_TC_TILE + 32u * ks);
-                            const unsigned int d = d0 + g * 128u;
-                            bay_mma(d, ah, xh, (c | ks) != 0u ? 1u : 0u);
-                            bay_mma(d, ah, xl, 1u);
-                            bay_mma(d, al, xh, 1u);
+                            product(ks, 1u, (c | ks) != 0u ? 1u : 0u);
+                            product(ks, 2u, 1u);
                         }
+#pragma unroll
+                        for (unsigned int ks = 0; ks < 4u; ++ks) product(ks, 0u, 1u);
+#else
+#pragma unroll
+                        for (unsigned int ks = 0; ks < 4u; ++ks) {
+                            product(ks, 0u, (c | ks) != 0u ? 1u : 0u);
+                            product(ks, 1u, 1u);
+                            product(ks, 2u, 1u);
+                        }
+#endif
                     }
                     bay_mma_commit(b_empty + 8u * s);  // the stage is free once these finish
                 }
@@ -1105,7 +1165,6 @@ __device__ __forceinline__ void bay_gemm_rows_tc_impl(const bay_stretch_params& 
         //      groups' partial sums of a walker are combined at the end in group order.
         constexpr unsigned int GPS = 4u / BAY_TC_G;        // groups per walker sub-tile
         constexpr unsigned int NCOL = 128u / GPS;          // rows of a tile per group
-        const unsigned int et = threadIdx.x - 64u;
         const unsigned int grp = (warp - 2u) >> 2, q = warp & 3u;
         const unsigned int g = grp / GPS;
         const unsigned int c0 = NCOL * (grp % GPS);
@@ -1113,40 +1172,73 @@ __device__ __forceinline__ void bay_gemm_rows_tc_impl(const bay_stretch_params& 
         const unsigned int kw = k0 + g * 128u + wl;
         const bool wv = kw < nk;
         const unsigned int kc = wv ? kw : nk - 1u;
+#if BAY_TC_ATM
+        // the walker operand into tensor memory: group e takes the 64-feature chunk e, a
+        // thread its walker's 128 bytes of hi and of lo (rows up to the padded walker count)
+        if (grp < BAY_TC_KC) {
+            const unsigned int ta = tmem + ((32u * q) << 16) + 256u + 64u * grp;
+#pragma unroll
+            for (unsigned int h = 0; h < 2u; ++h) {
+                const uint4* src = reinterpret_cast<const uint4*>(
+                    (h ? P.s_bl : P.s_bh) + (size_t)kw * P.tc_fp + 64u * grp);
+                uint4 v[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = src[i];
+                bay_tmem_st32(ta + 32u * h, v);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        }
+        bay_tc_fence_before();
+        __syncwarp();
+        if (lane == 0u)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b_wop) : "memory");
+#endif
         float prep[BAY_PREP_LEN];
 #pragma unroll
         for (int i = 0; i < BAY_PREP_LEN; ++i) prep[i] = P.s_prep[(size_t)kc * BAY_PREP_LEN + i];
         const float* xw = P.s_y + (size_t)kc * DIM;
-        const float* auxg = P.gemm_lay + (size_t)rb * BAY_AUXS;   // [rows_pad][AUXS]
-        constexpr unsigned int MA = (BAY_TC_AUXF + BAY_TC_NEPI - 1u) / BAY_TC_NEPI;
+        // The groups of the same rows (one per sub-tile) are a set: they stage the rows' aux
+        // values and wait for a tile together, on a named barrier of their own, so that the
+        // sets drift apart and one's waiting is under another's arithmetic (a scheduler has a
+        // warp of every group).
+        constexpr unsigned int NSET = BAY_TC_NEPI / GPS;   // threads of a set
+        constexpr unsigned int AUXS = NCOL * BAY_AUXS;     // aux values of its rows of a tile
+        const unsigned int set = grp % GPS, es = g * 128u + ((threadIdx.x - 64u) & 127u);
+        const float* auxg = P.gemm_lay + (size_t)(rb + c0) * BAY_AUXS;   // [rows_pad][AUXS]
+        constexpr unsigned int MA = (AUXS + NSET - 1u) / NSET;
         float apre[MA];
 #pragma unroll
         for (unsigned int m = 0; m < MA; ++m) {
-            const unsigned int j = et + m * BAY_TC_NEPI;
-            apre[m] = (j < BAY_TC_AUXF && ntile > 0u) ? __ldg(auxg + j) : 0.0f;
+            const unsigned int j = es + m * NSET;
+            apre[m] = (j < AUXS && ntile > 0u) ? __ldg(auxg + j) : 0.0f;
         }
         float sum = 0.0f, cmp = 0.0f;
+#ifdef BAY_GEMM_TERMS16
+        float carry[BAY_GEMM_CARRY_LEN];
+        BAY_GEMM_CARRY_INIT(carry);
+#endif
         bool ok = true;
         for (unsigned int t = 0; t < ntile; ++t) {
             const unsigned int b = t & 1u;
             float* sa = saux + b * BAY_TC_AUXF;
 #pragma unroll
             for (unsigned int m = 0; m < MA; ++m) {
-                const unsigned int j = et + m * BAY_TC_NEPI;
-                if (j < BAY_TC_AUXF) sa[j] = apre[m];
+                const unsigned int j = es + m * NSET;
+                if (j < AUXS) sa[c0 * BAY_AUXS + j] = apre[m];
             }
             // next tile's aux values, in flight during this tile
 #pragma unroll
             for (unsigned int m = 0; m < MA; ++m) {
-                const unsigned int j = et + m * BAY_TC_NEPI;
-                apre[m] = (j < BAY_TC_AUXF && t + 1u < ntile)
+                const unsigned int j = es + m * NSET;
+                apre[m] = (j < AUXS && t + 1u < ntile)
                     ? __ldg(auxg + (size_t)(t + 1u) * BAY_TC_AUXF + j) : 0.0f;
             }
-            // one thread waits for the accumulator; the decision is shared so that every
-            // epilogue thread leaves the loop together (the named barrier is not bounded)
-            if (et == 0u) flags[2 + b] = bay_tc_wait(b_tfull + 8u * b, (t >> 1) & 1u, abort, status) ? 1u : 0u;
-            asm volatile("bar.sync 1, %0;" ::"r"(BAY_TC_NEPI) : "memory");
-            if (!flags[2 + b]) {
+            // one thread of the set waits for the accumulator; the decision is shared so that
+            // the set leaves the loop together (the named barrier is not bounded)
+            volatile unsigned int* go = flags + 2u + 2u * set + b;
+            if (es == 0u) *go = bay_tc_wait(b_tfull + 8u * b, (t >> 1) & 1u, abort, status) ? 1u : 0u;
+            asm volatile("bar.sync %0, %1;" ::"r"(1u + set), "r"(NSET) : "memory");
+            if (!*go) {
                 ok = false;
                 break;
             }
@@ -1155,7 +1247,7 @@ __device__ __forceinline__ void bay_gemm_rows_tc_impl(const bay_stretch_params& 
             const unsigned int r0 = rb + t * 128u;
             const unsigned int nrow = re - r0 < 128u ? re - r0 : 128u;
             const unsigned int ta = tmem + ((32u * q) << 16) + b * (128u * BAY_TC_G) + g * 128u + c0;
-#pragma unroll 1
+#pragma unroll BAY_TC_EPI_UNROLL
             for (unsigned int j0 = 0; j0 < NCOL; j0 += 16u) {
                 float v[16];
                 bay_tmem_ld16(ta + j0, v);
@@ -1170,22 +1262,30 @@ __device__ __forceinline__ void bay_gemm_rows_tc_impl(const bay_stretch_params& 
                     av[4 * i + 2] = a4.z;
                     av[4 * i + 3] = a4.w;
                 }
-                if (jb + 16u <= nrow) {
+#ifdef BAY_GEMM_TERMS16
+                if (jb + 16u <= nrow) {      // the model's sum of the rows' terms, and its carry
+                    v[0] = BAY_GEMM_TERMS16(v, av, (uint64_t)(r0 + jb), xw, prep, carry);
+                } else
+#endif
+                {
+                    if (jb + 16u <= nrow) {
 #pragma unroll
-                    for (unsigned int jj = 0; jj < 16u; ++jj)
-                        v[jj] = BAY_GEMM_TERM(v[jj], &av[jj * BAY_AUXS], (uint64_t)(r0 + jb + jj),
-                                              xw, prep);
-                } else {
+                        for (unsigned int jj = 0; jj < 16u; ++jj)
+                            v[jj] = BAY_GEMM_TERM(v[jj], &av[jj * BAY_AUXS],
+                                                  (uint64_t)(r0 + jb + jj), xw, prep);
+                    } else {
 #pragma unroll
-                    for (unsigned int jj = 0; jj < 16u; ++jj)
-                        v[jj] = jb + jj < nrow
-                            ? BAY_GEMM_TERM(v[jj], &av[jj * BAY_AUXS], (uint64_t)(r0 + jb + jj), xw, prep)
-                            : 0.0f;
+                        for (unsigned int jj = 0; jj < 16u; ++jj)
+                            v[jj] = jb + jj < nrow
+                                ? BAY_GEMM_TERM(v[jj], &av[jj * BAY_AUXS], (uint64_t)(r0 + jb + jj), xw,
+                                                prep)
+                                : 0.0f;
+                    }
+#pragma unroll
+                    for (unsigned int w = 8u; w >= 1u; w >>= 1)
+#pragma unroll
+                        for (unsigned int i = 0; i < w; ++i) v[i] = __fadd_rn(v[i], v[i + w]);
                 }
-#pragma unroll
-                for (unsigned int w = 8u; w >= 1u; w >>= 1)
-#pragma unroll
-                    for (unsigned int i = 0; i < w; ++i) v[i] = __fadd_rn(v[i], v[i + w]);
                 const float yk = __fsub_rn(v[0], cmp);
                 const float s2 = __fadd_rn(sum, yk);
                 cmp = __fsub_rn(__fsub_rn(s2, sum), yk);
@@ -1199,12 +1299,30 @@ __device__ __forceinline__ void bay_gemm_rows_tc_impl(const bay_stretch_params& 
         // the groups' partial sums of each walker, combined as compensated pairs in group
         // order; stage 0 is free once the last tile's MMAs (hence its copies) are complete
         float* xchg = (float*)(sm + BAY_TC_WBYTES);        // [4 groups][128 lanes][hi, lo]
+#ifdef BAY_GEMM_TERMS16
+        {
+            bay_cf c, r;
+            r.hi = sum;
+            r.lo = -cmp;
+            c.hi = BAY_GEMM_CARRY_END(carry, &c.lo);
+            r = bay_cadd(r, c);
+            sum = r.hi;
+            cmp = -r.lo;
+        }
+#endif
         if (ok) {
             xchg[2 * (grp * 128u + wl)] = sum;
             xchg[2 * (grp * 128u + wl) + 1] = -cmp;
         }
-        asm volatile("bar.sync 1, %0;" ::"r"(BAY_TC_NEPI) : "memory");
-        if (ok && grp % GPS == 0u && wv) {
+        {   // all written; a walker's groups of different sets may have left at different tiles
+            unsigned int all;
+            asm volatile(
+                "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, 5, %2, p;\n"
+                " selp.u32 %0, 1, 0, q;\n}\n"
+                : "=r"(all) : "r"(ok ? 1u : 0u), "r"(BAY_TC_NEPI) : "memory");
+            ok = all != 0u;
+        }
+        if (ok && set == 0u && wv) {
             bay_cf a;
             a.hi = sum;
             a.lo = -cmp;
