@@ -335,6 +335,16 @@ size_t gemm_smem_bytes(const bay_model* m, uint64_t rows) {
                             kGemmWalkers * dpad + np * auxs);
 }
 
+// Plain form: dynamic shared memory of a launch of `ctas` CTAs, the whole params where they are
+// staged (bay_stage_begin) or 0.  Up to 48 KB they are (4 CTAs of 256 threads an SM still fit);
+// up to 200 KB where every CTA has an SM to itself anyway.  16-byte-aligned params only.
+constexpr size_t kPlainSmem = 48 * 1024 - 4096, kPlainSmemMax = 200 * 1024;
+size_t plain_smem(const float* params, uint64_t n_params, uint64_t ctas, int sm_count) {
+    const uint64_t bytes = (n_params * sizeof(float) + 15) & ~15ull;
+    if (n_params == 0 || (uintptr_t)params % 16) return 0;
+    return bytes <= (ctas <= (uint64_t)sm_count ? kPlainSmemMax : kPlainSmem) ? (size_t)bytes : 0;
+}
+
 // Streamed GEMM form: walkers per CTA of the propose kernel (BAY_PW), their rows in at most
 // 48 KB of shared memory (8 rows up to 1,535 coordinates, 2 up to the largest dim of 4,096).
 uint32_t gemm_propose_walkers(uint32_t dim) { return (dim | 1u) * 8 * sizeof(float) <= 49152 ? 8u : 2u; }
@@ -549,6 +559,18 @@ struct bay_sampler {
         return model->form == BAY_FORM_PLAIN ? model->cta : model->wpc;
     }
 
+    // Plain form: CTAs that share a group of model->cta walkers.  Below one group an SM the
+    // default group of 256 is four CTAs of 64 threads, a cluster in the accu launch, which
+    // combines the group's sums as one CTA does: 8,192 walkers x 1,000 rows are 128 CTAs then,
+    // 5.7 us a bare launch, and 8 with 32.
+    uint32_t plain_split() const {
+        if (model->form != BAY_FORM_PLAIN || model->cta != 256 || grid() >= (unsigned)ctx->sm_count) return 1u;
+        // (not where the params are staged by whole CTAs alone)
+        return plain_smem(params, n_params, 4ull * grid(), ctx->sm_count) ||
+                       !plain_smem(params, n_params, grid(), ctx->sm_count)
+                   ? 4u : 1u;
+    }
+
     // CTAs of the launch that writes the accu statistics (and so of the partials)
     unsigned grid() const { return (unsigned)((K + per_cta() - 1) / per_cta()); }
 
@@ -625,8 +647,8 @@ struct bay_sampler {
         return p;
     }
 
-    // pdl = false launches the resident tensor-core kernels without programmatic
-    // dependent launch (the body of a conditional graph node)
+    // pdl = false launches without programmatic dependent launch (the body of a conditional
+    // graph node)
     void launch_half(bool accu, uint32_t half, uint32_t step_off, cudaStream_t st, bool pdl = true) {
         if (streaming) {
             launch_streaming(accu ? 1 : 0, half, step_off, st);
@@ -635,34 +657,36 @@ struct bay_sampler {
         if (st == ctx->stream) bay::count_launches(1);
         bay_stretch_params p = make_params(half, step_off);
         void* args[] = {&p};
-        if (tcr || model->form == BAY_FORM_TILED) {
-            // programmatic dependent launch: the kernel sets up its barriers (tensor memory,
-            // data copies) and reads what the previous kernel of the stream does not write,
-            // then waits (griddepcontrol.wait) for that kernel to complete, so all this
-            // overlaps its tail
-            CUlaunchAttribute at[1];
-            at[0].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
-            at[0].value.programmaticStreamSerializationAllowed = 1;
-            CUlaunchConfig cfg{};
-            cfg.gridDimX = tcr ? (grid() + tr_g - 1) / tr_g : grid() * model->tslices;
-            cfg.gridDimY = 1;
-            cfg.gridDimZ = 1;
-            cfg.blockDimX = tcr ? 256 * tr_g : model->cta;
-            cfg.blockDimY = 1;
-            cfg.blockDimZ = 1;
-            cfg.sharedMemBytes = (unsigned)smem_move;
-            cfg.hStream = (CUstream)st;
-            cfg.attrs = at;
-            cfg.numAttrs = pdl ? 1 : 0;
-            CUkernel k = tcr ? model->k_tr[accu ? 1 : 0] : (accu ? model->k_accu : model->k_bare);
-            cu_check(g_cu.LaunchKernelEx(&cfg, (CUfunction)k, args, nullptr),
-                     tcr ? "cuLaunchKernelEx(stretch, tensor cores)" : "cuLaunchKernelEx(stretch, tiled)");
-            return;
+        // programmatic dependent launch: the kernel sets up its barriers (tensor memory, data
+        // copies) and reads what the previous kernel of the stream does not write, then waits
+        // (griddepcontrol.wait) for that kernel to complete, so all this overlaps its tail
+        const bool tiled = model->form == BAY_FORM_TILED, plain = model->form == BAY_FORM_PLAIN;
+        const uint32_t split = plain_split();
+        CUlaunchAttribute at[2];
+        at[0].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+        at[0].value.programmaticStreamSerializationAllowed = 1;
+        CUlaunchConfig cfg{};
+        cfg.gridDimX = tcr ? (grid() + tr_g - 1) / tr_g : grid() * (tiled ? model->tslices : split);
+        cfg.gridDimY = 1;
+        cfg.gridDimZ = 1;
+        cfg.blockDimX = tcr ? 256 * tr_g : model->cta / split;
+        cfg.blockDimY = 1;
+        cfg.blockDimZ = 1;
+        cfg.sharedMemBytes = (unsigned)(tcr || tiled ? smem_move
+                                        : plain ? plain_smem(params, n_params, cfg.gridDimX, ctx->sm_count)
+                                                : smem);
+        cfg.hStream = (CUstream)st;
+        cfg.attrs = at;
+        cfg.numAttrs = pdl ? 1 : 0;
+        if (accu && split > 1) {
+            CUlaunchAttribute& cl = at[cfg.numAttrs++];
+            cl.id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+            cl.value.clusterDim.x = split;
+            cl.value.clusterDim.y = 1;
+            cl.value.clusterDim.z = 1;
         }
-        CUkernel k = accu ? model->k_accu : model->k_bare;
-        cu_check(g_cu.LaunchKernel((CUfunction)k, grid(), 1, 1, model->cta, 1, 1,
-                                   (unsigned)smem, (CUstream)st, args, nullptr),
-                 "cuLaunchKernel(stretch)");
+        CUkernel k = tcr ? model->k_tr[accu ? 1 : 0] : (accu ? model->k_accu : model->k_bare);
+        cu_check(g_cu.LaunchKernelEx(&cfg, (CUfunction)k, args, nullptr), "cuLaunchKernelEx(stretch)");
     }
 
     void ctl_op(const bay_ctl_op& op) {
@@ -677,9 +701,13 @@ struct bay_sampler {
         bay::count_launches(1);
         bay_stretch_params p = make_params(0, 0);
         void* args[] = {&p};
-        const unsigned g = (unsigned)((W + per_cta() - 1) / per_cta());
+        const bool plain = model->form == BAY_FORM_PLAIN;
+        const uint32_t block = tcr ? 256 : plain ? model->cta / plain_split() : model->cta;
+        const uint64_t per = plain ? block : per_cta();
+        const unsigned g = (unsigned)((W + per - 1) / per);
         cu_check(g_cu.LaunchKernel((CUfunction)(tcr ? model->k_tr[2] : model->k_logfn), g, 1, 1,
-                                   tcr ? 256 : model->cta, 1, 1, (unsigned)smem,
+                                   block, 1, 1,
+                                   (unsigned)(plain ? plain_smem(params, n_params, g, ctx->sm_count) : smem),
                                    (CUstream)ctx->stream, args, nullptr),
                  "cuLaunchKernel(logfn)");
     }
@@ -1156,6 +1184,13 @@ int bay_model_compile(bay_ctx* c, const bay_model_desc* d, bay_model** out) {
                     cu_check(g_cu.LibraryGetKernel(&m->k_evidence, m->lib, "bay_points_evidence"),
                              "GetKernel(evidence)");
                 }
+            }
+            if (d->form == BAY_FORM_PLAIN) {
+                CUdevice dev = (CUdevice)c->device;
+                for (CUkernel k : {m->k_bare, m->k_accu, m->k_logfn, m->k_points, m->k_evidence})
+                    cu_check(g_cu.KernelSetAttribute(CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES,
+                                                     (int)kPlainSmemMax, k, dev),
+                             "cuKernelSetAttribute(smem)");
             }
             if (d->form == BAY_FORM_TILED) {
                 CUdevice dev = (CUdevice)c->device;

@@ -208,16 +208,28 @@ __device__ __forceinline__ float bay_cf_total(float a, bay_cf s) {
 // shuffles, per-warp sums staged in shared memory (one barrier per 64 dims), combined
 // across warps with compensated fp32 in warp order, stored to part[(step_off*2 + half)][dim][cta].  The
 // per-step ensemble means are reduced from these partials by a separate kernel.
+// Where the group's CTA is split over a cluster (plain form, small ensembles), the warps' sums
+// meet in the first CTA's shared memory: the same warps, combined in the same order.
 #define BAY_SUM_CHUNK 64
+__device__ __forceinline__ void bay_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ void bay_accu_epilogue(const bay_stretch_params& P, bool accepted, bool valid,
                                   const float* mine, float (*red)[BAY_SUM_CHUNK],
-                                  unsigned int slot, unsigned int nslots) {
+                                  unsigned int slot, unsigned int nslots,
+                                  unsigned int ncta = 1u, unsigned int rank = 0u) {
     const int n_acc = __syncthreads_count(accepted);
     if (threadIdx.x == 0 && n_acc) atomicAdd(&P.ctl->accepted, (unsigned long long)n_acc);
     if (P.means_cap == 0) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nwarps = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = (rank * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = ncta * (blockDim.x >> 5);
     float* out = P.part + ((size_t)P.step_off * 2 + P.half) * DIM * nslots + slot;
+    unsigned int first = 0;                   // the first CTA's `red`
+    if (ncta > 1u) {
+        bay_cluster_sync();                   // every CTA of the cluster is there
+        asm("mapa.shared::cluster.u32 %0, %1, 0;"
+            : "=r"(first) : "r"((unsigned int)__cvta_generic_to_shared(&red[0][0])));
+    }
 #pragma unroll
     for (int d0 = 0; d0 < DIM; d0 += BAY_SUM_CHUNK) {
 #pragma unroll
@@ -225,11 +237,19 @@ __device__ void bay_accu_epilogue(const bay_stretch_params& P, bool accepted, bo
             float v = valid ? mine[d] : 0.0f;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if (lane == 0) red[warp][d - d0] = v;
+            if (lane == 0) {
+                if (ncta > 1u)
+                    asm volatile("st.shared::cluster.f32 [%0], %1;"
+                                 ::"r"(first + 4u * (unsigned int)(warp * BAY_SUM_CHUNK + d - d0)), "f"(v)
+                                 : "memory");
+                else
+                    red[warp][d - d0] = v;
+            }
         }
-        __syncthreads();
+        if (ncta > 1u) bay_cluster_sync();
+        else __syncthreads();
         const int nd = (DIM - d0) < BAY_SUM_CHUNK ? (DIM - d0) : BAY_SUM_CHUNK;
-        for (int d = threadIdx.x; d < nd; d += blockDim.x) {
+        for (int d = threadIdx.x; d < nd && rank == 0u; d += blockDim.x) {
             bay_cf s;
             s.hi = 0.0f;
             s.lo = 0.0f;
@@ -241,7 +261,10 @@ __device__ void bay_accu_epilogue(const bay_stretch_params& P, bool accepted, bo
             }
             out[(size_t)(d0 + d) * nslots] = __fadd_rn(s.hi, s.lo);
         }
-        __syncthreads();
+        if (d0 + BAY_SUM_CHUNK < DIM) {       // the next chunk's sums overwrite red
+            if (ncta > 1u) bay_cluster_sync();
+            else __syncthreads();
+        }
     }
 }
 
@@ -286,7 +309,6 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
     const unsigned int tid = threadIdx.x;
     const unsigned int k0 = blockIdx.x * BAY_WT;
     const unsigned int nk = LOGFN_ONLY ? P.W : P.K;
-    const unsigned int step = P.ctl->step[kind] + P.step_off;
     const float* hyper = P.params + P.data_len;
     float* X = P.xs + (LOGFN_ONLY ? 0 : (size_t)P.half * P.K * DIM);
     const float* S = P.xs + (size_t)(1u - P.half) * P.K * DIM;
@@ -310,6 +332,12 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
             ::"r"((unsigned int)__cvta_generic_to_shared(As)), "l"(P.gemm_lay), "r"(lay_bytes),
             "r"(bar) : "memory");
     }
+    // Launched with programmatic dependent launch: the matrix never changes, the rest waits
+    // for the previous launch
+    if (!LOGFN_ONLY) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     // 2. proposals (Philox, z, partner) for the tile, then Y in both layouts; each thread
     //    keeps all its gather loads in flight before it uses any of them
     if (!LOGFN_ONLY && tid < BAY_WT) {
@@ -318,7 +346,7 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
             const unsigned int stream = ACCU ? (P.half ? 2222u : 1111u) : (P.half ? 4444u : 3333u);
             bay_u4 c;
             c.x = k;
-            c.y = step;
+            c.y = P.ctl->step[kind] + P.step_off;
             c.z = stream;
             c.w = 0xbeeff00du;
             const bay_u4 r = bay_philox4x32_10(c, P.ctl->seed[kind] + P.half, 0xdecafbadu);
@@ -2166,8 +2194,85 @@ extern "C" __global__ void __launch_bounds__(1024, 1) bay_tcr_run_accu(bay_stret
 // ---------------------------------------------------------------- plain form
 // One thread per walker of the moving half, the model's LOGFN evaluated per thread
 // (the reference's structure, with SoA coalesced loads and registers for Y).
+
+// The params staged in shared memory (dynamic, as much as the host gave the launch; none: they
+// stay in global memory).  A density's loop reads them in order, all threads alike, a load
+// every few arithmetic instructions of one dependent sum: from global memory, L1 hits
+// included, a row of 2-D Gaussian data took 31 clocks however few warps there were, from
+// shared memory 8 (8,192 walkers x 1,000 rows: 18.8 us a launch, now 5.7).
+// One bulk copy, begun before the launch waits for its predecessor (the params never
+// change while a sampler runs), the last floats past its 16-byte multiple by plain loads.
+struct bay_plain_sync {
+    unsigned long long bar;
+};
+__device__ __forceinline__ unsigned int bay_dyn_smem() {
+    unsigned int n;
+    asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(n));
+    return n;
+}
+__device__ __forceinline__ void bay_stage_begin(bay_plain_sync* sy, const float* p, unsigned int n,
+                                                unsigned int staged) {
+    extern __shared__ __align__(16) float bay_psm[];
+    if (!staged) return;
+    const unsigned int bar = (unsigned int)__cvta_generic_to_shared(&sy->bar), bytes = (n * 4u) & ~15u;
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+                     : "memory");
+        if (bytes)
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                ::"r"((unsigned int)__cvta_generic_to_shared(bay_psm)), "l"(p), "r"(bytes), "r"(bar)
+                : "memory");
+    }
+    if (bytes / 4u + threadIdx.x < n && threadIdx.x < 4u)
+        bay_psm[bytes / 4u + threadIdx.x] = p[bytes / 4u + threadIdx.x];
+    __syncthreads();
+}
+// Bounded wait (2 s) for the copy; false, with status bit 1 set, when it gave up.
+__device__ __forceinline__ bool bay_stage_wait(bay_plain_sync* sy, unsigned int staged,
+                                               unsigned int* status) {
+    if (!staged) return true;
+    const unsigned int bar = (unsigned int)__cvta_generic_to_shared(&sy->bar);
+    unsigned long long t0 = 0;
+    for (unsigned int it = 0;; ++it) {
+        unsigned int ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n"
+            " selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok) : "r"(bar) : "memory");
+        if (ok) return true;
+        if ((it & 15u) == 0u) {
+            unsigned long long t;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            if (it == 0u) {
+                t0 = t;
+            } else if (t - t0 > 2000000000ull) {
+                if (status) atomicOr(status, 1u);
+                return false;
+            }
+        }
+    }
+}
+__device__ __forceinline__ float bay_density(unsigned int staged, unsigned int data_len,
+                                             unsigned int params_len, const float* params,
+                                             const float* x) {
+    extern __shared__ __align__(16) float bay_psm[];
+    return staged ? BAY_LOGFN(data_len, params_len, bay_psm, DIM, x)
+                  : BAY_LOGFN(data_len, params_len, params, DIM, x);
+}
+
+// Launched with programmatic dependent launch.  A group of BAY_CTA walkers is a CTA, or a
+// cluster of smaller ones where the ensemble has fewer groups than the device has SMs.
 template <bool ACCU>
 __device__ __forceinline__ void bay_stretch_plain(const bay_stretch_params& P) {
+    __shared__ bay_plain_sync sSync;
+    const unsigned int staged = bay_dyn_smem();
+    bay_stage_begin(&sSync, P.params, (unsigned int)P.data_len + P.params_len, staged);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const unsigned int kind = ACCU ? 1u : 0u;
     const unsigned int k = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = k < P.K;
@@ -2195,9 +2300,10 @@ __device__ __forceinline__ void bay_stretch_plain(const bay_stretch_params& P) {
             const float s = bay_partner_coord(S, P.K, j, i);
             Y[i] = __fmaf_rn(z, __fsub_rn(X[(size_t)k * DIM + i], s), s);
         }
-        const float ly = BAY_LOGFN((unsigned int)P.data_len, P.params_len, P.params, DIM, Y);
         const float lx = P.logfn[(size_t)P.half * P.K + k];
-        accepted = bay_accept(u2, z, ly, lx, beta);
+        const bool ok = bay_stage_wait(&sSync, staged, &P.ctl->status);
+        const float ly = bay_density(staged, (unsigned int)P.data_len, P.params_len, P.params, Y);
+        accepted = ok && bay_accept(u2, z, ly, lx, beta);
         if (accepted) {
 #pragma unroll
             for (int i = 0; i < DIM; ++i) X[(size_t)k * DIM + i] = Y[i];
@@ -2206,10 +2312,15 @@ __device__ __forceinline__ void bay_stretch_plain(const bay_stretch_params& P) {
 #pragma unroll
             for (int i = 0; i < DIM; ++i) Y[i] = X[(size_t)k * DIM + i];
         }
+    } else {
+        bay_stage_wait(&sSync, staged, &P.ctl->status);   // the copy lands before the CTA may end
     }
     if (ACCU) {
         __shared__ float red[BAY_CTA / 32][BAY_SUM_CHUNK];
-        bay_accu_epilogue(P, accepted, valid, Y, red, blockIdx.x, gridDim.x);
+        unsigned int ncta, rank;
+        asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ncta));
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        bay_accu_epilogue(P, accepted, valid, Y, red, blockIdx.x / ncta, gridDim.x / ncta, ncta, rank);
     }
 }
 
@@ -2222,12 +2333,16 @@ extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_accu(bay_stret
 
 // logfn over all W walkers (nvidia-gtx-mcmc-stretch.cu:197-206), SoA input.
 extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_logfn_all(bay_stretch_params P) {
+    __shared__ bay_plain_sync sSync;
+    const unsigned int staged = bay_dyn_smem();
+    bay_stage_begin(&sSync, P.params, (unsigned int)P.data_len + P.params_len, staged);
     const unsigned int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= P.W) return;
+    const bool ok = bay_stage_wait(&sSync, staged, &P.ctl->status);
+    if (k >= P.W || !ok) return;
     float x[DIM];
 #pragma unroll
     for (int i = 0; i < DIM; ++i) x[i] = P.xs[(size_t)k * DIM + i];
-    P.logfn[k] = BAY_LOGFN((unsigned int)P.data_len, P.params_len, P.params, DIM, x);
+    P.logfn[k] = bay_density(staged, (unsigned int)P.data_len, P.params_len, P.params, x);
 }
 
 // Density engines (reference cuda/engines/nvidia-gtx-distribution.cu logpdf/pdf and
@@ -2236,12 +2351,16 @@ extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_logfn_all(bay_stretch_
 extern "C" __global__ void __launch_bounds__(BAY_CTA)
 bay_points_logfn(unsigned long long n, unsigned int data_len, unsigned int params_len,
                  const float* params, const float* x, float* out, unsigned int exp_out) {
+    __shared__ bay_plain_sync sSync;
+    const unsigned int staged = bay_dyn_smem();
+    bay_stage_begin(&sSync, params, data_len + params_len, staged);
+    const bool ok = bay_stage_wait(&sSync, staged, nullptr);   // given up: NaN, not a stale value
     for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
          i += (unsigned long long)gridDim.x * blockDim.x) {
         float p[DIM];
 #pragma unroll
         for (int d = 0; d < DIM; ++d) p[d] = x[i * DIM + d];
-        const float v = BAY_LOGFN(data_len, params_len, params, DIM, p);
+        const float v = ok ? bay_density(staged, data_len, params_len, params, p) : __int_as_float(0x7fc00000);
         out[i] = exp_out ? expf(v) : v;
     }
 }
@@ -2253,12 +2372,16 @@ bay_points_evidence(unsigned long long n, unsigned int data_len, unsigned int pa
                     const float* params, const float* x, double* part) {
     __shared__ double red[BAY_CTA];
     double s = 0.0;
+    __shared__ bay_plain_sync sSync;
+    const unsigned int staged = bay_dyn_smem();
+    bay_stage_begin(&sSync, params, data_len + params_len, staged);
+    const bool ok = bay_stage_wait(&sSync, staged, nullptr);   // given up: NaN, not a stale value
     for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
          i += (unsigned long long)gridDim.x * blockDim.x) {
         float p[DIM];
 #pragma unroll
         for (int d = 0; d < DIM; ++d) p[d] = x[i * DIM + d];
-        s += (double)expf(BAY_LOGFN(data_len, params_len, params, DIM, p));
+        s += (double)expf(bay_density(staged, data_len, params_len, params, p));
     }
     red[threadIdx.x] = s;
     __syncthreads();
