@@ -451,6 +451,9 @@ __device__ __forceinline__ void bay_batch_rows_impl(const bay_batch_params& P, u
         out[0] = a.hi;
         out[1] = a.lo;
     }
+    // the persistent launch's next item, of another member perhaps and so laid out
+    // differently, is staged over `red` only after these threads have read it
+    __syncthreads();
 }
 
 // Every slice's CTA decides for the tile's walkers (the current log density comes from the
