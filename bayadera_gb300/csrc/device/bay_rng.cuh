@@ -150,14 +150,6 @@ __device__ __forceinline__ bay_v4 operator*(float a, bay_v4 b) { return {a * b.x
 __device__ __forceinline__ bay_v4 operator+(bay_v4 a, float b) { return {a.x + b, a.y + b, a.z + b, a.w + b}; }
 __device__ __forceinline__ bay_v4 operator-(bay_v4 a, float b) { return {a.x - b, a.y - b, a.z - b, a.w - b}; }
 __device__ __forceinline__ bay_v4 operator*(bay_v4 a, float b) { return {a.x * b, a.y * b, a.z * b, a.w * b}; }
-// lane-wise IEEE add and subtract, never contracted (the engine's sums)
-__device__ __forceinline__ bay_v4 bay_v4_add_rn(bay_v4 a, bay_v4 b) {
-    return {__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w)};
-}
-__device__ __forceinline__ bay_v4 bay_v4_sub_rn(bay_v4 a, bay_v4 b) {
-    return {__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z), __fsub_rn(a.w, b.w)};
-}
-
 // Two floats in a 64-bit register pair: one instruction for both (the same fp32 rate as two,
 // half the issue slots).  Lane-wise IEEE operations, flushing like the module's scalar ones.
 typedef unsigned long long bay_f2;
@@ -181,6 +173,11 @@ __device__ __forceinline__ bay_f2 bay_f2_add(bay_f2 a, bay_f2 b) {
     asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ bay_f2 bay_f2_sub(bay_f2 a, bay_f2 b) {
+    bay_f2 r;
+    asm("sub.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ bay_f2 bay_f2_mul(bay_f2 a, bay_f2 b) {
     bay_f2 r;
     asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
@@ -192,4 +189,29 @@ __device__ __forceinline__ bay_f2 bay_f2_fma(bay_f2 a, bay_f2 b, bay_f2 c) {
     return r;
 }
 
+// Lane-wise IEEE operations of bay_v4, never contracted: the engine's sums, and row terms
+// that are written with them.  Additions and squares two lanes an instruction; a product is
+// four, because the compiler contracts a packed product and a packed addition into one
+// multiply-add in spite of their .rn (where it sees them together, so not in every kernel).
+__device__ __forceinline__ bay_v4 bay_v4_from(bay_f2 lo, bay_f2 hi) {
+    return {bay_f2_x(lo), bay_f2_y(lo), bay_f2_x(hi), bay_f2_y(hi)};
+}
+__device__ __forceinline__ bay_f2 bay_v4_lo(bay_v4 a) { return bay_f2_of(a.x, a.y); }
+__device__ __forceinline__ bay_f2 bay_v4_hi(bay_v4 a) { return bay_f2_of(a.z, a.w); }
+__device__ __forceinline__ bay_v4 bay_v4_add_rn(bay_v4 a, bay_v4 b) {
+    return bay_v4_from(bay_f2_add(bay_v4_lo(a), bay_v4_lo(b)), bay_f2_add(bay_v4_hi(a), bay_v4_hi(b)));
+}
+__device__ __forceinline__ bay_v4 bay_v4_sub_rn(bay_v4 a, bay_v4 b) {
+    return bay_v4_from(bay_f2_sub(bay_v4_lo(a), bay_v4_lo(b)), bay_f2_sub(bay_v4_hi(a), bay_v4_hi(b)));
+}
+// a * (b * b)
+__device__ __forceinline__ bay_v4 bay_v4_mul_sq_rn(bay_v4 a, bay_v4 b) {
+    const bay_f2 lo = bay_f2_mul(bay_v4_lo(b), bay_v4_lo(b)), hi = bay_f2_mul(bay_v4_hi(b), bay_v4_hi(b));
+    return {__fmul_rn(a.x, bay_f2_x(lo)), __fmul_rn(a.y, bay_f2_y(lo)), __fmul_rn(a.z, bay_f2_x(hi)),
+            __fmul_rn(a.w, bay_f2_y(hi))};
+}
+__device__ __forceinline__ bay_v4 bay_v4_sub_rn(float a, bay_v4 b) {
+    const bay_f2 q = bay_f2_of(a, a);
+    return bay_v4_from(bay_f2_sub(q, bay_v4_lo(b)), bay_f2_sub(q, bay_v4_hi(b)));
+}
 #endif

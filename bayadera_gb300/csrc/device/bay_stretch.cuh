@@ -2489,8 +2489,8 @@ __device__ __forceinline__ void bay_tile_begin(const bay_stretch_params& P, bay_
 }
 
 // Sum over all data rows of BAY_TILE_TERM(row, prep of walker w) for the CTA's walkers
-// w < BAY_WPC (prep: [BAY_WPC][BAY_PREP_LEN] in shared memory) -> out[w] (compensated
-// pairs), the copies begun by bay_tile_begin.  Every thread of the CTA calls it.  Returns
+// w < BAY_WPC (prep: [BAY_WPC][BAY_PREP_LEN] in shared memory) -> *out of thread w (a
+// compensated pair), the copies begun by bay_tile_begin.  Every thread of the CTA calls it.  Returns
 // false (and sets the status) when a bounded wait for a copy gave up; out is then
 // incomplete.
 // With BAY_TILE_TERM4 (the model's row term over bay_v4) and BAY_WPC a multiple of 4, a
@@ -2591,12 +2591,12 @@ __device__ __forceinline__ bool bay_tiled_logfn_rows(const bay_stretch_params& P
         if (lane < WS) red[warp][WV * lane + j] = v;
     }
     __syncthreads();
+    // (a walker's total is its thread's: BAY_WPC <= 32, all in warp 0)
     if (tid < BAY_WPC) {
         bay_cf s = red[0][tid];
         for (unsigned int i = 1; i < BAY_CTA / 32u; ++i) s = bay_cadd(s, red[i][tid]);
-        out[tid] = s;
+        *out = s;
     }
-    __syncthreads();
     return ok;
 }
 
@@ -2607,8 +2607,6 @@ __device__ __forceinline__ void bay_stretch_tiled(const bay_stretch_params& P) {
     __shared__ float sPrep[BAY_WPC][BAY_PREP_LEN];
     __shared__ float sW[BAY_WPC], sZ[BAY_WPC], sU2[BAY_WPC];
     __shared__ bay_cf sRed[BAY_CTA / 32][BAY_WPC];
-    __shared__ bay_cf sSum[BAY_WPC];
-    __shared__ float red1[BAY_CTA / 32][BAY_SUM_CHUNK];
     const unsigned int step = P.ctl->step[kind] + P.step_off;
     const unsigned int seed = P.ctl->seed[kind] + P.half;
     const float a = P.ctl->a;
@@ -2633,7 +2631,7 @@ __device__ __forceinline__ void bay_stretch_tiled(const bay_stretch_params& P) {
     // wait for the previous launch; the partner row, from the half that launch moves, after.
     const unsigned int t0 = threadIdx.x, kk = k0 + t0;
     const bool mine_ok = t0 < BAY_WPC && kk < P.K;
-    float xr[DIM], z = 0.0f, u2 = 0.0f;
+    float xr[DIM], z = 0.0f, u2 = 0.0f, lx = 0.0f;
     unsigned int j = 0;
     if (mine_ok) {
         bay_u4 c;
@@ -2647,6 +2645,7 @@ __device__ __forceinline__ void bay_stretch_tiled(const bay_stretch_params& P) {
         u2 = bay_u01(r.z);
 #pragma unroll
         for (int i = 0; i < DIM; ++i) xr[i] = X[(size_t)kk * DIM + i];
+        lx = P.logfn[(size_t)P.half * P.K + kk];
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -2675,7 +2674,9 @@ __device__ __forceinline__ void bay_stretch_tiled(const bay_stretch_params& P) {
         }
     }
     __syncthreads();
-    bool ok = bay_tiled_logfn_rows(P, sPrep, sRed, sSum, &sSync, rb, rn);
+    bay_cf sum;
+    sum.hi = sum.lo = 0.0f;
+    bool ok = bay_tiled_logfn_rows(P, sPrep, sRed, &sum, &sSync, rb, rn);
     bool accepted = false;
     const unsigned int t = threadIdx.x, k = k0 + t;
     const bool valid = t < BAY_WPC && k < P.K;
@@ -2684,7 +2685,7 @@ __device__ __forceinline__ void bay_stretch_tiled(const bay_stretch_params& P) {
         // rejected), take the group's ticket; the last slice combines them in slice order
         __shared__ unsigned int sLast;
         float2* part = reinterpret_cast<float2*>(P.t_part);
-        if (valid) part[(size_t)k * NS + sl] = ok ? make_float2(sSum[t].hi, sSum[t].lo)
+        if (valid) part[(size_t)k * NS + sl] = ok ? make_float2(sum.hi, sum.lo)
                                                  : make_float2(__int_as_float(0x7fc00000), 0.0f);
         __threadfence();
         __syncthreads();
@@ -2704,29 +2705,39 @@ __device__ __forceinline__ void bay_stretch_tiled(const bay_stretch_params& P) {
                 b.lo = v.y;
                 a = bay_cadd(a, b);
             }
-            sSum[t] = a;
+            sum = a;
         }
         ok = true;
-        __syncthreads();
     }
-    float mine[DIM];
-    if (valid) {
-        if (ok) {
-            const float ly = bay_cf_total(sW[t], sSum[t]);
-            const float lx = P.logfn[(size_t)P.half * P.K + k];
-            accepted = bay_accept(sU2[t], sZ[t], ly, lx, beta);
-            if (accepted) {
+    // the rest is the walkers' warp's: decision, write-back, and the group's statistics (the
+    // warps' sums in warp order, of which the others' are zeros)
+    if (t >= 32u) return;
+    if (valid && ok) {
+        const float ly = bay_cf_total(sW[t], sum);
+        accepted = bay_accept(sU2[t], sZ[t], ly, lx, beta);
+        if (accepted) {
 #pragma unroll
-                for (int i = 0; i < DIM; ++i) X[(size_t)k * DIM + i] = sY[t][i];
-                P.logfn[(size_t)P.half * P.K + k] = ly;
-            }
-        }
-        if (ACCU) {
-#pragma unroll
-            for (int i = 0; i < DIM; ++i) mine[i] = accepted ? sY[t][i] : X[(size_t)k * DIM + i];
+            for (int i = 0; i < DIM; ++i) X[(size_t)k * DIM + i] = sY[t][i];
+            P.logfn[(size_t)P.half * P.K + k] = ly;
         }
     }
-    if (ACCU) bay_accu_epilogue(P, accepted, valid, mine, red1, g, groups);
+    if (ACCU) {
+        const unsigned int bal = __ballot_sync(0xffffffffu, accepted);
+        if (t == 0 && bal) atomicAdd(&P.ctl->accepted, (unsigned long long)__popc(bal));
+        if (P.means_cap == 0) return;
+        float* out = P.part + ((size_t)P.step_off * 2 + P.half) * DIM * groups + g;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            float v = valid ? (accepted ? sY[t][d] : xr[d]) : 0.0f;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            bay_cf s, w;
+            s.hi = s.lo = w.lo = 0.0f;
+            w.hi = v;
+            s = bay_cadd(s, w);
+            if (t == 0) out[(size_t)d * groups] = __fadd_rn(s.hi, s.lo);
+        }
+    }
 }
 
 extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_bare(bay_stretch_params P) {
@@ -2741,7 +2752,8 @@ extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_logfn_all(bay_stretch_
     __shared__ float sPrep[BAY_WPC][BAY_PREP_LEN];
     __shared__ float sW[BAY_WPC];
     __shared__ bay_cf sRed[BAY_CTA / 32][BAY_WPC];
-    __shared__ bay_cf sSum[BAY_WPC];
+    bay_cf sum;
+    sum.hi = sum.lo = 0.0f;
     const float* hyper = P.params + P.data_len;
     const unsigned long long n_rows = P.data_len / BAY_ROW_LEN;
     const unsigned int k0 = blockIdx.x * BAY_WPC;
@@ -2765,8 +2777,8 @@ extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_logfn_all(bay_stretch_
         }
     }
     __syncthreads();
-    const bool ok = bay_tiled_logfn_rows(P, sPrep, sRed, sSum, &sSync, 0ull, n_rows);
+    const bool ok = bay_tiled_logfn_rows(P, sPrep, sRed, &sum, &sSync, 0ull, n_rows);
     const unsigned int t = threadIdx.x, k = k0 + t;
-    if (ok && t < BAY_WPC && k < P.W) P.logfn[k] = bay_cf_total(sW[t], sSum[t]);
+    if (ok && t < BAY_WPC && k < P.W) P.logfn[k] = bay_cf_total(sW[t], sum);
 }
 #endif
