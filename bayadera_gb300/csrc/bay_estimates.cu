@@ -42,6 +42,20 @@ __device__ __forceinline__ Place place_of(uint32_t D, uint32_t gx, uint32_t tile
     return p;
 }
 
+// The thread's kBatch values from row r on (`none` past the last row), all loads in flight.
+__device__ __forceinline__ void load_batch(float (&v)[kBatch], const float* col, uint64_t r,
+                                           uint64_t stride, uint64_t W, uint32_t D, float none) {
+    if (r + (kBatch - 1) * stride < W) {
+        const float* q = col + r * D;
+        const uint64_t step = stride * D;
+#pragma unroll
+        for (uint32_t i = 0; i < kBatch; ++i) v[i] = __ldg(q + i * step);
+    } else {
+#pragma unroll
+        for (uint32_t i = 0; i < kBatch; ++i) v[i] = r + i * stride < W ? __ldg(col + (r + i * stride) * D) : none;
+    }
+}
+
 // red[thread] summed over the rows of each dimension in a fixed tree; the sum of dimension
 // dl is in red[dl].
 __device__ __forceinline__ void rows_sum(const Place& p, double* red) {
@@ -146,12 +160,13 @@ moments_pass(const float* __restrict__ x, uint32_t D, uint64_t W, uint32_t gx, u
         const float* col = x + p.d0 + p.dl;
         fp_sum f;
         uint32_t held = 0;
+        float ahead[kBatch];
+        load_batch(ahead, col, p.r0, p.stride, W, D, c);
         for (uint64_t r = p.r0; r < W; r += kBatch * p.stride) {
             float v[kBatch];
-            const bool full = r + (kBatch - 1) * p.stride < W;
 #pragma unroll
-            for (uint32_t i = 0; i < kBatch; ++i)
-                v[i] = full || r + i * p.stride < W ? __ldg(col + (r + i * p.stride) * D) : c;
+            for (uint32_t i = 0; i < kBatch; ++i) v[i] = ahead[i];
+            load_batch(ahead, col, r + kBatch * p.stride, p.stride, W, D, c);
             const fp_sum before = f;
             float top = 0.0f;
 #pragma unroll
@@ -233,12 +248,13 @@ limits_pass(const float* __restrict__ x, uint32_t D, uint64_t W, uint32_t gx, ui
     float mn = nan, mx = nan;
     if (p.on) {
         const float* col = x + p.d0 + p.dl;
+        float ahead[kBatch];
+        load_batch(ahead, col, p.r0, p.stride, W, D, nan);
         for (uint64_t r = p.r0; r < W; r += kBatch * p.stride) {
             float v[kBatch];
-            const bool full = r + (kBatch - 1) * p.stride < W;
 #pragma unroll
-            for (uint32_t i = 0; i < kBatch; ++i)
-                v[i] = full || r + i * p.stride < W ? __ldg(col + (r + i * p.stride) * D) : nan;
+            for (uint32_t i = 0; i < kBatch; ++i) v[i] = ahead[i];
+            load_batch(ahead, col, r + kBatch * p.stride, p.stride, W, D, nan);
 #pragma unroll
             for (uint32_t i = 0; i < kBatch; ++i) {
                 mn = fminf(mn, v[i]);
@@ -300,12 +316,14 @@ hist_count(const float* __restrict__ x, uint32_t D, uint64_t W, uint32_t gx, uin
         const float fb = (float)bins;
         uint32_t* mine = h + ((threadIdx.x >> 5) % copies) * nh + p.dl * bins;
         const float* col = x + p.d0 + p.dl;
+        float ahead[kBatch];
+        load_batch(ahead, col, p.r0, p.stride, W, D, 0.0f);
         for (uint64_t r = p.r0; r < W; r += kBatch * p.stride) {
             float v[kBatch];
             const bool full = r + (kBatch - 1) * p.stride < W;
 #pragma unroll
-            for (uint32_t i = 0; i < kBatch; ++i)
-                v[i] = full || r + i * p.stride < W ? __ldg(col + (r + i * p.stride) * D) : 0.0f;
+            for (uint32_t i = 0; i < kBatch; ++i) v[i] = ahead[i];
+            load_batch(ahead, col, r + kBatch * p.stride, p.stride, W, D, 0.0f);
 #pragma unroll
             for (uint32_t i = 0; i < kBatch; ++i) {
                 const float q = __fmul_rn(__fdiv_rn(__fsub_rn(v[i], lo), range), fb);

@@ -55,9 +55,11 @@ struct bay_stretch_params {
     unsigned int tc_fp;
     unsigned int gbar_extra;
     unsigned int t_slices;
-    unsigned int pad_t;
+    unsigned int beta_set;
     float* t_part;
     unsigned int* t_ticket;
+    float beta;
+    unsigned int pad_t;
 };
 
 enum {

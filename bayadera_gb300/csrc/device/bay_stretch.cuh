@@ -114,10 +114,15 @@ struct bay_stretch_params {
     // slice's CTA leaves its walkers' partial sums in t_part[k][slice] (hi, lo) and takes a
     // ticket in t_ticket[group]; the last one combines them in slice order and decides
     unsigned int t_slices;
-    unsigned int pad_t;
-    float* t_part;
+    unsigned int beta_set;          // bare: beta of this launch below instead of the control
+    float* t_part;                  // block's (an annealing step's)
     unsigned int* t_ticket;
+    float beta;
+    unsigned int pad_t;
 };
+__device__ __forceinline__ float bay_beta(const bay_stretch_params& P) {
+    return P.beta_set ? P.beta : P.ctl->beta;
+}
 
 __device__ __forceinline__ float bay_stretch_z(float a, float u1) {
     // z = (a - 2 + 1/a) u1^2 + 2 (1 - 1/a) u1 + 1/a with the first product fused and
@@ -493,7 +498,7 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
         if (LOGFN_ONLY) {
             P.logfn[k] = ly;
         } else {
-            accepted = bay_accept(sU2[tid], sZ[tid], ly, sLx[tid], ACCU ? 1.0f : P.ctl->beta);
+            accepted = bay_accept(sU2[tid], sZ[tid], ly, sLx[tid], ACCU ? 1.0f : bay_beta(P));
             if (accepted) P.logfn[(size_t)P.half * P.K + k] = ly;
         }
     }
@@ -787,7 +792,7 @@ __device__ __forceinline__ void bay_gemm_accept_impl(const bay_stretch_params& P
             P.logfn[k] = ly;
         } else {
             const float* zu = P.s_zu + 3 * (size_t)k;      // stretch factor, uniform, log density
-            accepted = bay_accept(zu[1], zu[0], ly, zu[2], MODE == 1 ? 1.0f : P.ctl->beta);
+            accepted = bay_accept(zu[1], zu[0], ly, zu[2], MODE == 1 ? 1.0f : bay_beta(P));
             if (accepted && blockIdx.y == 0u) P.logfn[(size_t)P.half * P.K + k] = ly;
         }
     }
@@ -1690,7 +1695,7 @@ __device__ __forceinline__ void bay_stretch_tcr(const bay_stretch_params& P, uns
     // control words, constant during a launch: separate kernels between chunks write them,
     // and a launch after one of those starts only once it completed
     const unsigned int step0 = P.ctl->step[kind], seed0 = P.ctl->seed[kind];
-    const float a_str = P.ctl->a, beta = ACCU ? 1.0f : P.ctl->beta;
+    const float a_str = P.ctl->a, beta = ACCU ? 1.0f : bay_beta(P);
     // tiles g * gridDim.x + blockIdx.x, + G * gridDim.x, ...: consecutive tiles on
     // different SMs, every SM busy when the tiles outnumber the CTAs
     const unsigned int tile0 = g * gridDim.x + blockIdx.x;
@@ -2279,7 +2284,7 @@ __device__ __forceinline__ void bay_stretch_plain(const bay_stretch_params& P) {
     const unsigned int step = P.ctl->step[kind] + P.step_off;
     const unsigned int seed = P.ctl->seed[kind] + P.half;
     const float a = P.ctl->a;
-    const float beta = ACCU ? 1.0f : P.ctl->beta;
+    const float beta = ACCU ? 1.0f : bay_beta(P);
     const unsigned int stream = ACCU ? (P.half ? 2222u : 1111u) : (P.half ? 4444u : 3333u);
     float* X = P.xs + (size_t)P.half * P.K * DIM;
     const float* S = P.xs + (size_t)(1u - P.half) * P.K * DIM;
@@ -2610,7 +2615,7 @@ __device__ __forceinline__ void bay_stretch_tiled(const bay_stretch_params& P) {
     const unsigned int step = P.ctl->step[kind] + P.step_off;
     const unsigned int seed = P.ctl->seed[kind] + P.half;
     const float a = P.ctl->a;
-    const float beta = ACCU ? 1.0f : P.ctl->beta;
+    const float beta = ACCU ? 1.0f : bay_beta(P);
     const unsigned int stream = ACCU ? (P.half ? 2222u : 1111u) : (P.half ? 4444u : 3333u);
     float* X = P.xs + (size_t)P.half * P.K * DIM;
     const float* S = P.xs + (size_t)(1u - P.half) * P.K * DIM;
