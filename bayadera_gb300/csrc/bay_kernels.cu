@@ -7,6 +7,7 @@
 #include <atomic>
 
 #include "bay_kernels.cuh"
+#include "device/bay_normal.cuh"
 #include "device/bay_rng.cuh"
 
 namespace {
@@ -113,24 +114,35 @@ __global__ void init_uniform(float* xs, uint32_t D, uint64_t W, uint32_t seed,
 
 // N(mean, sd^2) init: element e = w*D + d uses pair p = e/2, Philox(ctr {p, 0x6e6f726d,
 // 0x77616c6b, 0xbeeff00d}, key {seed, 0x9a55a9e5}); Box-Muller in FP64 on words 0, 1, the
-// even element the cosine's.  FP64 issue bounds it, so a thread makes a pair: one element
-// per thread evaluated the pair's logarithm and both functions twice (3,276,800 elements:
-// 500 us).  Members (n, off, count, seeds): blockIdx.y's block of count values at off, so
+// even element the cosine's.  A thread makes a pair, in pairs of floats where their bound
+// settles the rounding (device/bay_normal.cuh), else in FP64, whose issue bounded the kernel:
+// 3,276,800 elements 263 us (500 us one element a thread), now 27.  Members (n, off, count, seeds): blockIdx.y's block of count values at off, so
 // that a batch of samplers is one launch.
 __device__ __forceinline__ void normal_pairs(float* xs, uint64_t n, uint32_t seed, float mean,
                                              float sd) {
     for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; 2 * p < n;
          p += (uint64_t)gridDim.x * blockDim.x) {
-        bay_u4 c;
-        c.x = (unsigned)p;
-        c.y = 0x6e6f726du;
-        c.z = 0x77616c6bu;
-        c.w = 0xbeeff00du;
-        const bay_u4 r = bay_philox4x32_10(c, seed, 0x9a55a9e5u);
-        const double rr = sqrt(-2.0 * log((double)bay_u01(r.y)));
-        const double t = 6.283185307179586 * (double)bay_u01(r.x);
-        xs[2 * p] = (float)((double)mean + (double)sd * (rr * cos(t)));
-        if (2 * p + 1 < n) xs[2 * p + 1] = (float)((double)mean + (double)sd * (rr * sin(t)));
+        bay_u4 ctr;
+        ctr.x = (unsigned)p;
+        ctr.y = 0x6e6f726du;
+        ctr.z = 0x77616c6bu;
+        ctr.w = 0xbeeff00du;
+        const bay_u4 r = bay_philox4x32_10(ctr, seed, 0x9a55a9e5u);
+        const float u0 = bay_u01(r.x), u1 = bay_u01(r.y);
+        const bay_df radius = bay_df_radius(u1);
+        bay_df c, s;
+        bay_df_circle(u0, c, s);
+        float x0, x1;
+        const bool ok0 = bay_df_normal(mean, sd, radius, c, &x0);
+        const bool ok1 = bay_df_normal(mean, sd, radius, s, &x1);
+        if (!(ok0 && ok1)) {
+            const double rr = sqrt(-2.0 * log((double)u1));
+            const double t = 6.283185307179586 * (double)u0;
+            x0 = (float)((double)mean + (double)sd * (rr * cos(t)));
+            x1 = (float)((double)mean + (double)sd * (rr * sin(t)));
+        }
+        xs[2 * p] = x0;
+        if (2 * p + 1 < n) xs[2 * p + 1] = x1;
     }
 }
 __global__ void init_normal(float* xs, uint64_t n, uint32_t seed, float mean, float sd) {
