@@ -116,8 +116,8 @@ __global__ void init_uniform(float* xs, uint32_t D, uint64_t W, uint32_t seed,
 // 0x77616c6b, 0xbeeff00d}, key {seed, 0x9a55a9e5}); Box-Muller in FP64 on words 0, 1, the
 // even element the cosine's.  A thread makes a pair, in pairs of floats where their bound
 // settles the rounding (device/bay_normal.cuh), else in FP64, whose issue bounded the kernel:
-// 3,276,800 elements 263 us (500 us one element a thread), now 27.  Members (n, off, count, seeds): blockIdx.y's block of count values at off, so
-// that a batch of samplers is one launch.
+// 3,276,800 elements 263 us (500 us one element a thread), now 27.  Members (off, count,
+// seed): blockIdx.y's block of count values at off, so that a batch of samplers is one launch.
 __device__ __forceinline__ void normal_pairs(float* xs, uint64_t n, uint32_t seed, float mean,
                                              float sd) {
     for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; 2 * p < n;

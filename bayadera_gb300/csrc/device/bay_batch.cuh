@@ -153,7 +153,20 @@ __device__ __forceinline__ unsigned int bay_div_dim(unsigned int e, unsigned int
 // The tile's proposals in shared memory serve the model's walker terms, which read a whole
 // row per thread; from global memory, in 256-walker tiles, that chain of loads and the 130
 // elements per thread took 25 us for 48 members of up to 130 dimensions, now 7.9 us.
-template <int MODE>  // 0 bare, 1 accu, 2 log density of the current positions (all W)
+// The three launches of a half-step are programmatic dependent launches (PDL): each reads its
+// work list, the members' table and the rows, which never change while a batch runs, then
+// waits for the launch before it to complete, and lets the next one start.  Every launch
+// waits before it touches anything that an earlier one writes, so that after its wait all
+// earlier launches are complete.  (The persistent launch has its grid barriers instead.)
+template <bool PDL>
+__device__ __forceinline__ void bay_batch_wait() {
+    if (PDL) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+}
+
+template <int MODE, bool PDL>  // 0 bare, 1 accu, 2 log density of the current positions (all W)
 __device__ __forceinline__ void bay_batch_propose_impl(const bay_batch_params& P, unsigned int idx) {
     extern __shared__ __align__(16) float bay_bsm[];
     __shared__ float sZ[32];
@@ -166,6 +179,7 @@ __device__ __forceinline__ void bay_batch_propose_impl(const bay_batch_params& P
     const unsigned int k = T.k0 + tid;
     const unsigned int nt = nk - T.k0 < T.n ? nk - T.k0 : T.n;   // walkers of the tile
     const unsigned int kind = MODE == 1 ? 1u : 0u;
+    bay_batch_wait<PDL>();
     if (MODE != 2 && tid < nt) {
         const unsigned int stream = MODE == 1 ? (P.half ? 2222u : 1111u) : (P.half ? 4444u : 3333u);
         bay_u4 c;
@@ -254,7 +268,7 @@ __device__ __forceinline__ void bay_batch_propose_impl(const bay_batch_params& P
 #else
 #define BAY_HAS_TERM4 0
 #endif
-template <int MODE, unsigned int WPT>  // MODE 0: move (K walkers), 2: log density of all W
+template <int MODE, unsigned int WPT, bool PDL>  // MODE 0: move (K walkers), 2: log density of all W
 __device__ __forceinline__ void bay_batch_rows_impl(const bay_batch_params& P, unsigned int idx) {
     extern __shared__ __align__(16) float bay_bsm[];
     const bay_bitem I = P.items[idx];
@@ -270,8 +284,24 @@ __device__ __forceinline__ void bay_batch_rows_impl(const bay_batch_params& P, u
     float* Rs = Pr + ((wpc * BAY_PREP_LEN + 3u) & ~3u);                // [nr][BAY_ROW_STRIDE]
     float* red = Rs + M.chunk_rows * BAY_ROW_STRIDE;                   // [256][WPT][2]
     const unsigned int nv = nk - I.k0 < wpc ? nk - I.k0 : wpc;   // walkers of the item
-    // stage the item's walkers, their prep values and its chunk of rows (coalesced,
-    // every load issued before any is used)
+    // the item's chunk of rows first: they do not depend on the launch before
+    const float* Rg = P.params + M.params + r0 * BAY_ROW_LEN;
+    // a row per thread: its BAY_ROW_LEN floats (adjacent lanes, adjacent rows: every byte
+    // of the loaded sectors used), stored as 16-byte words (padding zero)
+#pragma unroll 2
+    for (unsigned int rr = tid; rr < nr; rr += blockDim.x) {
+        const float* src = Rg + (size_t)rr * BAY_ROW_LEN;
+        float v[BAY_ROW_STRIDE];
+#pragma unroll
+        for (int i = 0; i < BAY_ROW_STRIDE; ++i) v[i] = i < BAY_ROW_LEN ? __ldg(src + i) : 0.0f;
+#pragma unroll
+        for (int q = 0; q < BAY_ROW_STRIDE / 4; ++q)
+            *reinterpret_cast<float4*>(Rs + rr * BAY_ROW_STRIDE + 4 * q) =
+                make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    }
+    // then the item's walkers and their prep values (coalesced, every load issued before any
+    // is used)
+    bay_batch_wait<PDL>();
     const float* Yg = P.y + M.xs + (size_t)I.k0 * dim;
     {
         // warp by warp, no division by the runtime dimension: one walker per warp pass
@@ -295,20 +325,6 @@ __device__ __forceinline__ void bay_batch_rows_impl(const bay_batch_params& P, u
         const unsigned int ww = e / BAY_PREP_LEN, i = e - ww * BAY_PREP_LEN;
         if (VEC) Pr[((ww >> 2) * BAY_PREP_LEN + i) * 4u + (ww & 3u)] = v;
         else Pr[e] = v;
-    }
-    const float* Rg = P.params + M.params + r0 * BAY_ROW_LEN;
-    // a row per thread: its BAY_ROW_LEN floats (adjacent lanes, adjacent rows: every byte
-    // of the loaded sectors used), stored as 16-byte words (padding zero)
-#pragma unroll 2
-    for (unsigned int rr = tid; rr < nr; rr += blockDim.x) {
-        const float* src = Rg + (size_t)rr * BAY_ROW_LEN;
-        float v[BAY_ROW_STRIDE];
-#pragma unroll
-        for (int i = 0; i < BAY_ROW_STRIDE; ++i) v[i] = i < BAY_ROW_LEN ? __ldg(src + i) : 0.0f;
-#pragma unroll
-        for (int q = 0; q < BAY_ROW_STRIDE / 4; ++q)
-            *reinterpret_cast<float4*>(Rs + rr * BAY_ROW_STRIDE + 4 * q) =
-                make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
     }
     __syncthreads();
     // walkers fastest: a warp's lanes are up to 32 walkers on the same row (a broadcast)
@@ -462,7 +478,7 @@ __device__ __forceinline__ void bay_batch_rows_impl(const bay_batch_params& P, u
 // CTA per tile moved up to 130 elements per thread and, for the sums, walked 256 rows per
 // thread: 22 us bare, 35 us accu for 48 members, now 6.2 and 8.5 us.  The accu sums go over a staged copy: thread (coordinate,
 // group of 32 walkers), compensated in walker order, the eight groups combined in order.
-template <int MODE>  // 0 bare, 1 accu, 2 log density of the current positions
+template <int MODE, bool PDL>  // 0 bare, 1 accu, 2 log density of the current positions
 __device__ __forceinline__ void bay_batch_accept_impl(const bay_batch_params& P, unsigned int idx) {
     extern __shared__ __align__(16) float bay_bsm[];   // accu: [256][33] new positions
     const bay_btile T = P.atiles[idx];
@@ -471,6 +487,7 @@ __device__ __forceinline__ void bay_batch_accept_impl(const bay_batch_params& P,
     const unsigned int dim = M.dim, tid = threadIdx.x;
     const unsigned int k = T.k0 + tid;
     const bool valid = k < nk;
+    if (PDL) asm volatile("griddepcontrol.wait;" ::: "memory");   // (lets the next start below)
     bool accepted = false;
     if (valid) {
         const size_t wk = (size_t)M.walker0 + k;
@@ -530,6 +547,7 @@ __device__ __forceinline__ void bay_batch_accept_impl(const bay_batch_params& P,
             }
         }
     }
+    if (PDL) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // (also: the persistent launch's next tile rewrites sAcc and the staged positions only
     // after every thread has read them)
     __syncthreads();
@@ -581,40 +599,40 @@ __device__ __forceinline__ void bay_batch_means_impl(const bay_batch_params& P) 
 }
 
 extern "C" __global__ void __launch_bounds__(256) bay_batch_propose_bare(bay_batch_params P) {
-    bay_batch_propose_impl<0>(P, blockIdx.x);
+    bay_batch_propose_impl<0, true>(P, blockIdx.x);
 }
 extern "C" __global__ void __launch_bounds__(256) bay_batch_propose_accu(bay_batch_params P) {
-    bay_batch_propose_impl<1>(P, blockIdx.x);
+    bay_batch_propose_impl<1, true>(P, blockIdx.x);
 }
 extern "C" __global__ void __launch_bounds__(256) bay_batch_propose_logfn(bay_batch_params P) {
-    bay_batch_propose_impl<2>(P, blockIdx.x);
+    bay_batch_propose_impl<2, true>(P, blockIdx.x);
 }
 extern "C" __global__ void __launch_bounds__(256) bay_batch_rows_move(bay_batch_params P) {
-    bay_batch_rows_impl<0, 1u>(P, blockIdx.x);
+    bay_batch_rows_impl<0, 1u, true>(P, blockIdx.x);
 }
 extern "C" __global__ void __launch_bounds__(256) bay_batch_rows_logfn(bay_batch_params P) {
-    bay_batch_rows_impl<2, 1u>(P, blockIdx.x);
+    bay_batch_rows_impl<2, 1u, true>(P, blockIdx.x);
 }
 extern "C" __global__ void __launch_bounds__(256) bay_batch_rows_move2(bay_batch_params P) {
-    bay_batch_rows_impl<0, 2u>(P, blockIdx.x);
+    bay_batch_rows_impl<0, 2u, true>(P, blockIdx.x);
 }
 extern "C" __global__ void __launch_bounds__(256) bay_batch_rows_logfn2(bay_batch_params P) {
-    bay_batch_rows_impl<2, 2u>(P, blockIdx.x);
+    bay_batch_rows_impl<2, 2u, true>(P, blockIdx.x);
 }
 extern "C" __global__ void __launch_bounds__(256) bay_batch_rows_move4(bay_batch_params P) {
-    bay_batch_rows_impl<0, 4u>(P, blockIdx.x);
+    bay_batch_rows_impl<0, 4u, true>(P, blockIdx.x);
 }
 extern "C" __global__ void __launch_bounds__(256) bay_batch_rows_logfn4(bay_batch_params P) {
-    bay_batch_rows_impl<2, 4u>(P, blockIdx.x);
+    bay_batch_rows_impl<2, 4u, true>(P, blockIdx.x);
 }
 extern "C" __global__ void __launch_bounds__(256) bay_batch_accept_bare(bay_batch_params P) {
-    bay_batch_accept_impl<0>(P, blockIdx.x);
+    bay_batch_accept_impl<0, true>(P, blockIdx.x);
 }
 extern "C" __global__ void __launch_bounds__(256) bay_batch_accept_accu(bay_batch_params P) {
-    bay_batch_accept_impl<1>(P, blockIdx.x);
+    bay_batch_accept_impl<1, true>(P, blockIdx.x);
 }
 extern "C" __global__ void __launch_bounds__(256) bay_batch_accept_logfn(bay_batch_params P) {
-    bay_batch_accept_impl<2>(P, blockIdx.x);
+    bay_batch_accept_impl<2, true>(P, blockIdx.x);
 }
 extern "C" __global__ void __launch_bounds__(128) bay_batch_means(bay_batch_params P) {
     bay_batch_means_impl(P);
@@ -638,17 +656,17 @@ __device__ __forceinline__ void bay_batch_run_impl(bay_batch_params P, unsigned 
                                P.gbar_extra))
                 return;
             for (unsigned int t = blockIdx.x; t < P.n_ptiles; t += gridDim.x)
-                bay_batch_propose_impl<MODE>(P, t);
+                bay_batch_propose_impl<MODE, false>(P, t);
             if (!bay_grid_sync(&P.ctl->gbar_count, &P.ctl->abort, &P.ctl->status, gridDim.x, ++k,
                                P.gbar_extra))
                 return;
             for (unsigned int i = blockIdx.x; i < P.n_items; i += gridDim.x)
-                bay_batch_rows_impl<0, WPT>(P, i);
+                bay_batch_rows_impl<0, WPT, false>(P, i);
             if (!bay_grid_sync(&P.ctl->gbar_count, &P.ctl->abort, &P.ctl->status, gridDim.x, ++k,
                                P.gbar_extra))
                 return;
             for (unsigned int t = blockIdx.x; t < P.n_atiles; t += gridDim.x)
-                bay_batch_accept_impl<MODE>(P, t);
+                bay_batch_accept_impl<MODE, false>(P, t);
         }
     }
 }
