@@ -34,7 +34,15 @@ inline REAL logistic_term(const REAL eta, const REAL* aux, const uint64_t row, c
 // [1, 2), of the even and the odd rows' products and their exponents' sum (an integer's
 // bits), and carry_end gives the product's -log as hi + lo.  A multiplication's relative
 // rounding error, 2^-24 at most, is one of the sum; a fast-math logarithm a row has an
-// absolute one of about 2^-23.
+// absolute one of about 2^-23.  The exponential's argument is raised by 4e-8: fast math's
+// exp2 comes out low by that much of an octave on average, which no longer cancels against the
+// logarithms' mean error.  Relative RMS errors against 64 bits over 1,048,576 x 64, 100,000 x 20,
+// 50,007 x 128, 400,000 x 200 and 10,000 x 3 (rows x features): a logarithm a row 5.2, 4.5, 6.9,
+// 10.7 and 2.5e-8; this without the raise 5.5, 4.5, 7.4, 11.2 and 2.8e-8, with it 5.2, 4.4,
+// 6.9, 10.2 and 2.5e-8.
+inline REAL logistic_exp_neg_abs(const REAL eta) {
+    return exp2f(fmaf(fabsf(eta), -1.44269504f, 4.0e-8f));
+}
 inline void logistic_carry_init(REAL* carry) {
     carry[0] = carry[1] = 1.0f;
     carry[2] = __int_as_float(0);
@@ -44,7 +52,7 @@ inline REAL logistic_terms16(const REAL* eta, const REAL* aux, const uint64_t ro
     bay_f2 p = bay_f2_of(carry[0], carry[1]), s = bay_f2_of(0.0f, 0.0f), m = s;
 #pragma unroll
     for (int i = 0; i < 16; i += 2) {
-        const bay_f2 t = bay_f2_of(expf(-fabsf(eta[i])), expf(-fabsf(eta[i + 1])));
+        const bay_f2 t = bay_f2_of(logistic_exp_neg_abs(eta[i]), logistic_exp_neg_abs(eta[i + 1]));
         p = bay_f2_fma(p, t, p);
         s = bay_f2_fma(bay_f2_of(aux[i], aux[i + 1]), bay_f2_of(eta[i], eta[i + 1]), s);
         m = bay_f2_add(m, bay_f2_of(fmaxf(eta[i], 0.0f), fmaxf(eta[i + 1], 0.0f)));
