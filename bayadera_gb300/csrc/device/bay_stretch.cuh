@@ -1474,6 +1474,27 @@ __device__ __forceinline__ void bay_tr_ld8(const float* row, unsigned int u, boo
     }
 }
 
+// The gather of the resident tensor-core form takes rows in items of BAY_TR_V dims.  Rows of
+// at most 64 dims, even: of what one aligned load brings, 16 or 8 bytes, so that consecutive
+// threads read consecutive addresses (8-dim items read every row's sectors 2 to 4 times from
+// L1): 65,536 walkers of 50 and of 20 dims 7.1 -> 6.6 and 5.5 -> 5.0 us a launch.  Else 8
+// dims, a whole unit of the A operand: longer rows take several rounds of loads either way
+// (98 and 100 dims 13.2 -> 13.5 and 27.0 -> 27.2 us with the short items), odd ones single
+// floats whose halves would go to the operand one at a time or in a pass of their own (63
+// dims 7.6 -> 8.3 us).
+#define BAY_TR_V (DIM > 64u || DIM % 2u ? 8u : (DIM % 4u ? 2u : 4u))
+__device__ __forceinline__ void bay_tr_ld(const float* row, unsigned int u, bool ok, float (&v)[8]) {
+    bay_tr_ld8(row, u, ok, v);
+}
+__device__ __forceinline__ void bay_tr_ld(const float* row, unsigned int u, bool ok, float (&v)[4]) {
+    const float4 a = ok ? *(const float4*)(row + 4u * u) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ void bay_tr_ld(const float* row, unsigned int u, bool ok, float (&v)[2]) {
+    const float2 a = ok ? *(const float2*)(row + 2u * u) : make_float2(0.0f, 0.0f);
+    v[0] = a.x; v[1] = a.y;
+}
+
 // the store counterpart of bay_tr_ld8 (dims past DIM are not written)
 __device__ __forceinline__ void bay_tr_st8(float* row, unsigned int u, const float (&v)[8]) {
     const unsigned int d0 = 8u * u;
@@ -1500,6 +1521,22 @@ __device__ __forceinline__ void bay_tr_put_a(unsigned int s_a, unsigned int w, u
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
                  ::"r"(s_a + BAY_TC_KC * BAY_TR_ATOM + off), "r"(lw[0]), "r"(lw[1]), "r"(lw[2]),
                  "r"(lw[3]) : "memory");
+}
+// its halves (4 features) and quarters (2 features), the same places
+__device__ __forceinline__ void bay_tr_put_a(unsigned int s_a, unsigned int w, unsigned int u,
+                                             const unsigned int (&hw)[2], const unsigned int (&lw)[2]) {
+    const unsigned int off = (u >> 4) * BAY_TR_ATOM + w * 128u + ((((u >> 1) & 7u) ^ (w & 7u)) << 4) +
+                             8u * (u & 1u);
+    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(s_a + off), "r"(hw[0]), "r"(hw[1]) : "memory");
+    asm volatile("st.shared.v2.b32 [%0], {%1, %2};"
+                 ::"r"(s_a + BAY_TC_KC * BAY_TR_ATOM + off), "r"(lw[0]), "r"(lw[1]) : "memory");
+}
+__device__ __forceinline__ void bay_tr_put_a(unsigned int s_a, unsigned int w, unsigned int u,
+                                             const unsigned int (&hw)[1], const unsigned int (&lw)[1]) {
+    const unsigned int off = (u >> 5) * BAY_TR_ATOM + w * 128u + ((((u >> 2) & 7u) ^ (w & 7u)) << 4) +
+                             4u * (u & 3u);
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(s_a + off), "r"(hw[0]) : "memory");
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(s_a + BAY_TC_KC * BAY_TR_ATOM + off), "r"(lw[0]) : "memory");
 }
 
 // Grid barrier k (k = 1, 2, ... within a launch) of a cooperative launch (every CTA
@@ -1559,11 +1596,12 @@ __device__ __forceinline__ int bay_gsync_count(unsigned int g, bool p) {
                  : "=r"(n) : "r"(g + 1u), "r"((unsigned int)p) : "memory");
     return n;
 }
-__device__ __forceinline__ bool bay_gsync_and(unsigned int g, bool p) {
+// n = 256: the group's threads; 128: those that still take part
+__device__ __forceinline__ bool bay_gsync_and(unsigned int g, bool p, unsigned int n) {
     unsigned int r;
-    asm volatile("{\n .reg .pred q, o;\n setp.ne.u32 q, %2, 0;\n bar.red.and.pred o, %1, 256, q;\n"
+    asm volatile("{\n .reg .pred q, o;\n setp.ne.u32 q, %2, 0;\n bar.red.and.pred o, %1, %3, q;\n"
                  " selp.u32 %0, 1, 0, o;\n}\n"
-                 : "=r"(r) : "r"(g + 1u), "r"((unsigned int)p) : "memory");
+                 : "=r"(r) : "r"(g + 1u), "r"((unsigned int)p), "r"(n) : "memory");
     return r != 0u;
 }
 
@@ -1703,6 +1741,14 @@ __device__ __forceinline__ void bay_stretch_tcr(const bay_stretch_params& P, uns
     constexpr unsigned int NU = (DIM + 7u) / 8u;               // 8-dim units of a row
     constexpr unsigned int NQ = BAY_TR_W * NU;                  // (walker, unit) items
     constexpr unsigned int IB = 2u;                             // items in flight per thread
+    // the gather's items: V consecutive dims of a row
+    constexpr unsigned int V = BAY_TR_V, RV = (DIM + V - 1u) / V;   // items of a row
+    constexpr unsigned int NV = BAY_TR_W * RV;                       // of a tile
+    constexpr unsigned int NB = (NV + 255u) / 256u;                  // of a thread
+    // in flight per thread: 16 floats of each row, 32 where the shared memory leaves an SM 512
+    // threads at most (80 dims 12.8 -> 12.1 us a launch)
+    constexpr unsigned int FL = DIM > 64u && !PERSIST ? 32u : 16u;
+    constexpr unsigned int CH = FL / V < NB ? FL / V : NB;
     // 2. proposals (Philox, z, partner) and the current log densities of a tile's walkers
     auto proposals = [&](unsigned int tile, unsigned int half, unsigned int step) {
         const unsigned int k0 = tile * BAY_TR_W;
@@ -1725,20 +1771,33 @@ __device__ __forceinline__ void bay_stretch_tcr(const bay_stretch_params& P, uns
     // the first gather pass's own rows (the tile's walkers): kept in registers, or, in the
     // persistent form (64 registers a thread at 1,024 threads), parked in Yw by the thread
     // that later reads them back
-    float xpre[IB][8];
+    float xpre[CH][V];
     auto own_rows = [&](const float* Xt, unsigned int nt) {
 #pragma unroll
-        for (unsigned int b = 0; b < IB; ++b) {
+        for (unsigned int b = 0; b < CH; ++b) {
             const unsigned int q = b * 256u + tid;
-            const unsigned int w = q / NU, u = q - w * NU;
-            bay_tr_ld8(Xt + (size_t)w * DIM, u, q < NQ && w < nt, xpre[b]);
-            if (PERSIST && q < NQ) {
+            const unsigned int w = q / RV, u = q - w * RV;
+            bay_tr_ld(V == 8u ? Xt + (size_t)w * DIM : Xt + V * (q - u), u, q < nt * RV, xpre[b]);
+            if (PERSIST && q < NV) {
 #pragma unroll
-                for (unsigned int i = 0; i < 8u; ++i)
-                    if (8u * u + i < DIM) Yw[w * BAY_TR_DPAD + 8u * u + i] = xpre[b][i];
+                for (unsigned int i = 0; i < V; ++i)
+                    if (V * u + i < DIM) Yw[w * BAY_TR_DPAD + V * u + i] = xpre[b][i];
             }
         }
     };
+#if BAY_GEMM_COEF == 0
+    // the A operand's 16-byte units past the row's dims, zero for every tile (a unit with
+    // some of them gets those later)
+    {
+        constexpr unsigned int U0 = V == 8u ? NU : DIM / 8u, U1 = BAY_TC_KC * 8u;
+        constexpr unsigned int NZ = U1 > U0 ? U1 - U0 : 0u;
+        const unsigned int zw[4] = {0u, 0u, 0u, 0u};
+        for (unsigned int q = tid; q < BAY_TR_W * NZ; q += 256u) {
+            const unsigned int w = q / (NZ ? NZ : 1u);
+            bay_tr_put_a(s_a, w, U0 + (q - w * NZ), zw, zw);
+        }
+    }
+#endif
     if (!PERSIST) {
         // One launch per half-step: this half's walkers last moved two launches back, so
         // their rows and log densities, like the draws, are final once the previous launch
@@ -1782,51 +1841,51 @@ __device__ __forceinline__ void bay_stretch_tcr(const bay_stretch_params& P, uns
         own_rows(Xt, nt);
     }
     bay_gsync(g);
-    // 3. Y of the tile (walker-major rows of odd stride) from (walker, 8-dim unit) items:
-    //    consecutive threads take consecutive units of a row (the tile's own rows are one
-    //    contiguous block, a partner's row is 4 * DIM contiguous bytes), IB items' loads in
-    //    flight per thread; with the coefficients at dim 0 the same thread splits its unit
-    //    into bf16 hi + lo and writes it to the A operand
-    for (unsigned int q0 = 0; q0 < NQ; q0 += IB * 256u) {
-        float xv[IB][8], sv[IB][8];
+    // 3. Y of the tile (walker-major rows of odd stride): consecutive threads take
+    //    consecutive items of a row (the tile's own rows are one contiguous block, a
+    //    partner's row is 4 * DIM contiguous bytes), CH items' loads in flight per thread;
+    //    with the coefficients at dim 0 the same thread splits its item into bf16 hi + lo
+    //    and writes it to the A operand
+    for (unsigned int q0 = 0; q0 < NV; q0 += CH * 256u) {
+        float xv[CH][V], sv[CH][V];
 #pragma unroll
-        for (unsigned int b = 0; b < IB; ++b) {
+        for (unsigned int b = 0; b < CH; ++b) {
             const unsigned int q = q0 + b * 256u + tid;
-            const unsigned int w = q / NU, u = q - w * NU;
-            const bool ok = q < NQ && w < nt;
+            const unsigned int w = q / RV, u = q - w * RV;
+            const bool ok = q < nt * RV;
             if (q0 == 0u && PERSIST) {
 #pragma unroll
-                for (unsigned int i = 0; i < 8u; ++i)
-                    xv[b][i] = (q < NQ && 8u * u + i < DIM) ? Yw[w * BAY_TR_DPAD + 8u * u + i] : 0.0f;
+                for (unsigned int i = 0; i < V; ++i)
+                    xv[b][i] = (q < NV && V * u + i < DIM) ? Yw[w * BAY_TR_DPAD + V * u + i] : 0.0f;
             } else if (q0 == 0u) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) xv[b][i] = xpre[b][i];
+                for (unsigned int i = 0; i < V; ++i) xv[b][i] = xpre[b][i];
             } else {
-                bay_tr_ld8(Xt + (size_t)w * DIM, u, ok, xv[b]);
+                bay_tr_ld(V == 8u ? Xt + (size_t)w * DIM : Xt + V * (q - u), u, ok, xv[b]);
             }
-            if (!LOGFN_ONLY) bay_tr_ld8(S + (size_t)sJ[g][ok ? w : 0u] * DIM, u, ok, sv[b]);
+            if (!LOGFN_ONLY) bay_tr_ld(S + (size_t)sJ[g][ok ? w : 0u] * DIM, u, ok, sv[b]);
         }
 #pragma unroll
-        for (unsigned int b = 0; b < IB; ++b) {
+        for (unsigned int b = 0; b < CH; ++b) {
             const unsigned int q = q0 + b * 256u + tid;
-            if (q < NQ) {
-                const unsigned int w = q / NU, u = q - w * NU;
-                float y[8];
+            if (q < NV) {
+                const unsigned int w = q / RV, u = q - w * RV;
+                float y[V];
                 const float z = LOGFN_ONLY ? 0.0f : sZ[g][w];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (unsigned int i = 0; i < V; ++i) {
                     y[i] = LOGFN_ONLY ? xv[b][i]
                                       : (w < nt ? __fmaf_rn(z, __fsub_rn(xv[b][i], sv[b][i]), sv[b][i]) : 0.0f);
-                    if (8u * u + i < DIM) Yw[w * BAY_TR_DPAD + 8u * u + i] = y[i];
+                    if (V * u + i < DIM) Yw[w * BAY_TR_DPAD + V * u + i] = y[i];
                 }
 #if BAY_GEMM_COEF == 0
-                if (u < BAY_TC_KC * 8u) {
-                    unsigned int hw[4], lw[4];
+                if (V * u < BAY_TC_KC * 64u) {
+                    unsigned int hw[V / 2u], lw[V / 2u];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const unsigned int f = 8u * u + 2u * i;
-                        bay_split_bf16x2(f < BAY_GEMM_F ? y[2 * i] : 0.0f,
-                                         f + 1u < BAY_GEMM_F ? y[2 * i + 1] : 0.0f, hw[i], lw[i]);
+                    for (unsigned int i = 0; i < V; i += 2u) {
+                        const unsigned int f = V * u + i;
+                        bay_split_bf16x2(f < BAY_GEMM_F ? y[i] : 0.0f,
+                                         f + 1u < BAY_GEMM_F ? y[i + 1u] : 0.0f, hw[i / 2u], lw[i / 2u]);
                     }
                     bay_tr_put_a(s_a, w, u, hw, lw);
                 }
@@ -1834,17 +1893,7 @@ __device__ __forceinline__ void bay_stretch_tcr(const bay_stretch_params& P, uns
             }
         }
     }
-#if BAY_GEMM_COEF == 0
-    // 4. A units past the row's last unit are zero
-    if (BAY_TC_KC * 8u > NU) {
-        constexpr unsigned int NZ = BAY_TC_KC * 8u > NU ? BAY_TC_KC * 8u - NU : 1u;
-        const unsigned int zw[4] = {0u, 0u, 0u, 0u};
-        for (unsigned int q = tid; q < BAY_TR_W * NZ; q += 256u) {
-            const unsigned int w = q / NZ;
-            bay_tr_put_a(s_a, w, NU + (q - w * NZ), zw, zw);
-        }
-    }
-#else
+#if BAY_GEMM_COEF != 0
     // 4. the A operand from Yw (coefficients at dim BAY_GEMM_COEF): 16-byte units of hi, lo
     bay_gsync(g);
     for (unsigned int q = tid; q < BAY_TR_W * BAY_TC_KC * 8u; q += 256u) {
@@ -1862,6 +1911,45 @@ __device__ __forceinline__ void bay_stretch_tcr(const bay_stretch_params& P, uns
 #endif
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // A visible to the MMAs
     bay_gsync(g);
+    // One launch per half-step (FAST): the MMAs and all that follows are the business of the
+    // epilogue's warps 0, 1, 4 and 5; warps 2, 3, 6 and 7 leave here, after the statistics of
+    // the previous half-step in an accu launch -- this tile of the other half, final since
+    // the previous launch completed and not written by this one: (step_off, 0) from the
+    // launch of half 1, (step_off - 1, 1) from the launch of half 0 (the chunk's last one has
+    // a launch of its own).  The same slots and order as bay_tr_sums_pass1 / pass2.
+    // Their loads so run under the MMAs and the epilogue: 30,000 walkers of 99 dims 16.3 ->
+    // 14.5 us an accu launch, 65,536 of 50 8.0 -> 7.8.
+    constexpr bool FAST = !PERSIST && !LOGFN_ONLY;
+    const unsigned int hand_id = 1u + G + g;        // named barriers 1..G are the groups'
+    if (FAST && (warp & 2u)) {
+        if (ACCU && P.means_cap != 0 && (half == 1u || step_off > 0u)) {
+            float* const prev_out = P.part +
+                ((size_t)(half == 1u ? step_off : step_off - 1u) * 2 + (1u - half)) * DIM * ntiles + tile;
+            const unsigned int i0 = (warp >> 2) * 64u + (warp & 1u) * 32u + lane;
+            const float* rows = P.xs + (size_t)(1u - half) * P.K * DIM + (size_t)k0 * DIM;
+            for (unsigned int t = i0; t < BAY_TR_NG * DIM; t += 128u) {
+                const unsigned int wg = t / DIM, d = t - wg * DIM;
+                float v = 0.0f;
+#pragma unroll
+                for (unsigned int i = 0; i < BAY_TR_WG; ++i) {
+                    const unsigned int w = wg * BAY_TR_WG + i;
+                    if (w < nt) v = __fadd_rn(v, rows[(size_t)w * DIM + d]);
+                }
+                if (BAY_TR_NG == 1u) prev_out[(size_t)d * ntiles] = v;
+                else red2[t] = v;
+            }
+            if (BAY_TR_NG > 1u) {
+                asm volatile("bar.sync %0, 128;" ::"r"(1u + 2u * G + g) : "memory");
+                for (unsigned int d = i0; d < DIM; d += 128u) {
+                    float a = 0.0f;
+#pragma unroll
+                    for (unsigned int wg = 0; wg < BAY_TR_NG; ++wg) a = __fadd_rn(a, red2[wg * DIM + d]);
+                    prev_out[(size_t)d * ntiles] = a;
+                }
+            }
+        }
+        continue;                                   // the tile is done (one per launch)
+    }
     // 5. one thread: wait for the image, issue the MMAs, commit; the others precompute
     if (tid == 0) {
         unsigned int ok = bay_tc_wait(bar_img, 0u, nullptr, status) ? 1u : 0u;   // once done, stays
@@ -1872,6 +1960,9 @@ __device__ __forceinline__ void bay_stretch_tcr(const bay_stretch_params& P, uns
             for (unsigned int c = 0; c < BAY_TC_KC; ++c) {
 #pragma unroll
                 for (unsigned int ks = 0; ks < 4u; ++ks) {
+                    // past the features both sides are zeros (4,096 walkers of 98 and of 20
+                    // dims 6.2 -> 6.1 and 3.16 -> 3.06 us a launch without those products)
+                    if (64u * c + 16u * ks >= BAY_GEMM_F) break;
                     const unsigned int ao = c * BAY_TR_ATOM + 32u * ks;
                     const unsigned int bo = c * NP * 128u + 32u * ks;
                     const unsigned long long ah = bay_sdesc(s_a + ao);
@@ -1900,60 +1991,14 @@ __device__ __forceinline__ void bay_stretch_tcr(const bay_stretch_params& P, uns
         for (int i = 0; i < BAY_PREP_LEN; ++i) sPrep[g][tid][i] = pr[i];
         sW[g][tid] = wt;
     }
-    // accu, one launch per half-step: while the MMAs run, the statistics of the previous
-    // half-step -- this tile of the other half, final since the previous launch completed
-    // and not written by this one: (step_off, 0) from the launch of half 1, (step_off - 1,
-    // 1) from the launch of half 0 (the chunk's last one has a launch of its own)
-    const bool prev_stats = ACCU && !PERSIST && P.means_cap != 0 && (half == 1u || step_off > 0u);
-    float* const prev_out = prev_stats
-        ? P.part + ((size_t)(half == 1u ? step_off : step_off - 1u) * 2 + (1u - half)) * DIM * ntiles + tile
-        : nullptr;
-    // (one launch per half-step: the statistics run on the warps idle in the epilogue)
-    if (prev_stats && PERSIST)
-        bay_tr_sums_pass1(P.xs + (size_t)(1u - half) * P.K * DIM + (size_t)k0 * DIM, nt, tid,
-                          red2, prev_out, ntiles);
     // every thread waits for the MMAs (bounded; the commit arrives even if none were issued)
     // and observes the image copy itself before reading the aux values it brought
     const bool mma_done = bay_tc_wait(bar_mma, mma_par, nullptr, status);
     mma_par ^= 1u;
     const bool img_done = bay_tc_wait(bar_img, 0u, nullptr, status);
-    // one verdict for the whole CTA (a wait that gave up in any thread fails the tile)
-    const bool ok = bay_gsync_and(g, mma_done && img_done) && sOk[g] != 0u;
+    // one verdict for the group's epilogue (a wait that gave up in any thread fails the tile)
+    const bool ok = bay_gsync_and(g, mma_done && img_done, FAST ? 128u : 256u) && sOk[g] != 0u;
     bay_tc_fence_after();
-    // One launch per half-step (FAST): the epilogue's warps 0 and 1 decide their walkers
-    // themselves once warps 4 and 5 have handed over the other half of the rows (a 128-
-    // thread named barrier), and write back their own rows; no group barrier follows.
-    // Meanwhile warps 2, 3, 6 and 7 finish the previous half-step's statistics (pass 1
-    // ended before the barrier above).
-    constexpr bool FAST = !PERSIST && !LOGFN_ONLY;
-    const unsigned int hand_id = 1u + G + g;        // named barriers 1..G are the groups'
-    if (FAST && prev_stats && (warp & 2u)) {
-        // warps 2, 3, 6, 7 (128 threads, idle in the epilogue): both passes of the previous
-        // half-step's statistics, the same slots and order as bay_tr_sums_pass1 / pass2,
-        // with a 128-thread named barrier between them
-        const unsigned int i0 = (warp >> 2) * 64u + (warp & 1u) * 32u + lane;
-        const float* rows = P.xs + (size_t)(1u - half) * P.K * DIM + (size_t)k0 * DIM;
-        for (unsigned int t = i0; t < BAY_TR_NG * DIM; t += 128u) {
-            const unsigned int wg = t / DIM, d = t - wg * DIM;
-            float v = 0.0f;
-#pragma unroll
-            for (unsigned int i = 0; i < BAY_TR_WG; ++i) {
-                const unsigned int w = wg * BAY_TR_WG + i;
-                if (w < nt) v = __fadd_rn(v, rows[(size_t)w * DIM + d]);
-            }
-            if (BAY_TR_NG == 1u) prev_out[(size_t)d * ntiles] = v;
-            else red2[t] = v;
-        }
-        if (BAY_TR_NG > 1u) {
-            asm volatile("bar.sync %0, 128;" ::"r"(1u + 2u * G + g) : "memory");
-            for (unsigned int d = i0; d < DIM; d += 128u) {
-                float a = 0.0f;
-#pragma unroll
-                for (unsigned int wg = 0; wg < BAY_TR_NG; ++wg) a = __fadd_rn(a, red2[wg * DIM + d]);
-                prev_out[(size_t)d * ntiles] = a;
-            }
-        }
-    }
     // 6. epilogue: warps 0, 1, 4, 5 read TMEM lanes 32 (w % 4) .. + 31 (walkers 0..63),
     //    rows [NP/2 * (w / 4), + NP/2) in 8-column loads; the two halves then combine
     if (32u * (warp & 3u) < BAY_TR_W) {
@@ -2014,7 +2059,7 @@ __device__ __forceinline__ void bay_stretch_tcr(const bay_stretch_params& P, uns
                     if (acc) {
                         P.logfn[(size_t)half * P.K + k] = ly;
                         const float* yr = &Yw[wl * BAY_TR_DPAD];
-#pragma unroll 1
+#pragma unroll 4
                         for (unsigned int u = 0; u < NU; ++u) {
                             float y[8];
 #pragma unroll
@@ -2042,7 +2087,6 @@ __device__ __forceinline__ void bay_stretch_tcr(const bay_stretch_params& P, uns
     }
     bay_tc_fence_before();
     bay_gsync(g);
-    if (prev_stats) bay_tr_sums_pass2(tid, red2, prev_out, ntiles);
     // 7. accept (one thread per walker), write-back, statistics
     bool accepted = false;
     if (tid < nt && ok) {
@@ -2159,7 +2203,7 @@ __device__ __forceinline__ void bay_stretch_tcr(const bay_stretch_params& P, uns
     }
 }
 
-// The per-launch move kernels hold BAY_TR_G tile groups per CTA (1 or 2): one matrix-image
+// The per-launch move kernels hold up to BAY_TR_G tile groups per CTA (1 or 2): one matrix-image
 // copy and one TMEM allocation serve BAY_TR_G tiles; group g takes tile g * gridDim.x +
 // blockIdx.x.  Same results for either.
 #ifndef BAY_TR_G
