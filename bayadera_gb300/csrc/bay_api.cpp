@@ -313,7 +313,8 @@ struct bay_model {
     CUkernel k_tr[6] = {};   // bare, accu, logfn, persistent bare, persistent accu, statistics
     uint32_t tc_g = 0, tc_stages = 0;
     size_t tc_smem = 0;
-    uint32_t tr_g = 1;   // resident tensor-core form: tile groups per CTA of the move kernels
+    uint32_t tr_g = 1;   // resident tensor-core form: most tile groups per CTA of the move kernels
+    bool tr_free = false;   // ... a sampler's choice
     // batch form: propose / accept in k_gp / k_ga, rows in k_gr, per-step means here
     CUkernel k_bmeans = nullptr;
     uint32_t row_len = 0;
@@ -369,6 +370,30 @@ constexpr size_t kTcSmemMax = 232448;  // opt-in dynamic shared memory per CTA, 
 constexpr size_t kBatchSmemMax = 160 * 1024;   // batched rows kernels: dynamic shared memory, at most
 constexpr uint32_t kTrWalkers = 64;  // walkers per tile of the resident tensor-core form
 constexpr uint32_t kTrGroups = 4;    // tile groups (256 threads each) per persistent CTA
+// Resident tensor-core form: dynamic shared memory of a move CTA before its tile groups
+// (alignment slack, the matrix image of np padded rows) and of a group (2 kc atoms of
+// kTrWalkers walker rows, the proposals and the reduction scratch -- at least the part of the
+// M = 128 MMA's 16 KB read that runs past the last atom, walker rows kTrWalkers..127, never
+// read back); the group stride is BAY_TR_GREG of the kernel.
+uint64_t tr_base_bytes(uint64_t rows, uint32_t features, uint32_t aux_len) {
+    const uint64_t np = (rows + 15) & ~15ull, kc = (features + 63) / 64, auxs = aux_len ? aux_len : 1;
+    return 1024 + ((2 * kc * np * 128 + np * auxs * 4 + 1023) & ~1023ull);
+}
+uint64_t tr_group_bytes(uint32_t dim, uint32_t features) {
+    const uint64_t kc = (features + 63) / 64, atom = 128ull * kTrWalkers;
+    const uint64_t tail = std::max<uint64_t>(16384 - atom, (uint64_t)kTrWalkers * (dim | 1u) * 4 + 2048);
+    return 2 * kc * atom + ((tail + 1023) & ~1023ull);
+}
+// Tile groups of a move CTA when the model leaves them free: two where an SM holds no second
+// CTA of one group (113,664 bytes each, beside 2 KB of static and 1 KB of reserved shared
+// memory), two groups fit, and the tiles are more than the SMs -- 65,536 walkers of 98 and
+// 128 dims 27.8 -> 18.9 and 24.0 -> 17.7 us a launch.  Where two such CTAs fit they overlap
+// with the next launch's and stay (94 dims 16.1, 17.4 us with two groups); with a tile an SM
+// at most two groups would leave SMs idle (4,096 walkers of 98 dims 6.2, 8.5 us).
+constexpr uint64_t kTrPairSmem = 113664;
+uint32_t tr_free_groups(uint64_t base, uint64_t greg, uint64_t tiles, uint64_t sms) {
+    return base + greg > kTrPairSmem && base + 2 * greg <= kGemmMaxSmem && tiles > sms ? 2u : 1u;
+}
 // With one sub-tile and at most 256 features the kernel holds the walker operand in tensor
 // memory (BAY_TC_ATM), which leaves its shared memory to more stages: the free choice is up to
 // 6 there too; which shapes may be asked for stays as if it were in shared memory.
@@ -1014,6 +1039,7 @@ struct Codegen {
     uint32_t tc_g = 0, tc_stages = 0;
     size_t tc_smem = 0;
     uint32_t tr_g = 1;
+    bool tr_free = false;
 };
 
 // Source and NVRTC options of a model's fused kernels (the reference's stretch-options,
@@ -1093,7 +1119,13 @@ Codegen codegen(const bay_model_desc* d, uint32_t wgs) {
                 fail(BAY_ERR_ARG, "tensor-core GEMM form: the asked sub-tiles / stages do not fit "
                                   "in shared memory");
             if (d->tc_groups > 2) fail(BAY_ERR_ARG, "tc_groups must be 0, 1 or 2");
-            g.tr_g = d->tc_groups ? d->tc_groups : 1u;
+            // free: compiled for two where a sampler may take two (a matrix of as many rows
+            // as features when their number is left to its parameters); it decides
+            g.tr_free = d->tc_groups == 0;
+            g.tr_g = d->tc_groups ? d->tc_groups
+                                  : tr_free_groups(tr_base_bytes(d->gemm_rows ? d->gemm_rows : d->gemm_features,
+                                                                 d->gemm_features, d->gemm_aux_len),
+                                                   tr_group_bytes(d->dim, d->gemm_features), 2, 1);
             opts.push_back("-DBAY_TR_G=" + std::to_string(g.tr_g) + "u");
             opts.push_back("-DBAY_GEMM_TC=1");
             opts.push_back("-DBAY_TC_G=" + std::to_string(g.tc_g));
@@ -1175,6 +1207,7 @@ int bay_model_compile(bay_ctx* c, const bay_model_desc* d, bay_model** out) {
             m->tc_stages = g.tc_stages;
             m->tc_smem = g.tc_smem;
             m->tr_g = g.tr_g;
+            m->tr_free = g.tr_free;
         }
         try {
             cu_check(g_cu.LibraryLoadData(&m->lib, cubin.data(), nullptr, nullptr, 0, nullptr,
@@ -1349,24 +1382,16 @@ static int sampler_create(bay_model* m, uint32_t seed, uint64_t walkers, const f
                 m->gemm_features <= 256) {
                 // resident on the tensor cores when the image, the walker operand and the
                 // proposals fit (layout in bay_stretch_tcr)
-                const uint64_t np = (s->gemm_rows + 15) & ~15ull, kc = (m->gemm_features + 63) / 64;
-                const uint64_t auxs = m->gemm_aux_len ? m->gemm_aux_len : 1;
-                const uint64_t img = 2 * kc * np * 128 + np * auxs * 4;
-                // image, then per tile group 2 kc atoms of kTrWalkers walker rows, the
-                // proposals and the reduction scratch -- at least the part of the M = 128
-                // MMA's 16 KB read that runs past the last atom (walker rows kTrWalkers..127,
-                // never read back); the group stride is BAY_TR_GREG of the kernel
-                const uint64_t atom = 128ull * kTrWalkers;
-                const uint64_t tail = (std::max<uint64_t>(16384 - atom,
-                                                          (uint64_t)kTrWalkers * (m->dim | 1u) * 4 + 2048) +
-                                       1023) & ~1023ull;
-                const uint64_t greg = 2 * kc * atom + tail;
-                const uint64_t base = 1024 + ((img + 1023) & ~1023ull);
+                const uint64_t np = (s->gemm_rows + 15) & ~15ull;
+                const uint64_t base = tr_base_bytes(s->gemm_rows, m->gemm_features, m->gemm_aux_len);
+                const uint64_t greg = tr_group_bytes(m->dim, m->gemm_features);
                 if (base + greg <= kGemmMaxSmem) {
                     s->tc = false;
                     s->tcr = true;
                     s->smem = (size_t)(base + greg);
                     s->tr_g = (base + m->tr_g * greg <= kGemmMaxSmem) ? m->tr_g : 1u;
+                    if (m->tr_free)
+                        s->tr_g = std::min(s->tr_g, tr_free_groups(base, greg, s->grid(), c->sm_count));
                     s->smem_move = (size_t)(base + s->tr_g * greg);
                     s->gemm_np = (uint32_t)np;
                     // persistent form: kTrGroups groups per CTA, their accumulators within
