@@ -310,6 +310,7 @@ struct bay_model {
     // shared-memory stages, dynamic shared memory
     CUkernel k_gt[2] = {nullptr, nullptr};
     // GEMM form on the tensor cores with the matrix resident: [bare, accu, logfn]
+    CUkernel k_gs = nullptr;      // resident GEMM form without tensor cores: statistics
     CUkernel k_tr[6] = {};   // bare, accu, logfn, persistent bare, persistent accu, statistics
     uint32_t tc_g = 0, tc_stages = 0;
     size_t tc_smem = 0;
@@ -699,6 +700,7 @@ struct bay_sampler {
         cfg.gridDimY = 1;
         cfg.gridDimZ = 1;
         cfg.blockDimX = tcr ? 256 * tr_g : model->cta / split;
+        if (accu && !tcr && model->form == BAY_FORM_GEMM) cfg.blockDimX += 64;   // statistics
         cfg.blockDimY = 1;
         cfg.blockDimZ = 1;
         cfg.sharedMemBytes = (unsigned)(tcr || tiled ? smem_move
@@ -774,9 +776,11 @@ struct bay_sampler {
 
     bool use_persistent() const { return tcr && persistent && tr_grid != 0; }
 
-    // per-launch resident tensor-core accu steps sum each half-step's positions in the
+    // per-launch accu steps of the resident GEMM forms sum each half-step's positions in the
     // next launch; the chunk's last half-step has a statistics launch of its own
-    bool tail_stats(bool accu) const { return accu && means_cap && tcr && !use_persistent(); }
+    bool tail_stats(bool accu) const {
+        return accu && means_cap && model->form == BAY_FORM_GEMM && !streaming && !use_persistent();
+    }
 
     // kernels one run_chunk of m steps launches
     uint32_t chunk_launches(bool accu, uint32_t m) const {
@@ -796,7 +800,8 @@ struct bay_sampler {
                 if (st == ctx->stream) bay::count_launches(1);
                 bay_stretch_params p = make_params(1, m - 1);
                 void* args[] = {&p};
-                cu_check(g_cu.LaunchKernel((CUfunction)model->k_tr[5], grid(), 1, 1, 256, 1, 1, 0,
+                cu_check(g_cu.LaunchKernel((CUfunction)(tcr ? model->k_tr[5] : model->k_gs), grid(), 1, 1,
+                                           256, 1, 1, 0,
                                            (CUstream)st, args, nullptr),
                          "cuLaunchKernel(statistics)");
             }
@@ -1281,6 +1286,7 @@ int bay_model_compile(bay_ctx* c, const bay_model_desc* d, bay_model** out) {
                     cu_check(g_cu.LibraryGetKernel(&m->k_gp[i], m->lib, gp[i]), "GetKernel(propose)");
                     cu_check(g_cu.LibraryGetKernel(&m->k_ga[i], m->lib, ga[i]), "GetKernel(accept)");
                 }
+                cu_check(g_cu.LibraryGetKernel(&m->k_gs, m->lib, "bay_gemm_stats"), "GetKernel(statistics)");
                 cu_check(g_cu.LibraryGetKernel(&m->k_gr[0], m->lib, "bay_gemm_rows_move"), "GetKernel(rows)");
                 cu_check(g_cu.LibraryGetKernel(&m->k_gr[1], m->lib, "bay_gemm_rows_logfn"), "GetKernel(rows)");
                 CUdevice dev = (CUdevice)c->device;

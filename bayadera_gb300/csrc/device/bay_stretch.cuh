@@ -294,6 +294,46 @@ __device__ void bay_accu_epilogue(const bay_stretch_params& P, bool accepted, bo
 #endif
 #define BAY_AUXS (BAY_GEMM_AUX > 0 ? BAY_GEMM_AUX : 1)
 
+// barriers of the eight warps that move a tile (accu launches have two more)
+__device__ __forceinline__ void bay_g_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ bool bay_g_or(bool p) {
+    unsigned int r;
+    asm volatile("{\n .reg .pred q, o;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred o, 1, 256, q;\n"
+                 " selp.u32 %0, 1, 0, o;\n}\n" : "=r"(r) : "r"((unsigned int)p) : "memory");
+    return r != 0u;
+}
+__device__ __forceinline__ int bay_g_count(bool p) {
+    int r;
+    asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %1, 0;\n bar.red.popc.u32 %0, 1, 256, q;\n}\n"
+                 : "=r"(r) : "r"((unsigned int)p) : "memory");
+    return r;
+}
+
+// The statistics of a tile: per-dim compensated sums of its nv walkers' positions (rows of DIM
+// floats) in walker order, dims t, t + stride, ...; out[d * gridDim.x]
+__device__ __forceinline__ void bay_g_sums(const float* rows, unsigned int nv, unsigned int t,
+                                           unsigned int stride, float* out) {
+    for (unsigned int d = t; d < DIM; d += stride) {
+        bay_cf s;
+        s.hi = 0.0f;
+        s.lo = 0.0f;
+        for (unsigned int w0 = 0; w0 < BAY_WT; w0 += 16u) {
+            float v[16];
+#pragma unroll
+            for (unsigned int i = 0; i < 16u; ++i)
+                v[i] = w0 + i < nv ? rows[(size_t)(w0 + i) * DIM + d] : 0.0f;
+#pragma unroll
+            for (unsigned int i = 0; i < 16u; ++i) {
+                bay_cf y;
+                y.hi = v[i];
+                y.lo = 0.0f;
+                if (w0 + i < nv) s = bay_cadd(s, y);
+            }
+        }
+        out[(size_t)d * gridDim.x] = __fadd_rn(s.hi, s.lo);
+    }
+}
+
 template <bool ACCU, bool LOGFN_ONLY>
 __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
     extern __shared__ __align__(128) float bay_smem[];
@@ -318,6 +358,20 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
     float* X = P.xs + (LOGFN_ONLY ? 0 : (size_t)P.half * P.K * DIM);
     const float* S = P.xs + (size_t)(1u - P.half) * P.K * DIM;
 
+    // accu: two more warps sum this tile of the other half, as the previous half-step left it
+    // ((step_off, 0) for half 1, (step_off - 1, 1) for half 0; the chunk's last half-step has
+    // a launch of its own), beside the eight that move the walkers.  At the end of the moving
+    // half's own launch the sums were a serial chain of 64 compensated additions that
+    // everything waited for: 12,290 walkers of 37 dimensions 8.3 -> 6.3 us a launch,
+    // 16,384 of 50 10.7 -> 7.4.
+    if (ACCU && tid >= 256u) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (P.means_cap != 0 && (P.half == 1u || P.step_off > 0u))
+            bay_g_sums(S + (size_t)k0 * DIM, nk - k0 < BAY_WT ? nk - k0 : BAY_WT, tid - 256u, 64u,
+                       P.part + ((size_t)(P.half == 1u ? P.step_off : P.step_off - 1u) * 2 + (1u - P.half)) *
+                           DIM * gridDim.x + blockIdx.x);
+        return;
+    }
     // 1. one TMA bulk copy (cp.async.bulk, completion counted on an mbarrier) brings the
     //    laid-out matrix and aux values into shared memory; it overlaps the proposals.
     const unsigned int lay_bytes =
@@ -328,7 +382,7 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    __syncthreads();
+    bay_g_sync();
     if (tid == 0) {
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
                      "r"(lay_bytes) : "memory");
@@ -362,7 +416,7 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
             sLx[tid] = P.logfn[(size_t)P.half * P.K + k];
         }
     }
-    __syncthreads();
+    bay_g_sync();
     {
         // The tile's own rows are one contiguous block of BAY_WT * DIM floats; element e is
         // (walker e / DIM, coordinate e % DIM), so a warp reads its own elements coalesced
@@ -394,10 +448,10 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
             }
         }
     }
-    __syncthreads();
+    bay_g_sync();
     // feature-major copy of the coefficient block for the register tiles (bank-conflict
     // free: consecutive lanes write consecutive walkers and read rows of odd stride)
-    for (unsigned int e = tid; e < BAY_GEMM_F * BAY_WT; e += blockDim.x) {
+    for (unsigned int e = tid; e < BAY_GEMM_F * BAY_WT; e += 256u) {
         const unsigned int f = e / BAY_WT, w = e - f * BAY_WT;
         Ys[e] = Yw[w * BAY_DPAD + BAY_GEMM_COEF + f];
     }
@@ -409,7 +463,7 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
                 "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
                 " selp.u32 %0, 1, 0, p;\n}\n"
                 : "=r"(done) : "r"(bar), "r"(0u) : "memory");
-        if (__syncthreads_or(!done)) {
+        if (bay_g_or(!done)) {
             if (tid == 0) atomicOr(&P.ctl->status, 1u);
             return;
         }
@@ -428,7 +482,7 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
         for (int i = 0; i < BAY_PREP_LEN; ++i) sPrep[tid][i] = pr[i];
         sW[tid] = wt;
     }
-    __syncthreads();
+    bay_g_sync();
     // 4. eta tiles and row terms
     const unsigned int wg = tid / BAY_NG, rg = tid - wg * BAY_NG;
     const unsigned int w0 = wg * BAY_RW;
@@ -445,7 +499,9 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
         for (int i = 0; i < BAY_RW; ++i)
 #pragma unroll
             for (int j = 0; j < BAY_RN; ++j) acc[i][j] = 0.0f;
-#pragma unroll 5
+        // 37, 60 and 77 dims 6.2, 6.4 and 12.6 us a launch unrolled by 5, 5.8, 6.3 and 10.7 by 10;
+        // 5.9, 9.4 and 14.9 in full
+#pragma unroll 10
         for (int f = 0; f < BAY_GEMM_F; ++f) {
             const float4 y = *reinterpret_cast<const float4*>(&Ys[f * BAY_WT + w0]);
             const float4 a = *reinterpret_cast<const float4*>(&As[(size_t)f * NP + n0]);
@@ -481,10 +537,9 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
         for (int o = BAY_NG / 2; o > 0; o >>= 1) v = bay_cadd(v, bay_cf_shfl_xor(v, o));
         if (rg == 0) sSum[w0 + i] = v;
     }
-    __syncthreads();
-    // 5. accept (one thread per walker), then the tile's rows written back cooperatively
-    //    (accepted walkers' proposals; for the accu statistics the rejected walkers' current
-    //    rows are copied into the tile), statistics
+    bay_g_sync();
+    // 5. accept (one thread per walker), then the accepted walkers' rows written back
+    //    cooperatively
     __shared__ unsigned char sAcc[BAY_WT];
     const unsigned int k = k0 + tid;
     const bool valid = tid < BAY_WT && k < nk;
@@ -504,44 +559,29 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
     }
     if (LOGFN_ONLY) return;
     if (tid < BAY_WT) sAcc[tid] = accepted ? 1 : 0;
-    const int n_acc = __syncthreads_count(accepted);
+    const int n_acc = bay_g_count(accepted);
     {
         float* Xt = X + (size_t)k0 * DIM;
         const unsigned int n_own = (nk - k0 < BAY_WT ? nk - k0 : BAY_WT) * DIM;
-        for (unsigned int e = tid; e < n_own; e += blockDim.x) {
+        for (unsigned int e = tid; e < n_own; e += 256u) {
             const unsigned int w = e / DIM, d = e - w * DIM;
             if (sAcc[w]) Xt[e] = Yw[w * BAY_DPAD + d];
-            else if (ACCU) Yw[w * BAY_DPAD + d] = Xt[e];
         }
     }
-    if (ACCU) {
-        __syncthreads();
-        if (tid == 0 && n_acc) atomicAdd(&P.ctl->accepted, (unsigned long long)n_acc);
-        if (P.means_cap != 0) {
-            float* out = P.part + ((size_t)P.step_off * 2 + P.half) * DIM * gridDim.x
-                + blockIdx.x;
-            const unsigned int nv = nk - k0 < BAY_WT ? nk - k0 : BAY_WT;
-            for (unsigned int d = tid; d < DIM; d += blockDim.x) {
-                bay_cf s;
-                s.hi = 0.0f;
-                s.lo = 0.0f;
-                for (unsigned int w = 0; w < nv; ++w) {
-                    bay_cf y;
-                    y.hi = Yw[w * BAY_DPAD + d];
-                    y.lo = 0.0f;
-                    s = bay_cadd(s, y);
-                }
-                out[(size_t)d * gridDim.x] = __fadd_rn(s.hi, s.lo);
-            }
-        }
-    }
+    if (ACCU && tid == 0 && n_acc) atomicAdd(&P.ctl->accepted, (unsigned long long)n_acc);
 }
 
 extern "C" __global__ void __launch_bounds__(256) bay_stretch_bare(bay_stretch_params P) {
     bay_stretch_gemm<false, false>(P);
 }
-extern "C" __global__ void __launch_bounds__(256) bay_stretch_accu(bay_stretch_params P) {
+extern "C" __global__ void __launch_bounds__(320) bay_stretch_accu(bay_stretch_params P) {
     bay_stretch_gemm<true, false>(P);
+}
+// the statistics of the last half-step of a chunk (half P.half, step P.step_off)
+extern "C" __global__ void __launch_bounds__(256) bay_gemm_stats(bay_stretch_params P) {
+    const unsigned int k0 = blockIdx.x * BAY_WT;
+    bay_g_sums(P.xs + ((size_t)P.half * P.K + k0) * DIM, P.K - k0 < BAY_WT ? P.K - k0 : BAY_WT, threadIdx.x,
+               256u, P.part + ((size_t)P.step_off * 2 + P.half) * DIM * gridDim.x + blockIdx.x);
 }
 extern "C" __global__ void __launch_bounds__(256) bay_logfn_all(bay_stretch_params P) {
     bay_stretch_gemm<false, true>(P);

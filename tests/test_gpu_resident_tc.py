@@ -49,13 +49,12 @@ def test_gather_groups_and_log_densities(factory, D, W):
         assert rate == other[3]
     # log densities: the split products are good to 2^-15 of each, their fp32 sum to 4 D 2^-24,
     # the row terms and their sum to 2^-21
-    P, x = precision(D).astype(np.float64), (pos if pos.shape[1] == D else pos.T).astype(np.float64)
+    P, x = precision(D).astype(np.float64), pos.T.astype(np.float64)
     want = -0.5 * np.einsum("wi,ij,wj->w", x, P, x)
     terms = 0.5 * np.einsum("wi,ij,wj->w", np.abs(x), np.abs(P), np.abs(x))
     assert np.all(np.abs(logfn - want) <= (2.0 ** -15 + 4 * D * 2.0 ** -24 + 2.0 ** -21) * terms + 1e-6)
     # the moves: the fp32 form's, but for decisions within the densities' error (two steps;
     # about 2^-15 of some D a decision, far below one in a hundred)
-    ref = run(factory, D, W, 2, tensor=False)[0]
-    ref = ref if ref.shape[1] == D else ref.T
+    ref = run(factory, D, W, 2, tensor=False)[0].T
     differ = np.count_nonzero(np.any(x != ref.astype(np.float64), axis=1))
     assert differ <= max(2, W // 50), differ
