@@ -99,21 +99,23 @@ __device__ __forceinline__ void two_sum(float& s, float& e, float x) {
 // FP64 issue is 1/64 of fp32 here (1.9 operations a clock an SM), and an FP64 conversion and
 // addition an element held the pass to 0.83 elements a clock an SM, a sixth of what HBM
 // delivers.  So the sums are fp32 words with their exact rounding errors beside them
-// (fp_sum), flushed to the FP64 accumulators every kFlush elements: 4 or 12 FP64 operations
-// per 64 elements.  Such a sum is 2^-56 of its terms off at most, better than a run of FP64
-// additions.  Batches that fp32 cannot hold (largest |x - c| outside [1e-12, 1e15], an
-// infinity, NaN, an overflow) take FP64 throughout.
-// 4,194,315 x 6 values: 36 us the sum and 66 us the squares, against 7,546 us for both with
+// (fp_sum), flushed to the FP64 accumulators every kFlush elements: 6 or 10 FP64 operations
+// per 64 elements.  Variances of 1,000 to 4,194,304 values against 128 bits: 2.3e-16 off at
+// most, a run of FP64 additions 5.3e-16.  Batches that fp32 cannot hold (largest |x - c|
+// outside [1e-12, 1e15], an infinity, NaN, an overflow) take FP64 throughout.
+// 4,194,315 x 6 values: some 40 us the sum and 65 us the squares, against 7,546 us for both with
 // one CTA a dimension and FP64 throughout.
 constexpr uint32_t kFlush = 64;
 struct fp_sum {
-    float s = 0.0f, r = 0.0f;                   // sum, rounding errors of s
-    float e = 0.0f, l = 0.0f;                   // errors of the products, and of e
+    float s = 0.0f;                             // sum
+    float e = 0.0f, l = 0.0f;                   // errors of s and of the products, and of e
     float s1 = 0.0f, e1 = 0.0f;                 // MODE 1: sum of x - c, its errors
     template <int MODE>
     __device__ __forceinline__ void add(float x, float c, float& top) {
         if (MODE == 0) {
-            two_sum(s, r, x);
+            float d = 0.0f;
+            two_sum(s, d, x);
+            two_sum(e, l, d);
             return;
         }
         float t = x, te = 0.0f;
@@ -124,23 +126,26 @@ struct fp_sum {
         // (t + te)^2 = q + qe + p + pe + te^2, the first four exact
         const float q = __fmul_rn(t, t), qe = __fmaf_rn(t, t, -q);
         const float t2 = __fadd_rn(t, t), p = __fmul_rn(t2, te), pe = __fmaf_rn(t2, te, -p);
-        two_sum(s, r, q);
+        // (the errors of s go to e as well: a plain fp32 sum of them would be 2^-49 of s off,
+        // all one way for a skewed column)
+        float d = 0.0f;
+        two_sum(s, d, q);
+        two_sum(e, l, d);
         two_sum(e, l, qe);
         two_sum(e, l, p);
         l = __fadd_rn(l, __fmaf_rn(te, te, pe));
     }
     template <int MODE>
     __device__ __forceinline__ bool good(float top) const {
-        const float f = MODE == 0 ? s + r : (s + r) + (s1 + e1);
+        const float f = MODE == 0 ? s + e : (s + e) + (s1 + e1);
         return isfinite(f) && (MODE == 0 || top == 0.0f || (top >= 1e-12f && top <= 1e15f));
     }
     template <int MODE>
     __device__ __forceinline__ void flush(double* acc) {
         acc[0] += (double)s;
-        acc[0] += (double)r;
+        acc[0] += (double)e;
+        acc[0] += (double)l;
         if (MODE == 1) {
-            acc[0] += (double)e;
-            acc[0] += (double)l;
             acc[MODE] += (double)s1;
             acc[MODE] += (double)e1;
         }

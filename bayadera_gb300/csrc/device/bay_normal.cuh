@@ -1,5 +1,5 @@
 // bay_normal.cuh -- the Box-Muller pair of the normal walker init, in pairs of floats with the
-// FP64 evaluation as its judge.
+// FP64 evaluation where they leave the rounding open.
 //
 // The init is defined by an FP64 formula rounded to fp32: x = mean + sd r cos(t) and
 // mean + sd r sin(t), r = sqrt(-2 log u1), t = 6.283185307179586 u0.  FP64 issue is 1/64 of

@@ -114,6 +114,22 @@ def test_acor_matches_oracle_at_the_split_edges(oracle, n, wgs, rho):
     assert np.allclose(got.mean, mean, rtol=0, atol=1e-13 * np.abs(x).max())
 
 
+# Skewed columns, whose fp32 rounding errors do not cancel: three levels of FP64 sums, a
+# division and a subtraction, each a rounding of 2^-53 at most, beside words good to 2^-60.
+@pytest.mark.parametrize("n", [1000, 8192, 262147, 2000003])
+def test_moments_of_skewed_columns_to_fp64_rounding(factory, n):
+    rng = np.random.default_rng(n)
+    z = rng.standard_normal((n, 3))
+    x = (np.stack([z[:, 0] ** 2, np.exp(2.0 * z[:, 1]), np.sign(z[:, 2]) * z[:, 2] ** 2 - 5.0], 1)
+         * [1.0, 1.0, 1.5]).astype(np.float32)
+    q = x.astype(np.longdouble)
+    mean = q.mean(0)
+    var = ((q - mean) ** 2).mean(0)
+    got_mean, got_var = factory.data_moments(x)
+    assert np.all(np.abs(got_mean - mean) <= 6 * 2.0 ** -53 * np.abs(mean))
+    assert np.all(np.abs(got_var - var) <= 6 * 2.0 ** -53 * var)
+
+
 def test_scratch_is_kept_bounded_and_given_back(oracle):
     """The kept call scratch: repeated calls of mixed sizes give the same results, it stays
     below its bound, and a context at its memory limit gets it back for a sampler."""
