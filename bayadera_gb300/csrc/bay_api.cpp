@@ -321,6 +321,7 @@ struct bay_model {
     uint32_t row_len = 0;
     // plain form: the density engines' point kernels
     CUkernel k_points = nullptr, k_evidence = nullptr;
+    CUkernel k_staged[5] = {};   // plain form, params in shared memory: bare, accu, logfn, points, evidence
 };
 
 namespace {
@@ -708,7 +709,7 @@ struct bay_sampler {
                                                 : smem);
         cfg.hStream = (CUstream)st;
         cfg.attrs = at;
-        cfg.numAttrs = pdl ? 1 : 0;
+        cfg.numAttrs = pdl && !(plain && !cfg.sharedMemBytes) ? 1 : 0;   // as bay_stretch_plain waits
         if (accu && split > 1) {
             CUlaunchAttribute& cl = at[cfg.numAttrs++];
             cl.id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
@@ -716,7 +717,9 @@ struct bay_sampler {
             cl.value.clusterDim.y = 1;
             cl.value.clusterDim.z = 1;
         }
-        CUkernel k = tcr ? model->k_tr[accu ? 1 : 0] : (accu ? model->k_accu : model->k_bare);
+        CUkernel k = tcr ? model->k_tr[accu ? 1 : 0]
+                         : plain && cfg.sharedMemBytes ? model->k_staged[accu ? 1 : 0]
+                                                       : (accu ? model->k_accu : model->k_bare);
         cu_check(g_cu.LaunchKernelEx(&cfg, (CUfunction)k, args, nullptr), "cuLaunchKernelEx(stretch)");
     }
 
@@ -736,9 +739,9 @@ struct bay_sampler {
         const uint32_t block = tcr ? 256 : plain ? model->cta / plain_split() : model->cta;
         const uint64_t per = plain ? block : per_cta();
         const unsigned g = (unsigned)((W + per - 1) / per);
-        cu_check(g_cu.LaunchKernel((CUfunction)(tcr ? model->k_tr[2] : model->k_logfn), g, 1, 1,
-                                   block, 1, 1,
-                                   (unsigned)(plain ? plain_smem(params, n_params, g, ctx->sm_count) : smem),
+        const size_t sm = plain ? plain_smem(params, n_params, g, ctx->sm_count) : smem;
+        CUkernel k = tcr ? model->k_tr[2] : plain && sm ? model->k_staged[2] : model->k_logfn;
+        cu_check(g_cu.LaunchKernel((CUfunction)k, g, 1, 1, block, 1, 1, (unsigned)sm,
                                    (CUstream)ctx->stream, args, nullptr),
                  "cuLaunchKernel(logfn)");
     }
@@ -1265,10 +1268,14 @@ int bay_model_compile(bay_ctx* c, const bay_model_desc* d, bay_model** out) {
             }
             if (d->form == BAY_FORM_PLAIN) {
                 CUdevice dev = (CUdevice)c->device;
-                for (CUkernel k : {m->k_bare, m->k_accu, m->k_logfn, m->k_points, m->k_evidence})
+                const char* st[5] = {"bay_stretch_bare_s", "bay_stretch_accu_s", "bay_logfn_all_s",
+                                     "bay_points_logfn_s", "bay_points_evidence_s"};
+                for (int i = 0; i < 5; ++i) {
+                    cu_check(g_cu.LibraryGetKernel(&m->k_staged[i], m->lib, st[i]), "GetKernel(staged)");
                     cu_check(g_cu.KernelSetAttribute(CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES,
-                                                     (int)kPlainSmemMax, k, dev),
+                                                     (int)kPlainSmemMax, m->k_staged[i], dev),
                              "cuKernelSetAttribute(smem)");
+                }
             }
             if (d->form == BAY_FORM_TILED) {
                 CUdevice dev = (CUdevice)c->device;

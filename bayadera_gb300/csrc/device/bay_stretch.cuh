@@ -2284,8 +2284,10 @@ extern "C" __global__ void __launch_bounds__(1024, 1) bay_tcr_run_accu(bay_stret
 // One thread per walker of the moving half, the model's LOGFN evaluated per thread
 // (the reference's structure, with SoA coalesced loads and registers for Y).
 
-// The params staged in shared memory (dynamic, as much as the host gave the launch; none: they
-// stay in global memory).  A density's loop reads them in order, all threads alike, a load
+// The params staged in shared memory (STAGED: kernels of their own, named _s, launched with
+// dynamic shared memory for them; else they stay in global memory).  One kernel for both, with
+// the density twice in it, had ptxas schedule the loads from global memory worse: 8,192 walkers
+// x 65,536 rows of 65 floats 43.8 -> 62.4 ms an accu launch.  A density's loop reads them in order, all threads alike, a load
 // every few arithmetic instructions of one dependent sum: from global memory, L1 hits
 // included, a row of 2-D Gaussian data took 31 clocks however few warps there were, from
 // shared memory 8 (8,192 walkers x 1,000 rows: 18.8 us a launch, now 5.7).
@@ -2294,15 +2296,10 @@ extern "C" __global__ void __launch_bounds__(1024, 1) bay_tcr_run_accu(bay_stret
 struct bay_plain_sync {
     unsigned long long bar;
 };
-__device__ __forceinline__ unsigned int bay_dyn_smem() {
-    unsigned int n;
-    asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(n));
-    return n;
-}
-__device__ __forceinline__ void bay_stage_begin(bay_plain_sync* sy, const float* p, unsigned int n,
-                                                unsigned int staged) {
+template <bool STAGED>
+__device__ __forceinline__ void bay_stage_begin(bay_plain_sync* sy, const float* p, unsigned int n) {
     extern __shared__ __align__(16) float bay_psm[];
-    if (!staged) return;
+    if (!STAGED) return;
     const unsigned int bar = (unsigned int)__cvta_generic_to_shared(&sy->bar), bytes = (n * 4u) & ~15u;
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
@@ -2321,9 +2318,9 @@ __device__ __forceinline__ void bay_stage_begin(bay_plain_sync* sy, const float*
     __syncthreads();
 }
 // Bounded wait (2 s) for the copy; false, with status bit 1 set, when it gave up.
-__device__ __forceinline__ bool bay_stage_wait(bay_plain_sync* sy, unsigned int staged,
-                                               unsigned int* status) {
-    if (!staged) return true;
+template <bool STAGED>
+__device__ __forceinline__ bool bay_stage_wait(bay_plain_sync* sy, unsigned int* status) {
+    if (!STAGED) return true;
     const unsigned int bar = (unsigned int)__cvta_generic_to_shared(&sy->bar);
     unsigned long long t0 = 0;
     for (unsigned int it = 0;; ++it) {
@@ -2345,23 +2342,26 @@ __device__ __forceinline__ bool bay_stage_wait(bay_plain_sync* sy, unsigned int 
         }
     }
 }
-__device__ __forceinline__ float bay_density(unsigned int staged, unsigned int data_len,
-                                             unsigned int params_len, const float* params,
-                                             const float* x) {
+template <bool STAGED>
+__device__ __forceinline__ float bay_density(unsigned int data_len, unsigned int params_len,
+                                             const float* params, const float* x) {
     extern __shared__ __align__(16) float bay_psm[];
-    return staged ? BAY_LOGFN(data_len, params_len, bay_psm, DIM, x)
-                  : BAY_LOGFN(data_len, params_len, params, DIM, x);
+    if (STAGED) return BAY_LOGFN(data_len, params_len, bay_psm, DIM, x);
+    return BAY_LOGFN(data_len, params_len, params, DIM, x);
 }
 
-// Launched with programmatic dependent launch.  A group of BAY_CTA walkers is a CTA, or a
+// Launched with programmatic dependent launch where the params are staged (else a launch is
+// long, and the wait's place before the density costs its loop 1 %).  A group of BAY_CTA
+// walkers is a CTA, or a
 // cluster of smaller ones where the ensemble has fewer groups than the device has SMs.
-template <bool ACCU>
+template <bool ACCU, bool STAGED>
 __device__ __forceinline__ void bay_stretch_plain(const bay_stretch_params& P) {
     __shared__ bay_plain_sync sSync;
-    const unsigned int staged = bay_dyn_smem();
-    bay_stage_begin(&sSync, P.params, (unsigned int)P.data_len + P.params_len, staged);
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    bay_stage_begin<STAGED>(&sSync, P.params, (unsigned int)P.data_len + P.params_len);
+    if (STAGED) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     const unsigned int kind = ACCU ? 1u : 0u;
     const unsigned int k = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = k < P.K;
@@ -2390,8 +2390,8 @@ __device__ __forceinline__ void bay_stretch_plain(const bay_stretch_params& P) {
             Y[i] = __fmaf_rn(z, __fsub_rn(X[(size_t)k * DIM + i], s), s);
         }
         const float lx = P.logfn[(size_t)P.half * P.K + k];
-        const bool ok = bay_stage_wait(&sSync, staged, &P.ctl->status);
-        const float ly = bay_density(staged, (unsigned int)P.data_len, P.params_len, P.params, Y);
+        const bool ok = bay_stage_wait<STAGED>(&sSync, &P.ctl->status);
+        const float ly = bay_density<STAGED>((unsigned int)P.data_len, P.params_len, P.params, Y);
         accepted = ok && bay_accept(u2, z, ly, lx, beta);
         if (accepted) {
 #pragma unroll
@@ -2402,7 +2402,7 @@ __device__ __forceinline__ void bay_stretch_plain(const bay_stretch_params& P) {
             for (int i = 0; i < DIM; ++i) Y[i] = X[(size_t)k * DIM + i];
         }
     } else {
-        bay_stage_wait(&sSync, staged, &P.ctl->status);   // the copy lands before the CTA may end
+        bay_stage_wait<STAGED>(&sSync, &P.ctl->status);   // the copy lands before the CTA may end
     }
     if (ACCU) {
         __shared__ float red[BAY_CTA / 32][BAY_SUM_CHUNK];
@@ -2414,63 +2414,85 @@ __device__ __forceinline__ void bay_stretch_plain(const bay_stretch_params& P) {
 }
 
 extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_bare(bay_stretch_params P) {
-    bay_stretch_plain<false>(P);
+    bay_stretch_plain<false, false>(P);
 }
 extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_accu(bay_stretch_params P) {
-    bay_stretch_plain<true>(P);
+    bay_stretch_plain<true, false>(P);
+}
+extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_bare_s(bay_stretch_params P) {
+    bay_stretch_plain<false, true>(P);
+}
+extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_accu_s(bay_stretch_params P) {
+    bay_stretch_plain<true, true>(P);
 }
 
 // logfn over all W walkers (nvidia-gtx-mcmc-stretch.cu:197-206), SoA input.
-extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_logfn_all(bay_stretch_params P) {
+template <bool STAGED>
+__device__ __forceinline__ void bay_logfn_plain(const bay_stretch_params& P) {
     __shared__ bay_plain_sync sSync;
-    const unsigned int staged = bay_dyn_smem();
-    bay_stage_begin(&sSync, P.params, (unsigned int)P.data_len + P.params_len, staged);
+    bay_stage_begin<STAGED>(&sSync, P.params, (unsigned int)P.data_len + P.params_len);
     const unsigned int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool ok = bay_stage_wait(&sSync, staged, &P.ctl->status);
+    const bool ok = bay_stage_wait<STAGED>(&sSync, &P.ctl->status);
     if (k >= P.W || !ok) return;
     float x[DIM];
 #pragma unroll
     for (int i = 0; i < DIM; ++i) x[i] = P.xs[(size_t)k * DIM + i];
-    P.logfn[k] = bay_density(staged, (unsigned int)P.data_len, P.params_len, P.params, x);
+    P.logfn[k] = bay_density<STAGED>((unsigned int)P.data_len, P.params_len, P.params, x);
+}
+extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_logfn_all(bay_stretch_params P) {
+    bay_logfn_plain<false>(P);
+}
+extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_logfn_all_s(bay_stretch_params P) {
+    bay_logfn_plain<true>(P);
 }
 
 // Density engines (reference cuda/engines/nvidia-gtx-distribution.cu logpdf/pdf and
 // nvidia-gtx-likelihood.cu loglik/lik): the model's density at n points, x dim x n
 // column-major (point i's coordinates contiguous); exp_out selects the density itself.
-extern "C" __global__ void __launch_bounds__(BAY_CTA)
-bay_points_logfn(unsigned long long n, unsigned int data_len, unsigned int params_len,
+template <bool STAGED>
+__device__ __forceinline__ void
+bay_points_density(unsigned long long n, unsigned int data_len, unsigned int params_len,
                  const float* params, const float* x, float* out, unsigned int exp_out) {
     __shared__ bay_plain_sync sSync;
-    const unsigned int staged = bay_dyn_smem();
-    bay_stage_begin(&sSync, params, data_len + params_len, staged);
-    const bool ok = bay_stage_wait(&sSync, staged, nullptr);   // given up: NaN, not a stale value
+    bay_stage_begin<STAGED>(&sSync, params, data_len + params_len);
+    const bool ok = bay_stage_wait<STAGED>(&sSync, nullptr);   // given up: NaN, not a stale value
     for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
          i += (unsigned long long)gridDim.x * blockDim.x) {
         float p[DIM];
 #pragma unroll
         for (int d = 0; d < DIM; ++d) p[d] = x[i * DIM + d];
-        const float v = ok ? bay_density(staged, data_len, params_len, params, p) : __int_as_float(0x7fc00000);
+        const float v = ok ? bay_density<STAGED>(data_len, params_len, params, p) : __int_as_float(0x7fc00000);
         out[i] = exp_out ? expf(v) : v;
     }
+}
+extern "C" __global__ void __launch_bounds__(BAY_CTA)
+bay_points_logfn(unsigned long long n, unsigned int data_len, unsigned int params_len,
+                 const float* params, const float* x, float* out, unsigned int exp_out) {
+    bay_points_density<false>(n, data_len, params_len, params, x, out, exp_out);
+}
+extern "C" __global__ void __launch_bounds__(BAY_CTA)
+bay_points_logfn_s(unsigned long long n, unsigned int data_len, unsigned int params_len,
+                   const float* params, const float* x, float* out, unsigned int exp_out) {
+    bay_points_density<true>(n, data_len, params_len, params, x, out, exp_out);
 }
 
 // Evidence (nvidia-gtx-likelihood.cu evidence_reduce): per-CTA FP64 sums of exp(density)
 // over the points, each thread's points in order, then a fixed-order tree -> part[cta].
-extern "C" __global__ void __launch_bounds__(BAY_CTA)
-bay_points_evidence(unsigned long long n, unsigned int data_len, unsigned int params_len,
-                    const float* params, const float* x, double* part) {
+template <bool STAGED>
+__device__ __forceinline__ void
+bay_points_sum(unsigned long long n, unsigned int data_len, unsigned int params_len,
+               const float* params, const float* x, double* part) {
     __shared__ double red[BAY_CTA];
     double s = 0.0;
     __shared__ bay_plain_sync sSync;
-    const unsigned int staged = bay_dyn_smem();
-    bay_stage_begin(&sSync, params, data_len + params_len, staged);
-    const bool ok = bay_stage_wait(&sSync, staged, nullptr);   // given up: NaN, not a stale value
+    bay_stage_begin<STAGED>(&sSync, params, data_len + params_len);
+    const bool ok = bay_stage_wait<STAGED>(&sSync, nullptr);   // given up: NaN, not a stale value
     for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
          i += (unsigned long long)gridDim.x * blockDim.x) {
         float p[DIM];
 #pragma unroll
         for (int d = 0; d < DIM; ++d) p[d] = x[i * DIM + d];
-        s += (double)expf(bay_density(staged, data_len, params_len, params, p));
+        s += (double)expf(bay_density<STAGED>(data_len, params_len, params, p));
     }
     red[threadIdx.x] = s;
     __syncthreads();
@@ -2481,6 +2503,16 @@ bay_points_evidence(unsigned long long n, unsigned int data_len, unsigned int pa
         }
     }
     if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+}
+extern "C" __global__ void __launch_bounds__(BAY_CTA)
+bay_points_evidence(unsigned long long n, unsigned int data_len, unsigned int params_len,
+                    const float* params, const float* x, double* part) {
+    bay_points_sum<false>(n, data_len, params_len, params, x, part);
+}
+extern "C" __global__ void __launch_bounds__(BAY_CTA)
+bay_points_evidence_s(unsigned long long n, unsigned int data_len, unsigned int params_len,
+                      const float* params, const float* x, double* part) {
+    bay_points_sum<true>(n, data_len, params_len, params, x, part);
 }
 
 #else
