@@ -76,8 +76,9 @@ inline REAL logistic_walker(const uint64_t rows, const REAL* hyper, const uint32
     return -pr / (2.0f * hyper[0] * hyper[0]);
 }
 }
-// Streamed tensor-core form: two MUFU operations a row bounded the epilogue (16 a clock an SM:
-// 3.4 of the 4.0 ms of 8,192 walkers x 1,048,653 rows of 64 features), this is one.
+// Streamed tensor-core form: the epilogue's instruction issue bounds it; an exponential, a
+// logarithm and the scalar sums a row took 8,192 walkers x 1,048,653 rows of 64 features 4,160
+// us, these 2,680 to 2,770 (the split products alone 1,730 at the measured rate).
 #define BAY_GEMM_TERMS16 logistic_terms16
 #define BAY_GEMM_CARRY_LEN 3
 #define BAY_GEMM_CARRY_INIT logistic_carry_init
