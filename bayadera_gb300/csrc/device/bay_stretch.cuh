@@ -2483,11 +2483,11 @@ __device__ __forceinline__ void
 bay_points_sum(unsigned long long n, unsigned int data_len, unsigned int params_len,
                const float* params, const float* x, double* part) {
     __shared__ double red[BAY_CTA];
-    double s = 0.0;
     __shared__ bay_plain_sync sSync;
     bay_stage_begin<STAGED>(&sSync, params, data_len + params_len);
     const bool ok = bay_stage_wait<STAGED>(&sSync, nullptr);   // given up: NaN, not a stale value
-    for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
+    double s = ok ? 0.0 : (double)__int_as_float(0x7fc00000);
+    for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; ok && i < n;
          i += (unsigned long long)gridDim.x * blockDim.x) {
         float p[DIM];
 #pragma unroll
