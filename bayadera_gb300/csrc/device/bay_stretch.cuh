@@ -2391,8 +2391,11 @@ __device__ __forceinline__ void bay_stretch_plain(const bay_stretch_params& P) {
         }
         const float lx = P.logfn[(size_t)P.half * P.K + k];
         const bool ok = bay_stage_wait<STAGED>(&sSync, &P.ctl->status);
-        const float ly = bay_density<STAGED>((unsigned int)P.data_len, P.params_len, P.params, Y);
-        accepted = ok && bay_accept(u2, z, ly, lx, beta);
+        float ly = 0.0f;
+        if (ok) {   // else the params may be anything, lengths and offsets that it goes by too
+            ly = bay_density<STAGED>((unsigned int)P.data_len, P.params_len, P.params, Y);
+            accepted = bay_accept(u2, z, ly, lx, beta);
+        }
         if (accepted) {
 #pragma unroll
             for (int i = 0; i < DIM; ++i) X[(size_t)k * DIM + i] = Y[i];

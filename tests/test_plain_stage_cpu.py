@@ -63,7 +63,8 @@ def function(text, name):
     at = text.index(name + "(")
     start = text.rindex("template <", 0, at)
     end = text.index("\n}\n", at) + 3
-    return re.sub(r"asm(?: volatile)?\(.*?\);", ";", text[start:end], flags=re.S)
+    body = re.sub(r"asm(?: volatile)?\(.*?\);", ";", text[start:end], flags=re.S)
+    return body.replace("unsigned int ncta, rank;", "unsigned int ncta = 1u, rank = 0u;")
 
 
 def host_library(tmp_path, names, tail, stubs=""):
@@ -96,3 +97,66 @@ def test_points_are_not_evaluated_and_give_nan_where_the_params_did_not_land(tmp
         else:
             assert e != e and all(v != v for v in out[:n])
         assert list(out[n:]) == [7.0] * (5 - n)
+
+
+MOVE_STUBS = r"""
+#include <cstddef>
+#define BAY_SUM_CHUNK 64
+struct bay_u4 { unsigned int x, y, z, w; };
+struct ctl_ { unsigned int step[2], seed[2]; float a, beta; unsigned int status; };
+struct bay_stretch_params {
+    float* xs; float* logfn; const float* params; ctl_* ctl;
+    unsigned int K, half, step_off, params_len;
+    unsigned long long data_len;
+};
+static bay_u4 bay_philox4x32_10(bay_u4 c, unsigned int, unsigned int) { return c; }
+static float bay_u01(unsigned int) { return 0.5f; }
+static float bay_stretch_z(float, float) { return 0.5f; }
+static unsigned int bay_partner(float, unsigned int) { return 0u; }
+static float bay_partner_coord(const float* S, unsigned int, unsigned int j, int i) { return S[j * DIM + i]; }
+static float bay_beta(const bay_stretch_params&) { return 1.0f; }
+static bool bay_accept(float, float, float, float, float) { return true; }
+static float __fsub_rn(float a, float b) { return a - b; }
+static float __fmaf_rn(float a, float b, float c) { return a * b + c; }
+#undef BAY_CTA
+#define BAY_CTA 32
+static float kept[DIM];
+static bool counted;
+static void bay_accu_epilogue(const bay_stretch_params&, bool accepted, bool, const float* mine,
+                              float (*)[BAY_SUM_CHUNK], unsigned int, unsigned int, unsigned int, unsigned int) {
+    counted = accepted;
+    for (int i = 0; i < DIM; ++i) kept[i] = mine[i];
+}
+"""
+
+MOVE = r"""
+extern "C" void set_lands(int v) { lands = v != 0; evaluated = 0; }
+extern "C" int count() { return evaluated; }
+extern "C" unsigned int move(int accu, float* xs, float* logfn, const float* params, float* mine) {
+    ctl_ ctl = {};
+    ctl.a = 2.0f;
+    bay_stretch_params P = {xs, logfn, params, &ctl, 1u, 0u, 0u, 1u, 0ull};
+    counted = false;
+    if (accu) bay_stretch_plain<true, true>(P);
+    else bay_stretch_plain<false, true>(P);
+    for (int i = 0; i < DIM; ++i) mine[i] = kept[i];
+    return ctl.status | (counted ? 2u : 0u);
+}
+"""
+
+
+@pytest.mark.parametrize("accu", [0, 1])
+def test_moves_are_rejected_unevaluated_where_the_params_did_not_land(tmp_path, accu):
+    lib = host_library(tmp_path, ["bay_stretch_plain"], MOVE,
+                       MOVE_STUBS)
+    params = (C.c_float * 1)(0.5)
+    for lands in (1, 0):
+        xs, logfn, mine = (C.c_float * 4)(3.0, 4.0, 1.0, 2.0), (C.c_float * 2)(-9.0, -9.0), (C.c_float * 2)()
+        lib.set_lands(lands)
+        got = lib.move(accu, xs, logfn, params, mine)
+        assert lib.count() == lands
+        moved = [2.0, 3.0] if lands else [3.0, 4.0]
+        assert list(xs) == moved + [1.0, 2.0] and logfn[0] == (-6.5 if lands else -9.0)
+        if accu:
+            assert list(mine) == moved
+        assert got == ((2 if accu else 0) if lands else 1)
