@@ -294,6 +294,18 @@ __device__ void bay_accu_epilogue(const bay_stretch_params& P, bool accepted, bo
 #endif
 #define BAY_AUXS (BAY_GEMM_AUX > 0 ? BAY_GEMM_AUX : 1)
 
+// A row term f may come with a form for 16 rows (f_16, f_16_init and f_16_end, announced by the
+// macro f_16_carry, the number of values a thread carries over its rows).  It goes with the name
+// of the term that the model uses: a source may define f and use another term.
+#define BAY_CAT2(a, b) a##b
+#define BAY_CAT(a, b) BAY_CAT2(a, b)
+#define BAY_TERM16_CARRY BAY_CAT(BAY_GEMM_TERM, _16_carry)
+#if BAY_TERM16_CARRY
+#define BAY_TERM16 1
+#else
+#define BAY_TERM16 0
+#endif
+
 // barriers of the eight warps that move a tile (accu launches have two more)
 __device__ __forceinline__ void bay_g_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 __device__ __forceinline__ bool bay_g_or(bool p) {
@@ -923,9 +935,9 @@ extern "C" __global__ void __launch_bounds__(256) bay_gemm_accept_logfn(bay_stre
 // allocation and the MMA issue (one thread); warps 2 .. 17 -- epilogue, a thread per
 // walker and share of a tile's rows: tcgen05.ld of its TMEM lane, the model's row terms,
 // a compensated sum over the super-block's rows.  A model may give the terms of 16 rows at
-// once (BAY_GEMM_TERMS16: their sum, and BAY_GEMM_CARRY_LEN values that a thread carries over
-// its rows, whose contribution BAY_GEMM_CARRY_END adds at the end as hi + lo); rows past the
-// last whole batch of 16 take the term by itself.  Two accumulator buffers in TMEM let the
+// once (BAY_TERM16: their sum, and values that a thread carries over its rows, whose
+// contribution is added at the end as hi + lo); rows past the last whole batch of 16 take the
+// term by itself.  Two accumulator buffers in TMEM let the
 // MMAs of tile t + 1 run under the epilogue of tile t.  Every wait is bounded in time; a wait
 // that gives up sets the sampler's status word and the CTA's abort flag, and the CTA
 // drains its own copies and MMAs, frees its TMEM and exits.
@@ -953,12 +965,8 @@ extern "C" __global__ void __launch_bounds__(256) bay_gemm_accept_logfn(bay_stre
 // Order of a 64-feature chunk's products in the accumulator.  The tensor core cuts sums off
 // (toward zero), so that every product added to the large sum takes some 2^-25 of it: with a
 // model that sums its rows' terms exactly enough to show it, the small products come first.
-#ifdef BAY_GEMM_TERMS16
-#define BAY_TC_LO_FIRST 1
-#else
-#define BAY_TC_LO_FIRST 0
-#endif
-#ifdef BAY_GEMM_TERMS16
+#define BAY_TC_LO_FIRST BAY_TERM16
+#if BAY_TERM16
 #define BAY_TC_EPI_UNROLL 2     // its arithmetic bounds the launch: logistic 2.79 -> 2.52 ms
 #else
 #define BAY_TC_EPI_UNROLL 1     // (tensor-bound: robust_t 0.96 ms a launch, 0.975 unrolled)
@@ -1286,9 +1294,9 @@ __device__ __forceinline__ void bay_gemm_rows_tc_impl(const bay_stretch_params& 
             apre[m] = (j < AUXS && ntile > 0u) ? __ldg(auxg + j) : 0.0f;
         }
         float sum = 0.0f, cmp = 0.0f;
-#ifdef BAY_GEMM_TERMS16
-        float carry[BAY_GEMM_CARRY_LEN];
-        BAY_GEMM_CARRY_INIT(carry);
+#if BAY_TERM16
+        float carry[BAY_TERM16_CARRY];
+        BAY_CAT(BAY_GEMM_TERM, _16_init)(carry);
 #endif
         bool ok = true;
         for (unsigned int t = 0; t < ntile; ++t) {
@@ -1335,9 +1343,9 @@ __device__ __forceinline__ void bay_gemm_rows_tc_impl(const bay_stretch_params& 
                     av[4 * i + 2] = a4.z;
                     av[4 * i + 3] = a4.w;
                 }
-#ifdef BAY_GEMM_TERMS16
+#if BAY_TERM16
                 if (jb + 16u <= nrow) {      // the model's sum of the rows' terms, and its carry
-                    v[0] = BAY_GEMM_TERMS16(v, av, (uint64_t)(r0 + jb), xw, prep, carry);
+                    v[0] = BAY_CAT(BAY_GEMM_TERM, _16)(v, av, (uint64_t)(r0 + jb), xw, prep, carry);
                 } else
 #endif
                 {
@@ -1372,12 +1380,12 @@ __device__ __forceinline__ void bay_gemm_rows_tc_impl(const bay_stretch_params& 
         // the groups' partial sums of each walker, combined as compensated pairs in group
         // order; stage 0 is free once the last tile's MMAs (hence its copies) are complete
         float* xchg = (float*)(sm + BAY_TC_WBYTES);        // [4 groups][128 lanes][hi, lo]
-#ifdef BAY_GEMM_TERMS16
+#if BAY_TERM16
         {
             bay_cf c, r;
             r.hi = sum;
             r.lo = -cmp;
-            c.hi = BAY_GEMM_CARRY_END(carry, &c.lo);
+            c.hi = BAY_CAT(BAY_GEMM_TERM, _16_end)(carry, &c.lo);
             r = bay_cadd(r, c);
             sum = r.hi;
             cmp = -r.lo;

@@ -32,7 +32,7 @@ inline REAL logistic_term(const REAL eta, const REAL* aux, const uint64_t row, c
 // 16 rows' terms at once, aux = their y.  The rows' log(1 + exp(-|eta|)) are one logarithm
 // of a running product of 1 + exp(-|eta|), in (1, 2] each: carry holds the mantissas, in
 // [1, 2), of the even and the odd rows' products and their exponents' sum (an integer's
-// bits), and carry_end gives the product's -log as hi + lo.  A multiplication's relative
+// bits), and logistic_term_16_end gives the product's -log as hi + lo.  A multiplication's relative
 // rounding error, 2^-24 at most, is one of the sum; a fast-math logarithm a row has an
 // absolute one of about 2^-23.  The exponential's argument is raised by 4e-8: fast math's
 // exp2 comes out low by that much of an octave on average, which no longer cancels against the
@@ -43,12 +43,12 @@ inline REAL logistic_term(const REAL eta, const REAL* aux, const uint64_t row, c
 inline REAL logistic_exp_neg_abs(const REAL eta) {
     return exp2f(fmaf(fabsf(eta), -1.44269504f, 4.0e-8f));
 }
-inline void logistic_carry_init(REAL* carry) {
+inline void logistic_term_16_init(REAL* carry) {
     carry[0] = carry[1] = 1.0f;
     carry[2] = __int_as_float(0);
 }
-inline REAL logistic_terms16(const REAL* eta, const REAL* aux, const uint64_t row, const REAL* beta,
-                            const REAL* prep, REAL* carry) {
+inline REAL logistic_term_16(const REAL* eta, const REAL* aux, const uint64_t row, const REAL* beta,
+                             const REAL* prep, REAL* carry) {
     bay_f2 p = bay_f2_of(carry[0], carry[1]), s = bay_f2_of(0.0f, 0.0f), m = s;
 #pragma unroll
     for (int i = 0; i < 16; i += 2) {
@@ -63,7 +63,7 @@ inline REAL logistic_terms16(const REAL* eta, const REAL* aux, const uint64_t ro
     carry[1] = __int_as_float((b1 & 0x007fffff) | 0x3f800000);
     return (bay_f2_x(s) - bay_f2_x(m)) + (bay_f2_y(s) - bay_f2_y(m));
 }
-inline REAL logistic_carry_end(const REAL* carry, REAL* lo) {
+inline REAL logistic_term_16_end(const REAL* carry, REAL* lo) {
     const REAL e = (REAL)__float_as_int(carry[2]);
     const REAL h = __fmul_rn(e, 0.693147182f);               // ln 2 = 0.693147182 - 1.90465e-9
     *lo = -(fmaf(e, -1.90465430e-9f, fmaf(e, 0.693147182f, -h)) + logf(carry[0] * carry[1]));
@@ -79,7 +79,4 @@ inline REAL logistic_walker(const uint64_t rows, const REAL* hyper, const uint32
 // Streamed tensor-core form: the epilogue's instruction issue bounds it; an exponential, a
 // logarithm and the scalar sums a row took 8,192 walkers x 1,048,653 rows of 64 features 4,160
 // us, these 2,680 to 2,770 (the split products alone 1,730 at the measured rate).
-#define BAY_GEMM_TERMS16 logistic_terms16
-#define BAY_GEMM_CARRY_LEN 3
-#define BAY_GEMM_CARRY_INIT logistic_carry_init
-#define BAY_GEMM_CARRY_END logistic_carry_end
+#define logistic_term_16_carry 3
