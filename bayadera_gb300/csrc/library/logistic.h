@@ -79,4 +79,6 @@ inline REAL logistic_walker(const uint64_t rows, const REAL* hyper, const uint32
 // Streamed tensor-core form: the epilogue's instruction issue bounds it; an exponential, a
 // logarithm and the scalar sums a row took 8,192 walkers x 1,048,653 rows of 64 features 4,160
 // us, these 2,680 to 2,770 (the split products alone 1,730 at the measured rate).
+#if BAY_GEMM_AUX <= 1          // a row's y and nothing else
 #define logistic_term_16_carry 3
+#endif

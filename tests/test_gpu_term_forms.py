@@ -1,5 +1,6 @@
 """A row term's form for several rows goes with that term alone: a model whose source also
-holds the built-in logistic term, but names a term of its own, gets its own."""
+holds the built-in logistic term, but names a term of its own, gets its own, and
+one with more values a row than that form reads takes the term row by row."""
 import numpy as np
 import pytest
 
@@ -42,5 +43,35 @@ def test_a_source_with_the_logistic_term_and_a_term_of_its_own(n, F, sub):
     eta = X @ b.T
     want = 0.5 * (y[:, None] * eta - np.logaddexp(0.0, eta)).sum(0) - (b * b).sum(1) / 50.0
     bound = (0.5 * (2.0 ** -15 + 4 * F * 2.0 ** -24) * (np.abs(X) @ np.abs(b).T).sum(0)
+             + 2.0 ** -22 * (np.abs(eta) + 2.0).sum(0) + 2.0 ** -22 * np.abs(want) + 1e-6)
+    assert np.all(np.abs(got - want) <= bound)
+
+
+@pytest.mark.parametrize("aux", [0, 1, 2, 3])
+def test_the_logistic_term_with_other_values_beside_the_response(aux):
+    """aux values a row from the response on (none: the term reads a zero)."""
+    from bayadera_gb300 import models as M
+    from bayadera_gb300.engine import GB300BayaderaFactory
+    n, F = 1000, 6
+    rng = np.random.default_rng(aux)
+    X = (rng.standard_normal((n, F)) / np.sqrt(F)).astype(np.float32)
+    y = (rng.random(n) < 0.5).astype(np.float32)
+    rest = rng.standard_normal((n, 3)).astype(np.float32)
+    params = np.concatenate([np.concatenate([X, y[:, None], rest], axis=1).reshape(-1), np.array([5.0], np.float32)])
+    pos = rng.standard_normal((130, F)).astype(np.float32)
+    gemm = dict(M.logistic_model(F).gemm, ld=F + 4, aux_len=aux)
+    model = M.device_distribution_model(M.get_source("logistic"), name="logistic", dimension=F, params_size=1,
+                                        logpdf="logistic_logpdf", gemm=gemm)
+    with GB300BayaderaFactory() as f:
+        sf = f.mcmc_factory(model, form="gemm", tensor=True, streaming=True)
+        s = sf.create_sampler(1, 130, params)
+        s.init_position(pos)
+        got = s.logfn()
+        s.release()
+        sf.release()
+    X, b = X.astype(np.float64), pos.astype(np.float64)
+    eta = X @ b.T
+    want = ((y[:, None] if aux else 0.0) * eta - np.logaddexp(0.0, eta)).sum(0) - (b * b).sum(1) / 50.0
+    bound = ((2.0 ** -15 + 4 * F * 2.0 ** -24) * (np.abs(X) @ np.abs(b).T).sum(0)
              + 2.0 ** -22 * (np.abs(eta) + 2.0).sum(0) + 2.0 ** -22 * np.abs(want) + 1e-6)
     assert np.all(np.abs(got - want) <= bound)
