@@ -514,7 +514,8 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
         // bare launches of 12,290 walkers of 37, 16,384 of 48, 50, 64 and 80, 12,288 of 77 and 8,192
         // of 120 dims: 6.2, 7.0, 6.9, 7.8, 12.0, 12.7 and 15.9 us unrolled by 5; 5.8, 7.0, 7.0, 7.7,
         // 11.2, 10.9 and 15.8 by 10; 5.8, 6.4, 6.4, 7.7, 11.1, 10.9 and 14.7 by 20, at no size from
-        // 2 to 120 dims more than 0.6 % behind, accu launches included; 5.9 and 14.9 (37, 77) in full
+        // 2 to 120 dims more than 0.6 % behind those, accu launches included (by 16: 40 dims 5.6
+        // against 6.1, 48 dims 7.2 against 6.4); 5.9 and 14.9 (37, 77) in full
 #pragma unroll 20
         for (int f = 0; f < BAY_GEMM_F; ++f) {
             const float4 y = *reinterpret_cast<const float4*>(&Ys[f * BAY_WT + w0]);
