@@ -40,6 +40,9 @@ inline REAL logistic_term(const REAL eta, const REAL* aux, const uint64_t row, c
 // 50,007 x 128, 400,000 x 200 and 10,000 x 3 (rows x features): a logarithm a row 5.2, 4.5, 6.9,
 // 10.7 and 2.5e-8; this without the raise 5.5, 4.5, 7.4, 11.2 and 2.8e-8, with it 5.2, 4.4,
 // 6.9, 10.2 and 2.5e-8.
+// y eta - max(eta, 0) is taken row by row, exact for y of 0 or 1: summed apart, rows that are
+// classified right leave the rounding error of their |eta| where any other row is not (normal
+// eta of scale 100, 2 % of the labels flipped: 8.2e-6 RMS a batch of 16 rows, row by row 1.1e-6).
 inline REAL logistic_exp_neg_abs(const REAL eta) {
     return exp2f(fmaf(fabsf(eta), -1.44269504f, 4.0e-8f));
 }
@@ -49,19 +52,20 @@ inline void logistic_term_16_init(REAL* carry) {
 }
 inline REAL logistic_term_16(const REAL* eta, const REAL* aux, const uint64_t row, const REAL* beta,
                              const REAL* prep, REAL* carry) {
-    bay_f2 p = bay_f2_of(carry[0], carry[1]), s = bay_f2_of(0.0f, 0.0f), m = s;
+    bay_f2 p = bay_f2_of(carry[0], carry[1]), s = bay_f2_of(0.0f, 0.0f);
 #pragma unroll
     for (int i = 0; i < 16; i += 2) {
         const bay_f2 t = bay_f2_of(logistic_exp_neg_abs(eta[i]), logistic_exp_neg_abs(eta[i + 1]));
         p = bay_f2_fma(p, t, p);
-        s = bay_f2_fma(bay_f2_of(aux[i], aux[i + 1]), bay_f2_of(eta[i], eta[i + 1]), s);
-        m = bay_f2_add(m, bay_f2_of(fmaxf(eta[i], 0.0f), fmaxf(eta[i + 1], 0.0f)));
+        // y eta - max(eta, 0), exact for y of 0 or 1
+        s = bay_f2_add(s, bay_f2_fma(bay_f2_of(aux[i], aux[i + 1]), bay_f2_of(eta[i], eta[i + 1]),
+                                     bay_f2_of(fminf(-eta[i], 0.0f), fminf(-eta[i + 1], 0.0f))));
     }
     const int b0 = __float_as_int(bay_f2_x(p)), b1 = __float_as_int(bay_f2_y(p));
     carry[2] = __int_as_float(__float_as_int(carry[2]) + (b0 >> 23) + (b1 >> 23) - 254);
     carry[0] = __int_as_float((b0 & 0x007fffff) | 0x3f800000);
     carry[1] = __int_as_float((b1 & 0x007fffff) | 0x3f800000);
-    return (bay_f2_x(s) - bay_f2_x(m)) + (bay_f2_y(s) - bay_f2_y(m));
+    return bay_f2_x(s) + bay_f2_y(s);
 }
 inline REAL logistic_term_16_end(const REAL* carry, REAL* lo) {
     const REAL e = (REAL)__float_as_int(carry[2]);
