@@ -43,3 +43,19 @@ def test_flipped_labels_among_well_separated_rows(n, sub):
     want = -np.abs(X[flipped] @ pos.T).sum(0)
     got = log_densities(X, y.astype(np.float64), pos, sub)
     assert np.all(np.abs(got - want) <= 2.0 ** -20 * np.abs(want))
+
+
+# The fast exponential's mean error is taken out by a constant, which a compiler may make wrong.
+# The walkers' rounding errors, 2^-24 of each sum at most, average out over 1,024 of them (below
+# 2^-29); what the sums are off by on average is to stay below a quarter of a float's rounding.
+@pytest.mark.parametrize("n,spread", [(32768, 1.0), (32768, 0.25), (4096, 4.0)])
+def test_sums_have_no_mean_error(n, spread):
+    rng = np.random.default_rng(n + int(4 * spread))
+    F, W = 8, 1024
+    X = rng.integers(-24, 25, (n, F)) / 16.0
+    pos = spread * rng.integers(-16, 17, (W, F)) / 16.0
+    y = (rng.random(n) < 0.5).astype(np.float64)
+    eta = X @ pos.T
+    want = (y[:, None] * eta - np.logaddexp(0.0, eta)).sum(0)
+    got = log_densities(X, y, pos, 1)
+    assert abs(np.mean((got - want) / want)) <= 2.0 ** -26
