@@ -19,6 +19,7 @@
 #include <nvtx3/nvToolsExt.h>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -202,58 +203,43 @@ struct bay_ctx {
 
     // Device memory for the length of one call (arguments staged from the host, work copies):
     // a cudaMalloc and a cudaFree, which waits for the device, cost some tens of us each, so
-    // up to kScratchMax bytes of it are kept with the context, as much as a call has needed
-    // before.  Blocks are cut off in order and the whole is free again when the last is
-    // returned.  Calls hold the context's lock and finish on its stream before they return a
-    // block.  What does not fit, or not under mem_limit, is allocated for the call alone; an
-    // allocation that finds no room takes the idle scratch back.
+    // one block of at most kScratchMax bytes is kept with the context, as large as a call has
+    // needed.  A call says what it needs in all before it takes anything (Scratch) and gets the
+    // kept block for all of it or allocations of its own for all of it: a small part of a call
+    // never holds a block that its other parts then find no room beside.  An allocation that
+    // finds no room takes the kept memory back.
     static constexpr size_t kScratchMax = 64u << 20;
     char* sc_base = nullptr;
-    size_t sc_cap = 0, sc_used = 0, sc_want = 0, sc_total = 0;
-    uint32_t sc_live = 0;
-    void* scratch(size_t bytes) {
-        bytes = (bytes + 255) & ~(size_t)255;
-        if (bytes == 0) bytes = 256;
-        if (sc_live == 0) sc_total = 0;
-        sc_total += bytes;
-        if (sc_live == 0 && sc_want > sc_cap) {
-            give_back();
-            if (!over_limit(sc_want)) {
-                void* p = nullptr;
-                if (cudaMalloc(&p, sc_want) == cudaSuccess) {
-                    sc_base = (char*)p;
-                    sc_cap = sc_want;
-                    allocated += sc_cap;
-                } else {
-                    cudaGetLastError();
-                }
+    size_t sc_cap = 0;
+    bool sc_busy = false;
+    // the kept block, grown to `total` bytes where need be; NULL: allocate
+    char* scratch_block(size_t total) {
+        if (sc_busy || total > kScratchMax) return nullptr;
+        if (total > sc_cap) {
+            drop_scratch();
+            if (over_limit(total)) return nullptr;
+            void* p = nullptr;
+            if (cudaMalloc(&p, total) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
             }
+            sc_base = (char*)p;
+            sc_cap = total;
+            allocated += sc_cap;
         }
-        if (sc_total <= kScratchMax) sc_want = std::max(sc_want, sc_total);
-        if (sc_used + bytes <= sc_cap) {
-            void* p = sc_base + sc_used;
-            sc_used += bytes;
-            ++sc_live;
-            return p;
-        }
-        return alloc(bytes);
+        sc_busy = true;
+        return sc_base;
     }
-    void unscratch(void* p) {
-        if (!p) return;
-        if ((char*)p >= sc_base && (char*)p < sc_base + sc_cap) {
-            if (--sc_live == 0) sc_used = 0;
-        } else {
-            release(p);
-        }
+    void drop_scratch() {
+        if (sc_busy || !sc_base) return;
+        cudaFree(sc_base);
+        allocated -= sc_cap;
+        sc_base = nullptr;
+        sc_cap = 0;
     }
     // the kept memory that no call is using, back to the device
     void give_back() {
-        if (sc_live == 0 && sc_base) {
-            cudaFree(sc_base);
-            allocated -= sc_cap;
-            sc_base = nullptr;
-            sc_cap = sc_used = 0;
-        }
+        drop_scratch();
         release(est_ws);
         est_ws = nullptr;
         est_ws_bytes = 0;
@@ -288,6 +274,46 @@ struct bay_ctx {
         return est_ws;
     }
 };
+
+namespace {
+// One call's device memory, of the context's kept block or allocated; under the context's
+// lock.  It goes back when the call's work on the stream is done.
+struct Scratch {
+    bay_ctx* ctx;
+    char* base = nullptr;
+    size_t used = 0;
+    std::vector<void*> own;
+    bool done = false;
+    static size_t padded(size_t bytes) { return bytes ? (bytes + 255) & ~(size_t)255 : 256; }
+    // sizes: of every block the call will take (0: not taken)
+    Scratch(bay_ctx* c, std::initializer_list<size_t> sizes) : ctx(c) {
+        size_t total = 0;
+        for (size_t b : sizes) total += b ? padded(b) : 0;
+        own.reserve(sizes.size());
+        if (total) base = c->scratch_block(total);
+    }
+    void* take(size_t bytes) {
+        if (base) {
+            void* p = base + used;
+            used += padded(bytes);
+            return p;
+        }
+        own.push_back(nullptr);
+        return own.back() = ctx->alloc(bytes);
+    }
+    void finish() {
+        cuda_check(cudaStreamSynchronize(ctx->stream), "sync");
+        done = true;
+    }
+    ~Scratch() {
+        if (!done) cudaStreamSynchronize(ctx->stream);
+        if (base) ctx->sc_busy = false;
+        for (void* p : own) ctx->release(p);
+    }
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+};
+}  // namespace
 
 // ============================================================================ model
 struct bay_model {
@@ -1700,21 +1726,15 @@ int bay_init_position_limits(bay_sampler* s, uint32_t seed, const float* limits)
         if (!s || !limits) fail(BAY_ERR_ARG, "NULL argument");
         std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
         s->ctx->use();
-        float* dl = (float*)s->ctx->scratch(sizeof(float) * 2 * s->D);
-        try {
-            cuda_check(cudaMemcpyAsync(dl, limits, sizeof(float) * 2 * s->D, cudaMemcpyDefault,
-                                       s->ctx->stream),
-                       "cudaMemcpy(limits)");
-            cuda_check(bay::launch_init_uniform(s->xs, s->D, s->W, seed, dl, s->ctx->stream),
-                       "init_walkers");
-            s->launch_logfn_all();
-            cuda_check(cudaStreamSynchronize(s->ctx->stream), "sync");
-        } catch (...) {
-            cudaStreamSynchronize(s->ctx->stream);
-            s->ctx->unscratch(dl);
-            throw;
-        }
-        s->ctx->unscratch(dl);
+        Scratch sc(s->ctx, {sizeof(float) * 2 * s->D});
+        float* dl = (float*)sc.take(sizeof(float) * 2 * s->D);
+        cuda_check(cudaMemcpyAsync(dl, limits, sizeof(float) * 2 * s->D, cudaMemcpyDefault,
+                                   s->ctx->stream),
+                   "cudaMemcpy(limits)");
+        cuda_check(bay::launch_init_uniform(s->xs, s->D, s->W, seed, dl, s->ctx->stream),
+                   "init_walkers");
+        s->launch_logfn_all();
+        sc.finish();
         s->positioned = true;
         s->iteration_counter = 0;
     });
@@ -1875,10 +1895,10 @@ uint32_t acor_lag(uint64_t n, uint32_t wgs) {
     return (uint32_t)(l < 10 ? 10 : l);
 }
 
-// acor of a device-resident series -- value t of dimension d at t * D + d, or with rows at
-// d * n + t -- results to host or device arrays.
-int acor_device(bay_ctx* c, const float* d_series, uint32_t D, uint64_t n, bool rows, double* tau,
-                double* mean, double* sigma, uint32_t* lag_out) {
+// acor of a series in device or (staged) host memory -- value t of dimension d at t * D + d, or
+// with rows at d * n + t -- results to host or device arrays.
+int acor_series(bay_ctx* c, const float* series, bool staged, uint32_t D, uint64_t n, bool rows,
+                double* tau, double* mean, double* sigma, uint32_t* lag_out) {
     const uint32_t lag = acor_lag(n, c->wgs);
     if (lag_out) *lag_out = lag;
     if ((uint64_t)lag * 5 > n) {
@@ -1887,22 +1907,24 @@ int acor_device(bay_ctx* c, const float* d_series, uint32_t D, uint64_t n, bool 
         return BAY_ERR_ARG;
     }
     if (n > 0xffffffffull) fail(BAY_ERR_ARG, "series too long");
-    double* work = (double*)c->scratch(sizeof(double) * ((size_t)D * n + 3 * D));
-    try {
-        double* res = work + (size_t)D * n;
-        cuda_check(bay::launch_acor(d_series, D, (uint32_t)n, rows ? 1 : D, rows ? n : 1, c->wgs, lag,
-                                    work, res, res + D, res + 2 * D, c->stream),
-                   "acor");
-        if (tau) cuda_check(cudaMemcpyAsync(tau, res, sizeof(double) * D, cudaMemcpyDefault, c->stream), "copy");
-        if (mean) cuda_check(cudaMemcpyAsync(mean, res + D, sizeof(double) * D, cudaMemcpyDefault, c->stream), "copy");
-        if (sigma) cuda_check(cudaMemcpyAsync(sigma, res + 2 * D, sizeof(double) * D, cudaMemcpyDefault, c->stream), "copy");
-        cuda_check(cudaStreamSynchronize(c->stream), "sync");
-    } catch (...) {
-        cudaStreamSynchronize(c->stream);
-        c->unscratch(work);
-        throw;
+    const size_t copy = staged ? sizeof(float) * (size_t)D * n : 0;
+    const size_t wbytes = sizeof(double) * ((size_t)D * n + 3 * D);
+    Scratch sc(c, {copy, wbytes});
+    if (staged) {
+        float* d = (float*)sc.take(copy);
+        cuda_check(cudaMemcpyAsync(d, series, copy, cudaMemcpyHostToDevice, c->stream),
+                   "cudaMemcpy(series)");
+        series = d;
     }
-    c->unscratch(work);
+    double* work = (double*)sc.take(wbytes);
+    double* res = work + (size_t)D * n;
+    cuda_check(bay::launch_acor(series, D, (uint32_t)n, rows ? 1 : D, rows ? n : 1, c->wgs, lag, work,
+                                res, res + D, res + 2 * D, c->stream),
+               "acor");
+    if (tau) cuda_check(cudaMemcpyAsync(tau, res, sizeof(double) * D, cudaMemcpyDefault, c->stream), "copy");
+    if (mean) cuda_check(cudaMemcpyAsync(mean, res + D, sizeof(double) * D, cudaMemcpyDefault, c->stream), "copy");
+    if (sigma) cuda_check(cudaMemcpyAsync(sigma, res + 2 * D, sizeof(double) * D, cudaMemcpyDefault, c->stream), "copy");
+    sc.finish();
     return BAY_OK;
 }
 }  // namespace
@@ -2039,7 +2061,7 @@ int bay_run_sampler(bay_sampler* s, uint64_t n, float a, bay_run_result* res, do
                        "cudaMemcpy(means)");
         uint32_t lag = 0;
         const std::string keep = g_err;
-        res->acor_status = acor_device(s->ctx, s->means, s->D, n, false, tau, mean, sigma, &lag);
+        res->acor_status = acor_series(s->ctx, s->means, false, s->D, n, false, tau, mean, sigma, &lag);
         if (res->acor_status == BAY_OK) g_err = keep;
         res->lag = lag;
         cuda_check(cudaStreamSynchronize(s->ctx->stream), "sync");
@@ -2177,23 +2199,7 @@ static int acor_any(bay_ctx* c, const float* series, uint32_t D, uint64_t n, boo
         if (D == 0) fail(BAY_ERR_ARG, "dim must be >= 1");
         std::lock_guard<std::recursive_mutex> lk(c->mu);
         c->use();
-        if (is_device_ptr(series, c->device)) {
-            rc = acor_device(c, series, D, n, rows, tau, mean, sigma, lag);
-            return;
-        }
-        float* d = (float*)c->scratch(sizeof(float) * (size_t)D * std::max<uint64_t>(n, 1));
-        try {
-            cuda_check(cudaMemcpyAsync(d, series, sizeof(float) * (size_t)D * n,
-                                       cudaMemcpyHostToDevice, c->stream),
-                       "cudaMemcpy(series)");
-            rc = acor_device(c, d, D, n, rows, tau, mean, sigma, lag);
-        } catch (...) {
-            cudaStreamSynchronize(c->stream);
-            c->unscratch(d);
-            throw;
-        }
-        if (rc != BAY_OK) cudaStreamSynchronize(c->stream);   // the copy, nothing waited for it
-        c->unscratch(d);
+        rc = acor_series(c, series, !is_device_ptr(series, c->device), D, n, rows, tau, mean, sigma, lag);
     });
     return g != BAY_OK ? g : rc;
 }
