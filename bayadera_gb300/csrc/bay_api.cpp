@@ -424,7 +424,8 @@ uint32_t tr_free_groups(uint64_t base, uint64_t greg, uint64_t tiles, uint64_t s
 }
 // With one sub-tile and at most 256 features the kernel holds the walker operand in tensor
 // memory (BAY_TC_ATM), which leaves its shared memory to more stages: the free choice is up to
-// 6 there too; which shapes may be asked for stays as if it were in shared memory.
+// 6 there too, and may be asked for (it is the tuner's answer where no other shape is faster);
+// which other shapes may be asked for stays as if it were in shared memory.
 // want_g / want_s (0 = free) ask for a shape; false when no shape fits (or the asked one
 // does not).
 bool tc_plan(uint32_t features, uint32_t aux_len, uint32_t* G, uint32_t* S, size_t* smem,
@@ -436,9 +437,10 @@ bool tc_plan(uint32_t features, uint32_t aux_len, uint32_t* G, uint32_t* S, size
         const size_t fixed = (size_t)g * kc * 32768 + rest;
         if (fixed + 2 * 32768 > kTcSmemMax) continue;
         size_t st = std::min<size_t>(6, (kTcSmemMax - fixed) / 32768);
-        if (want_s && (want_s < 2 || want_s > st)) return false;
         const size_t held = g == 1 && kc <= 4 ? rest : fixed;
-        st = want_s ? want_s : std::min<size_t>(6, (kTcSmemMax - held) / 32768);
+        const size_t free_st = std::min<size_t>(6, (kTcSmemMax - held) / 32768);
+        if (want_s && want_s != free_st && (want_s < 2 || want_s > st)) return false;
+        st = want_s ? want_s : free_st;
         *G = g;
         *S = (uint32_t)st;
         *smem = held + st * 32768;
