@@ -348,6 +348,7 @@ struct bay_model {
     // plain form: the density engines' point kernels
     CUkernel k_points = nullptr, k_evidence = nullptr;
     CUkernel k_staged[5] = {};   // plain form, params in shared memory: bare, accu, logfn, points, evidence
+    bool staging = false;        // ... may be launched
 };
 
 namespace {
@@ -366,9 +367,11 @@ size_t gemm_smem_bytes(const bay_model* m, uint64_t rows) {
 
 // Plain form: dynamic shared memory of a launch of `ctas` CTAs, the whole params where they are
 // staged (bay_stage_begin) or 0.  Up to 48 KB they are (4 CTAs of 256 threads an SM still fit);
-// up to 200 KB where every CTA has an SM to itself anyway.  16-byte-aligned params only.
+// up to 200 KB where every CTA has an SM to itself anyway.  16-byte-aligned params only, and only
+// where the model's kernels may have the shared memory (their own static arrays take of it).
 constexpr size_t kPlainSmem = 48 * 1024 - 4096, kPlainSmemMax = 200 * 1024;
-size_t plain_smem(const float* params, uint64_t n_params, uint64_t ctas, int sm_count) {
+size_t plain_smem(const bay_model* m, const float* params, uint64_t n_params, uint64_t ctas, int sm_count) {
+    if (!m->staging) return 0;
     const uint64_t bytes = (n_params * sizeof(float) + 15) & ~15ull;
     if (n_params == 0 || (uintptr_t)params % 16) return 0;
     return bytes <= (ctas <= (uint64_t)sm_count ? kPlainSmemMax : kPlainSmem) ? (size_t)bytes : 0;
@@ -623,8 +626,8 @@ struct bay_sampler {
     uint32_t plain_split() const {
         if (model->form != BAY_FORM_PLAIN || model->cta != 256 || grid() >= (unsigned)ctx->sm_count) return 1u;
         // (not where the params are staged by whole CTAs alone)
-        return plain_smem(params, n_params, 4ull * grid(), ctx->sm_count) ||
-                       !plain_smem(params, n_params, grid(), ctx->sm_count)
+        return plain_smem(model, params, n_params, 4ull * grid(), ctx->sm_count) ||
+                       !plain_smem(model, params, n_params, grid(), ctx->sm_count)
                    ? 4u : 1u;
     }
 
@@ -733,7 +736,7 @@ struct bay_sampler {
         cfg.blockDimY = 1;
         cfg.blockDimZ = 1;
         cfg.sharedMemBytes = (unsigned)(tcr || tiled ? smem_move
-                                        : plain ? plain_smem(params, n_params, cfg.gridDimX, ctx->sm_count)
+                                        : plain ? plain_smem(model, params, n_params, cfg.gridDimX, ctx->sm_count)
                                                 : smem);
         cfg.hStream = (CUstream)st;
         cfg.attrs = at;
@@ -767,7 +770,7 @@ struct bay_sampler {
         const uint32_t block = tcr ? 256 : plain ? model->cta / plain_split() : model->cta;
         const uint64_t per = plain ? block : per_cta();
         const unsigned g = (unsigned)((W + per - 1) / per);
-        const size_t sm = plain ? plain_smem(params, n_params, g, ctx->sm_count) : smem;
+        const size_t sm = plain ? plain_smem(model, params, n_params, g, ctx->sm_count) : smem;
         CUkernel k = tcr ? model->k_tr[2] : plain && sm ? model->k_staged[2] : model->k_logfn;
         cu_check(g_cu.LaunchKernel((CUfunction)k, g, 1, 1, block, 1, 1, (unsigned)sm,
                                    (CUstream)ctx->stream, args, nullptr),
@@ -1300,9 +1303,11 @@ int bay_model_compile(bay_ctx* c, const bay_model_desc* d, bay_model** out) {
                                      "bay_points_logfn_s", "bay_points_evidence_s"};
                 for (int i = 0; i < 5; ++i) {
                     cu_check(g_cu.LibraryGetKernel(&m->k_staged[i], m->lib, st[i]), "GetKernel(staged)");
-                    cu_check(g_cu.KernelSetAttribute(CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES,
-                                                     (int)kPlainSmemMax, m->k_staged[i], dev),
-                             "cuKernelSetAttribute(smem)");
+                    // refused where the source's own static shared memory leaves less
+                    m->staging = (i == 0 || m->staging) &&
+                                 g_cu.KernelSetAttribute(CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES,
+                                                         (int)kPlainSmemMax, m->k_staged[i], dev) ==
+                                     CUDA_SUCCESS;
                 }
             }
             if (d->form == BAY_FORM_TILED) {
