@@ -23,6 +23,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -1079,7 +1080,82 @@ struct Codegen {
     size_t tc_smem = 0;
     uint32_t tr_g = 1;
     bool tr_free = false;
+    bool any_space = false;
 };
+
+// Whether a model's source may be given pointers into shared memory for its params and walker
+// rows.  Plain C reads through them as it does from global memory; a load that names its address
+// space (__ldg, inline PTX and the like) or a pointer made into one does not, and shared memory
+// that the source declares itself is counted against the kernels'.  So every identifier of the
+// compiler's own (two leading underscores) has to be a qualifier or an arithmetic function of the
+// lists below, and there is no inline assembly, token pasting or header other than <stdint.h>.
+// Other sources get global pointers everywhere they did before rows and params were staged.
+bool any_space_source(const char* source) {
+    static const std::set<std::string> known = {
+        "__device__", "__host__", "__constant__", "__forceinline__", "__inline__", "__inline", "__noinline__",
+        "__restrict__", "__restrict", "__align__", "__func__", "__FILE__", "__LINE__", "__VA_ARGS__",
+        "__cplusplus", "__CUDA_ARCH__", "__CUDACC__", "__CUDACC_RTC__", "__NVCC__",
+        "__expf", "__exp10f", "__logf", "__log2f", "__log10f", "__powf", "__sinf", "__cosf", "__tanf",
+        "__sincosf", "__fdividef", "__saturatef", "__int_as_float", "__float_as_int", "__uint_as_float",
+        "__float_as_uint", "__double_as_longlong", "__longlong_as_double", "__hiloint2double", "__clz",
+        "__clzll", "__popc", "__popcll", "__ffs", "__ffsll", "__brev", "__brevll", "__mul24", "__umul24",
+        "__mulhi", "__umulhi", "__mul64hi", "__umul64hi", "__byte_perm", "__sad", "__usad"};
+    static const char* const families[] = {
+        "__fadd_", "__fsub_", "__fmul_", "__fmaf_", "__fdiv_", "__frcp_", "__fsqrt_", "__frsqrt_", "__dadd_",
+        "__dsub_", "__dmul_", "__fma_", "__ddiv_", "__drcp_", "__dsqrt_", "__float2", "__double2", "__int2",
+        "__uint2", "__ll2", "__ull2", "__funnelshift_"};
+    std::string s;   // without the spliced line ends
+    for (const char* p = source; *p; ++p) {
+        if (*p == '\\') {
+            const char* q = p + 1;
+            while (*q == ' ' || *q == '\t' || *q == '\r') ++q;
+            if (*q == '\n') {
+                p = q;
+                continue;
+            }
+        }
+        s += *p;
+    }
+    const auto word_char = [](char c) { return std::isalnum((unsigned char)c) || c == '_'; };
+    for (size_t i = 0; i < s.size();) {
+        const char c = s[i];
+        if (s.compare(i, 2, "//") == 0) {
+            i = std::min(s.find('\n', i), s.size());
+        } else if (s.compare(i, 2, "/*") == 0) {
+            i = s.find("*/", i + 2);
+            if (i == std::string::npos) return false;
+            i += 2;
+        } else if (c == '\\' || s.compare(i, 2, "##") == 0 || s.compare(i, 2, "%:") == 0) {
+            return false;
+        } else if (c == '"' || c == '\'') {
+            for (++i; i < s.size() && s[i] != c; ++i)
+                if (s[i] == '\\') ++i;
+            ++i;
+        } else if (std::isdigit((unsigned char)c)) {   // digits may be parted by '
+            while (i < s.size() && (word_char(s[i]) || s[i] == '.' || s[i] == '\'')) ++i;
+        } else if (word_char(c)) {
+            size_t j = i;
+            while (j < s.size() && word_char(s[j])) ++j;
+            const std::string w = s.substr(i, j - i);
+            i = j;
+            if (w == "asm" || (w.back() == 'R' && i < s.size() && s[i] == '"')) return false;
+            if (w == "include") {
+                const size_t e = std::min(s.find('\n', i), s.size());
+                std::string h;
+                for (; i < e; ++i)
+                    if (!std::isspace((unsigned char)s[i])) h += s[i];
+                if (h.compare(0, 10, "<stdint.h>") != 0 && h.compare(0, 9, "<cstdint>") != 0) return false;
+            }
+            if (w.compare(0, 2, "__") == 0 && !known.count(w) &&
+                std::none_of(std::begin(families), std::end(families),
+                             [&](const char* f) { return w.compare(0, std::strlen(f), f) == 0; }))
+                return false;
+        } else {
+            ++i;
+        }
+    }
+    return true;
+}
 
 // Source and NVRTC options of a model's fused kernels (the reference's stretch-options,
 // nvidia_gtx.clj:630-633, retargeted to sm_103a).
@@ -1106,6 +1182,8 @@ Codegen codegen(const bay_model_desc* d, uint32_t wgs) {
             fail(BAY_ERR_ARG, "BAY_MODEL_PARTNER_ELEMENT applies to the plain and tiled forms");
         opts.push_back("-DBAY_PARTNER_ELEMENT=1");
     }
+    g.any_space = any_space_source(d->source);
+    opts.push_back(std::string("-DBAY_ANY_SPACE=") + (g.any_space ? "1" : "0"));
     uint32_t wpc = 1;
     if (d->form == BAY_FORM_PLAIN) {
         if (!valid_ident(d->logfn)) fail(BAY_ERR_ARG, "logfn must name a C function");
@@ -1297,7 +1375,7 @@ int bay_model_compile(bay_ctx* c, const bay_model_desc* d, bay_model** out) {
                              "GetKernel(evidence)");
                 }
             }
-            if (d->form == BAY_FORM_PLAIN) {
+            if (d->form == BAY_FORM_PLAIN && g.any_space) {
                 CUdevice dev = (CUdevice)c->device;
                 const char* st[5] = {"bay_stretch_bare_s", "bay_stretch_accu_s", "bay_logfn_all_s",
                                      "bay_points_logfn_s", "bay_points_evidence_s"};

@@ -2296,7 +2296,8 @@ extern "C" __global__ void __launch_bounds__(1024, 1) bay_tcr_run_accu(bay_stret
 // (the reference's structure, with SoA coalesced loads and registers for Y).
 
 // The params staged in shared memory (STAGED: kernels of their own, named _s, launched with
-// dynamic shared memory for them; else they stay in global memory).  One kernel for both, with
+// dynamic shared memory for them; else they stay in global memory, always so where the source
+// may read them by global loads alone: BAY_ANY_SPACE 0).  One kernel for both, with
 // the density twice in it, had ptxas schedule the loads from global memory worse: 8,192 walkers
 // x 65,536 rows of 65 floats 43.8 -> 62.4 ms an accu launch.  A density's loop reads them in order, all threads alike, a load
 // every few arithmetic instructions of one dependent sum: from global memory, L1 hits
@@ -2433,12 +2434,14 @@ extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_bare(bay_stret
 extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_accu(bay_stretch_params P) {
     bay_stretch_plain<true, false>(P);
 }
+#if BAY_ANY_SPACE
 extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_bare_s(bay_stretch_params P) {
     bay_stretch_plain<false, true>(P);
 }
 extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_accu_s(bay_stretch_params P) {
     bay_stretch_plain<true, true>(P);
 }
+#endif
 
 // logfn over all W walkers (nvidia-gtx-mcmc-stretch.cu:197-206), SoA input.
 template <bool STAGED>
@@ -2456,9 +2459,11 @@ __device__ __forceinline__ void bay_logfn_plain(const bay_stretch_params& P) {
 extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_logfn_all(bay_stretch_params P) {
     bay_logfn_plain<false>(P);
 }
+#if BAY_ANY_SPACE
 extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_logfn_all_s(bay_stretch_params P) {
     bay_logfn_plain<true>(P);
 }
+#endif
 
 // Density engines (reference cuda/engines/nvidia-gtx-distribution.cu logpdf/pdf and
 // nvidia-gtx-likelihood.cu loglik/lik): the model's density at n points, x dim x n
@@ -2484,11 +2489,13 @@ bay_points_logfn(unsigned long long n, unsigned int data_len, unsigned int param
                  const float* params, const float* x, float* out, unsigned int exp_out) {
     bay_points_density<false>(n, data_len, params_len, params, x, out, exp_out);
 }
+#if BAY_ANY_SPACE
 extern "C" __global__ void __launch_bounds__(BAY_CTA)
 bay_points_logfn_s(unsigned long long n, unsigned int data_len, unsigned int params_len,
                    const float* params, const float* x, float* out, unsigned int exp_out) {
     bay_points_density<true>(n, data_len, params_len, params, x, out, exp_out);
 }
+#endif
 
 // Evidence (nvidia-gtx-likelihood.cu evidence_reduce): per-CTA FP64 sums of exp(density)
 // over the points, each thread's points in order, then a fixed-order tree -> part[cta].
@@ -2523,11 +2530,13 @@ bay_points_evidence(unsigned long long n, unsigned int data_len, unsigned int pa
                     const float* params, const float* x, double* part) {
     bay_points_sum<false>(n, data_len, params_len, params, x, part);
 }
+#if BAY_ANY_SPACE
 extern "C" __global__ void __launch_bounds__(BAY_CTA)
 bay_points_evidence_s(unsigned long long n, unsigned int data_len, unsigned int params_len,
                       const float* params, const float* x, double* part) {
     bay_points_sum<true>(n, data_len, params_len, params, x, part);
 }
+#endif
 
 #else
 // ---------------------------------------------------------------- tiled form

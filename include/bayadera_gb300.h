@@ -80,6 +80,10 @@ int bay_launch_count(uint64_t* out);
  *          uint32_t dim, const REAL* x)
  * with params = data || hyperparameters; REAL is float; the source may include
  * <stdint.h>.  Compiled with -use_fast_math like the reference.
+ * params are generic pointers: where they fit they are staged in shared memory, so long as
+ * the source is plain C and arithmetic intrinsics.  A source that holds inline assembly,
+ * token pasting, a header other than <stdint.h>, shared memory of its own or another
+ * identifier with two leading underscores (__ldg, __cvta_...) gets them in global memory.
  *
  * BAY_FORM_TILED is the data-tiled form for likelihoods that sum over data rows:
  *   void  prep(const REAL* hyper, uint32_t hyper_len, uint32_t dim, const REAL* x,
