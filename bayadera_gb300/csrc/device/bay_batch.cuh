@@ -238,7 +238,8 @@ __device__ __forceinline__ void bay_batch_propose_impl(const bay_batch_params& P
     }
     __syncthreads();
     if (tid < nt) {
-        const float* y = bay_bsm + tid * dpad;
+        // (BAY_ANY_SPACE 0: the source may take global rows alone)
+        const float* y = BAY_ANY_SPACE ? bay_bsm + tid * dpad : Y + (size_t)tid * dim;
         const float* hyper = P.params + M.params + M.rows * BAY_ROW_LEN;
         float pr[BAY_PREP_LEN];
 #pragma unroll

@@ -644,9 +644,12 @@ __device__ __forceinline__ void bay_split_bf16x2(float a, float b, unsigned int&
 // walker evaluates the model's prep and walker terms in the model's own order.  2,048 walkers
 // of 257 coordinates: 5.1 us, 268 us with one thread per walker for the rows too (a sector
 // per float read or written); 8 walkers per CTA are 256 CTAs there.  BAY_PW is the host's (kernel grid), 8 while the rows fit in 48 KB.
+// A source that may take global rows alone (BAY_ANY_SPACE 0) gets the global copies instead.
 template <int MODE>  // 0 bare, 1 accu, 2 log density of the current positions
 __device__ __forceinline__ void bay_gemm_propose_impl(const bay_stretch_params& P) {
+#if BAY_ANY_SPACE
     __shared__ float sY[BAY_PW][DIM | 1];
+#endif
     const unsigned int kind = MODE == 1 ? 1u : 0u;
     const unsigned int nk = MODE == 2 ? P.W : P.K;
     const unsigned int k0 = blockIdx.x * BAY_PW;
@@ -690,7 +693,9 @@ __device__ __forceinline__ void bay_gemm_propose_impl(const bay_stretch_params& 
                 if (d >= DIM) continue;
                 const float v = MODE == 2 ? xv[q] : __fmaf_rn(z, __fsub_rn(xv[q], sv[q]), sv[q]);
                 y[d] = v;
+#if BAY_ANY_SPACE
                 sY[i][d] = v;
+#endif
                 const unsigned int f = d - BAY_GEMM_COEF;
                 if (d < BAY_GEMM_COEF || f >= BAY_GEMM_F) continue;
                 if (!P.s_bh) {
@@ -707,7 +712,11 @@ __device__ __forceinline__ void bay_gemm_propose_impl(const bay_stretch_params& 
     __syncthreads();
     const unsigned int k = k0 + threadIdx.x;
     if (threadIdx.x < BAY_PW && k < nk) {
+#if BAY_ANY_SPACE
         const float* y = sY[threadIdx.x];
+#else
+        const float* y = P.s_y + (size_t)k * DIM;
+#endif
         const float* hyper = P.params + P.data_len;
         float pr[BAY_PREP_LEN];
 #pragma unroll

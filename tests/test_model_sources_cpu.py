@@ -1,6 +1,8 @@
 """Which plain-form sources get kernels with their params in shared memory (named _s): plain C and
 arithmetic, not what names an address space or has shared memory of its own.  From ptxas' report,
 no device needed."""
+import re
+
 import pytest
 
 BASE = """
@@ -83,3 +85,28 @@ def test_the_built_in_models_may(native, monkeypatch, capfd):
                for k, v in M.likelihood_models().items()]
     for m in models:
         assert staged(m, monkeypatch, capfd, "built in"), m.name
+
+
+def test_a_gemm_source_with_shared_memory_of_its_own_can_be_launched(native, monkeypatch, capfd):
+    """The streamed propose kernel keeps 8 rows of 1,500 coordinates in static shared memory, which
+    leaves no room in the 48 KB of a launch for the source's: such a source's rows are read from
+    global memory."""
+    from bayadera_gb300 import models as M
+    from bayadera_gb300.engine import check_model
+    src = M.get_source("mvn_precision") + """
+extern "C" {
+inline void own_prep(const REAL* hyper, const uint32_t hyper_len, const uint32_t dim, const REAL* x, REAL* prep) {
+    __shared__ volatile REAL table[2048];
+    table[threadIdx.x] = x[0];
+    prep[0] = table[threadIdx.x];
+}
+}
+"""
+    gemm = dict(M.mvn_precision_model(8).gemm, prep="own_prep", features=8, ld=8, rows=8)
+    m = M.device_distribution_model(src, name="own", dimension=1500, params_size=64,
+                                    logpdf="mvn_precision_logpdf", gemm=gemm)
+    monkeypatch.setenv("BAY_PTXAS_VERBOSE", "1")
+    capfd.readouterr()
+    check_model(m, "gemm")
+    used = re.findall(r"entry function '(bay_gemm_propose_\w+)'.*?(\d+) bytes smem", capfd.readouterr().err, re.S)
+    assert len(used) == 3 and all(int(n) <= 48 * 1024 for _, n in used), used
