@@ -346,13 +346,26 @@ struct bay_model {
     // batch form: propose / accept in k_gp / k_ga, rows in k_gr, per-step means here
     CUkernel k_bmeans = nullptr;
     uint32_t row_len = 0;
-    // plain form: the density engines' point kernels
-    CUkernel k_points = nullptr, k_evidence = nullptr;
-    CUkernel k_staged[5] = {};   // plain form, params in shared memory: bare, accu, logfn, points, evidence
-    bool staging = false;        // ... may be launched
+    // plain form: the log densities' kernel [0], the moves' (bare, accu) [1] and the density engines'
+    // (points, evidence) [2], with the params in global memory or staged in shared memory: a module
+    // each, compiled when first needed (load_plain): a program needs three or four of the ten
+    // kernels.  Compiling a model and creating a sampler 560 -> 221 ms, a density engine and its
+    // first call 545 -> 199 ms (five kernels, none staged, in one module: 223 and 209 ms)
+    struct plain_module {
+        CUlibrary lib = nullptr;
+        CUkernel k[2] = {};
+        bool opted = false;                 // more than 48 KB of shared memory has been asked for
+    } plain[3][2];                          // [..][staged]
+    std::string plain_src, plain_id;
+    std::vector<std::string> plain_opts;
+    size_t staging[3] = {};                 // most bytes that may be staged
 };
 
 namespace {
+std::vector<char> nvrtc_compile(const std::string& src, const std::vector<std::string>& opts,
+                                const std::string& id);
+bool nvrtc_compiled(const std::vector<std::string>& opts, const std::string& id);
+
 constexpr uint32_t kGemmWalkers = 64;             // BAY_WT in device/bay_stretch.cuh
 constexpr size_t kGemmMaxSmem = 200 * 1024;       // dynamic shared memory cap per CTA
 
@@ -367,15 +380,66 @@ size_t gemm_smem_bytes(const bay_model* m, uint64_t rows) {
 }
 
 // Plain form: dynamic shared memory of a launch of `ctas` CTAs, the whole params where they are
-// staged (bay_stage_begin) or 0.  Up to 48 KB they are (4 CTAs of 256 threads an SM still fit);
+// staged (bay_stage_begin) or 0.  Up to 44 KB they are (4 CTAs of 256 threads an SM still fit);
 // up to 200 KB where every CTA has an SM to itself anyway.  16-byte-aligned params only, and only
 // where the model's kernels may have the shared memory (their own static arrays take of it).
 constexpr size_t kPlainSmem = 48 * 1024 - 4096, kPlainSmemMax = 200 * 1024;
-size_t plain_smem(const bay_model* m, const float* params, uint64_t n_params, uint64_t ctas, int sm_count) {
-    if (!m->staging) return 0;
+constexpr size_t kPlainSmemFree = 32 * 1024;   // without opting in: 48 KB with 1,024 threads' sums
+enum { kPlainLogfn = 0, kPlainMove = 1, kPlainPoints = 2 };
+size_t plain_smem(const bay_model* m, int group, const float* params, uint64_t n_params, uint64_t ctas) {
     const uint64_t bytes = (n_params * sizeof(float) + 15) & ~15ull;
     if (n_params == 0 || (uintptr_t)params % 16) return 0;
-    return bytes <= (ctas <= (uint64_t)sm_count ? kPlainSmemMax : kPlainSmem) ? (size_t)bytes : 0;
+    const size_t most = ctas <= (uint64_t)m->ctx->sm_count ? kPlainSmemMax : kPlainSmem;
+    return bytes <= std::min(most, m->staging[group]) ? (size_t)bytes : 0;
+}
+
+std::vector<std::string> plain_options(std::vector<std::string> opts, int group, bool staged) {
+    opts.push_back("-DBAY_PLAIN_GROUP=" + std::to_string(group));
+    opts.push_back(staged ? "-DBAY_PLAIN_STAGED=1" : "-DBAY_PLAIN_STAGED=0");
+    return opts;
+}
+
+// The plain form's module `group` for a launch with `smem` bytes of params staged (0: none), loaded;
+// false where that much shared memory is refused (the model's staging bound then falls below it).
+// Under the context's lock; not while a launch is being captured.
+bool load_plain(bay_model* m, int group, size_t smem) {
+    auto& p = m->plain[group][smem != 0];
+    if (!p.lib) {
+        const std::vector<std::string> opts = plain_options(m->plain_opts, group, smem != 0);
+        const std::vector<char> cubin = nvrtc_compile(m->plain_src, opts, m->plain_id);
+        const char* const names[3][2] = {{"bay_logfn_all", nullptr},
+                                         {"bay_stretch_bare", "bay_stretch_accu"},
+                                         {"bay_points_logfn", "bay_points_evidence"}};
+        bay_model::plain_module q;
+        cu_check(g_cu.LibraryLoadData(&q.lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0),
+                 "cuLibraryLoadData");
+        for (int i = 0; i < 2 && names[group][i]; ++i) {
+            const std::string name = std::string(names[group][i]) + (smem ? "_s" : "");
+            const CUresult r = g_cu.LibraryGetKernel(&q.k[i], q.lib, name.c_str());
+            if (r != CUDA_SUCCESS) {
+                g_cu.LibraryUnload(q.lib);
+                cu_check(r, "GetKernel(plain)");
+            }
+        }
+        p = q;
+    }
+    if (smem > kPlainSmemFree && !p.opted) {
+        for (CUkernel k : p.k)
+            if (k && g_cu.KernelSetAttribute(CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)kPlainSmemMax,
+                                             k, (CUdevice)m->ctx->device) != CUDA_SUCCESS) {
+                m->staging[group] = kPlainSmemFree;
+                return false;
+            }
+        p.opted = true;
+    }
+    return true;
+}
+// plain_smem of a launch whose module is loaded
+size_t plain_launch(bay_model* m, int group, const float* params, uint64_t n_params, uint64_t ctas) {
+    const size_t smem = plain_smem(m, group, params, n_params, ctas);
+    if (load_plain(m, group, smem)) return smem;
+    load_plain(m, group, 0);
+    return 0;
 }
 
 // Streamed GEMM form: walkers per CTA of the propose kernel (BAY_PW), their rows in at most
@@ -482,9 +546,23 @@ const char* kStdint =
     "typedef unsigned int uint32_t; typedef int int32_t;\n"
     "typedef unsigned long long uint64_t; typedef long long int64_t;\n";
 
-std::vector<char> nvrtc_compile(const std::string& src, const std::vector<std::string>& opts) {
-    std::string key = src;
+std::string cubin_key(const std::vector<std::string>& opts, const std::string& id) {
+    std::string key = id;
     for (auto& o : opts) key += "\n//" + o;
+    return key;
+}
+
+// Whether nvrtc_compile would find its answer in the cache.
+bool nvrtc_compiled(const std::vector<std::string>& opts, const std::string& id) {
+    std::lock_guard<std::mutex> g(g_cache_mu);
+    return g_cubin_cache.count(cubin_key(opts, id)) != 0;
+}
+
+// id: what tells src from other sources (a model's own source and form, which is a twentieth of
+// the whole; the source itself)
+std::vector<char> nvrtc_compile(const std::string& src, const std::vector<std::string>& opts,
+                                const std::string& id) {
+    const std::string key = cubin_key(opts, id);
     {
         std::lock_guard<std::mutex> g(g_cache_mu);
         auto it = g_cubin_cache.find(key);
@@ -627,8 +705,8 @@ struct bay_sampler {
     uint32_t plain_split() const {
         if (model->form != BAY_FORM_PLAIN || model->cta != 256 || grid() >= (unsigned)ctx->sm_count) return 1u;
         // (not where the params are staged by whole CTAs alone)
-        return plain_smem(model, params, n_params, 4ull * grid(), ctx->sm_count) ||
-                       !plain_smem(model, params, n_params, grid(), ctx->sm_count)
+        return plain_smem(model, kPlainMove, params, n_params, 4ull * grid()) ||
+                       !plain_smem(model, kPlainMove, params, n_params, grid())
                    ? 4u : 1u;
     }
 
@@ -737,7 +815,7 @@ struct bay_sampler {
         cfg.blockDimY = 1;
         cfg.blockDimZ = 1;
         cfg.sharedMemBytes = (unsigned)(tcr || tiled ? smem_move
-                                        : plain ? plain_smem(model, params, n_params, cfg.gridDimX, ctx->sm_count)
+                                        : plain ? plain_smem(model, kPlainMove, params, n_params, cfg.gridDimX)
                                                 : smem);
         cfg.hStream = (CUstream)st;
         cfg.attrs = at;
@@ -750,13 +828,30 @@ struct bay_sampler {
             cl.value.clusterDim.z = 1;
         }
         CUkernel k = tcr ? model->k_tr[accu ? 1 : 0]
-                         : plain && cfg.sharedMemBytes ? model->k_staged[accu ? 1 : 0]
-                                                       : (accu ? model->k_accu : model->k_bare);
+                         : plain ? model->plain[kPlainMove][cfg.sharedMemBytes != 0].k[accu ? 1 : 0]
+                                 : (accu ? model->k_accu : model->k_bare);
         cu_check(g_cu.LaunchKernelEx(&cfg, (CUfunction)k, args, nullptr), "cuLaunchKernelEx(stretch)");
     }
 
     void ctl_op(const bay_ctl_op& op) {
         cuda_check(bay::launch_ctl_apply(ctl, op, ctx->stream), "ctl_apply");
+    }
+
+    // CTAs of the plain form's log-density launch
+    uint64_t plain_logfn_grid() const {
+        const uint64_t per = model->cta / plain_split();
+        return (W + per - 1) / per;
+    }
+
+    // the plain form's modules that this sampler's launches take (the moves' first: the split
+    // goes by what they may stage)
+    void load_plain_kernels() {
+        uint32_t split;
+        do {
+            split = plain_split();
+            plain_launch(model, kPlainMove, params, n_params, (uint64_t)grid() * split);
+        } while (split != plain_split());
+        plain_launch(model, kPlainLogfn, params, n_params, plain_logfn_grid());
     }
 
     void launch_logfn_all() {
@@ -769,10 +864,9 @@ struct bay_sampler {
         void* args[] = {&p};
         const bool plain = model->form == BAY_FORM_PLAIN;
         const uint32_t block = tcr ? 256 : plain ? model->cta / plain_split() : model->cta;
-        const uint64_t per = plain ? block : per_cta();
-        const unsigned g = (unsigned)((W + per - 1) / per);
-        const size_t sm = plain ? plain_smem(model, params, n_params, g, ctx->sm_count) : smem;
-        CUkernel k = tcr ? model->k_tr[2] : plain && sm ? model->k_staged[2] : model->k_logfn;
+        const unsigned g = (unsigned)(plain ? plain_logfn_grid() : (W + per_cta() - 1) / per_cta());
+        const size_t sm = plain ? plain_smem(model, kPlainLogfn, params, n_params, g) : smem;
+        CUkernel k = tcr ? model->k_tr[2] : plain ? model->plain[kPlainLogfn][sm != 0].k[0] : model->k_logfn;
         cu_check(g_cu.LaunchKernel((CUfunction)k, g, 1, 1, block, 1, 1, (unsigned)sm,
                                    (CUstream)ctx->stream, args, nullptr),
                  "cuLaunchKernel(logfn)");
@@ -1073,7 +1167,7 @@ int bay_ctx_allocated(bay_ctx* c, uint64_t* out) {
 
 namespace {
 struct Codegen {
-    std::string src;
+    std::string src, id;
     std::vector<std::string> opts;
     uint32_t cta = 256, wpc = 1;
     uint32_t tc_g = 0, tc_stages = 0;
@@ -1104,54 +1198,56 @@ bool any_space_source(const char* source) {
         "__fadd_", "__fsub_", "__fmul_", "__fmaf_", "__fdiv_", "__frcp_", "__fsqrt_", "__frsqrt_", "__dadd_",
         "__dsub_", "__dmul_", "__fma_", "__ddiv_", "__drcp_", "__dsqrt_", "__float2", "__double2", "__int2",
         "__uint2", "__ll2", "__ull2", "__funnelshift_"};
-    std::string s;   // without the spliced line ends
-    for (const char* p = source; *p; ++p) {
-        if (*p == '\\') {
+    // without the spliced line ends (copied only where there is a backslash: a model's preparation
+    // pays for every pass over its source)
+    std::string spliced;
+    if (std::strchr(source, '\\')) {
+        for (const char* p = source; *p; ++p) {
             const char* q = p + 1;
-            while (*q == ' ' || *q == '\t' || *q == '\r') ++q;
-            if (*q == '\n') {
-                p = q;
-                continue;
-            }
+            if (*p == '\\')
+                while (*q == ' ' || *q == '\t' || *q == '\r') ++q;
+            if (*p == '\\' && *q == '\n') p = q;
+            else spliced += *p;
         }
-        s += *p;
+        source = spliced.c_str();
     }
-    const auto word_char = [](char c) { return std::isalnum((unsigned char)c) || c == '_'; };
-    for (size_t i = 0; i < s.size();) {
-        const char c = s[i];
-        if (s.compare(i, 2, "//") == 0) {
-            i = std::min(s.find('\n', i), s.size());
-        } else if (s.compare(i, 2, "/*") == 0) {
-            i = s.find("*/", i + 2);
-            if (i == std::string::npos) return false;
-            i += 2;
-        } else if (c == '\\' || s.compare(i, 2, "##") == 0 || s.compare(i, 2, "%:") == 0) {
-            return false;
-        } else if (c == '"' || c == '\'') {
-            for (++i; i < s.size() && s[i] != c; ++i)
-                if (s[i] == '\\') ++i;
-            ++i;
-        } else if (std::isdigit((unsigned char)c)) {   // digits may be parted by '
-            while (i < s.size() && (word_char(s[i]) || s[i] == '.' || s[i] == '\'')) ++i;
+    const auto word_char = [](char c) {
+        return (c >= 'a' && c <= 'z') || (c >= 'A' && c <= 'Z') || (c >= '0' && c <= '9') || c == '_';
+    };
+    for (const char* p = source; *p;) {
+        const char c = *p;
+        if (c >= '0' && c <= '9') {                          // digits may be parted by '
+            while (word_char(*p) || *p == '.' || *p == '\'') ++p;
         } else if (word_char(c)) {
-            size_t j = i;
-            while (j < s.size() && word_char(s[j])) ++j;
-            const std::string w = s.substr(i, j - i);
-            i = j;
-            if (w == "asm" || (w.back() == 'R' && i < s.size() && s[i] == '"')) return false;
-            if (w == "include") {
-                const size_t e = std::min(s.find('\n', i), s.size());
+            const char* w = p;
+            while (word_char(*p)) ++p;
+            const size_t len = (size_t)(p - w);
+            if ((len == 3 && !std::memcmp(w, "asm", 3)) || (p[-1] == 'R' && *p == '"')) return false;
+            if (len == 7 && !std::memcmp(w, "include", 7)) {
                 std::string h;
-                for (; i < e; ++i)
-                    if (!std::isspace((unsigned char)s[i])) h += s[i];
+                for (; *p && *p != '\n'; ++p)
+                    if (*p != ' ' && *p != '\t' && *p != '\r') h += *p;
                 if (h.compare(0, 10, "<stdint.h>") != 0 && h.compare(0, 9, "<cstdint>") != 0) return false;
             }
-            if (w.compare(0, 2, "__") == 0 && !known.count(w) &&
-                std::none_of(std::begin(families), std::end(families),
-                             [&](const char* f) { return w.compare(0, std::strlen(f), f) == 0; }))
+            if (c == '_' && len > 1 && w[1] == '_' && !known.count(std::string(w, len)) &&
+                std::none_of(std::begin(families), std::end(families), [&](const char* f) {
+                    return len > std::strlen(f) && !std::memcmp(w, f, std::strlen(f));
+                }))
                 return false;
+        } else if (c == '/' && p[1] == '/') {
+            while (*p && *p != '\n') ++p;
+        } else if (c == '/' && p[1] == '*') {
+            p = std::strstr(p + 2, "*/");
+            if (!p) return false;
+            p += 2;
+        } else if (c == '\\' || (c == '#' && p[1] == '#') || (c == '%' && p[1] == ':')) {
+            return false;
+        } else if (c == '"' || c == '\'') {
+            for (++p; *p && *p != c; ++p)
+                if (*p == '\\' && p[1]) ++p;
+            if (*p) ++p;
         } else {
-            ++i;
+            ++p;
         }
     }
     return true;
@@ -1182,8 +1278,10 @@ Codegen codegen(const bay_model_desc* d, uint32_t wgs) {
             fail(BAY_ERR_ARG, "BAY_MODEL_PARTNER_ELEMENT applies to the plain and tiled forms");
         opts.push_back("-DBAY_PARTNER_ELEMENT=1");
     }
-    g.any_space = any_space_source(d->source);
-    opts.push_back(std::string("-DBAY_ANY_SPACE=") + (g.any_space ? "1" : "0"));
+    if (d->form != BAY_FORM_TILED) {
+        g.any_space = any_space_source(d->source);
+        opts.push_back(std::string("-DBAY_ANY_SPACE=") + (g.any_space ? "1" : "0"));
+    }
     uint32_t wpc = 1;
     if (d->form == BAY_FORM_PLAIN) {
         if (!valid_ident(d->logfn)) fail(BAY_ERR_ARG, "logfn must name a C function");
@@ -1265,6 +1363,7 @@ Codegen codegen(const bay_model_desc* d, uint32_t wgs) {
     } else {
         fail(BAY_ERR_ARG, "unknown model form");
     }
+    g.id = std::string(d->source) + "\x1f" + std::to_string((int)d->form);
     std::string& src = g.src;
     src += "#include <stdint.h>\n";
     src += bay_embedded_rng;
@@ -1288,8 +1387,21 @@ extern "C" {
 int bay_model_check(const bay_model_desc* d, uint32_t wgs) {
     return guarded([&] {
         Codegen g = codegen(d, wgs ? wgs : 1024u);
-        nvrtc_compile(g.src, g.opts);
+        if (d->form == BAY_FORM_PLAIN) {
+            for (int which = 0; which < (g.any_space ? 6 : 3); ++which)
+                nvrtc_compile(g.src, plain_options(g.opts, which % 3, which / 3 != 0), g.id);
+            return;
+        }
+        nvrtc_compile(g.src, g.opts, g.id);
     });
+}
+
+static void unload(bay_model* m) {
+    if (m->lib) g_cu.LibraryUnload(m->lib);
+    for (auto& group : m->plain)
+        for (auto& p : group)
+            if (p.lib) g_cu.LibraryUnload(p.lib);
+    delete m;
 }
 
 int bay_model_compile(bay_ctx* c, const bay_model_desc* d, bay_model** out) {
@@ -1300,7 +1412,9 @@ int bay_model_compile(bay_ctx* c, const bay_model_desc* d, bay_model** out) {
         std::lock_guard<std::recursive_mutex> lk(c->mu);
         c->use();
         Codegen g = codegen(d, c->wgs);
-        std::vector<char> cubin = nvrtc_compile(g.src, g.opts);
+        const bool plain = d->form == BAY_FORM_PLAIN;
+        std::vector<char> cubin;
+        if (!plain) cubin = nvrtc_compile(g.src, g.opts, g.id);
         bay_model* m = new bay_model();
         m->ctx = c;
         m->dim = d->dim;
@@ -1327,6 +1441,20 @@ int bay_model_compile(bay_ctx* c, const bay_model_desc* d, bay_model** out) {
             m->tr_free = g.tr_free;
         }
         try {
+            if (plain) {
+                m->plain_src = std::move(g.src);
+                m->plain_id = g.id;
+                m->plain_opts = g.opts;
+                for (size_t& b : m->staging) b = g.any_space ? kPlainSmemMax : 0;
+                load_plain(m, kPlainLogfn, g.any_space ? 1 : 0);
+                // the density engines' too, where an earlier model of the source had them (and opted
+                // in, which loads their code now and not in the first call)
+                for (int staged = 0; staged < 2; ++staged)
+                    if (nvrtc_compiled(plain_options(m->plain_opts, kPlainPoints, staged != 0), m->plain_id))
+                        load_plain(m, kPlainPoints, staged ? kPlainSmemMax : 0);
+                *out = m;
+                return;
+            }
             cu_check(g_cu.LibraryLoadData(&m->lib, cubin.data(), nullptr, nullptr, 0, nullptr,
                                        nullptr, 0),
                      "cuLibraryLoadData");
@@ -1368,25 +1496,6 @@ int bay_model_compile(bay_ctx* c, const bay_model_desc* d, bay_model** out) {
                 cu_check(g_cu.LibraryGetKernel(&m->k_bare, m->lib, "bay_stretch_bare"), "GetKernel(bare)");
                 cu_check(g_cu.LibraryGetKernel(&m->k_accu, m->lib, "bay_stretch_accu"), "GetKernel(accu)");
                 cu_check(g_cu.LibraryGetKernel(&m->k_logfn, m->lib, "bay_logfn_all"), "GetKernel(logfn)");
-                if (d->form == BAY_FORM_PLAIN) {
-                    cu_check(g_cu.LibraryGetKernel(&m->k_points, m->lib, "bay_points_logfn"),
-                             "GetKernel(points)");
-                    cu_check(g_cu.LibraryGetKernel(&m->k_evidence, m->lib, "bay_points_evidence"),
-                             "GetKernel(evidence)");
-                }
-            }
-            if (d->form == BAY_FORM_PLAIN && g.any_space) {
-                CUdevice dev = (CUdevice)c->device;
-                const char* st[5] = {"bay_stretch_bare_s", "bay_stretch_accu_s", "bay_logfn_all_s",
-                                     "bay_points_logfn_s", "bay_points_evidence_s"};
-                for (int i = 0; i < 5; ++i) {
-                    cu_check(g_cu.LibraryGetKernel(&m->k_staged[i], m->lib, st[i]), "GetKernel(staged)");
-                    // refused where the source's own static shared memory leaves less
-                    m->staging = (i == 0 || m->staging) &&
-                                 g_cu.KernelSetAttribute(CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES,
-                                                         (int)kPlainSmemMax, m->k_staged[i], dev) ==
-                                     CUDA_SUCCESS;
-                }
             }
             if (d->form == BAY_FORM_TILED) {
                 CUdevice dev = (CUdevice)c->device;
@@ -1436,8 +1545,7 @@ int bay_model_compile(bay_ctx* c, const bay_model_desc* d, bay_model** out) {
                 }
             }
         } catch (...) {
-            if (m->lib) g_cu.LibraryUnload(m->lib);
-            delete m;
+            unload(m);
             throw;
         }
         *out = m;
@@ -1447,8 +1555,7 @@ int bay_model_compile(bay_ctx* c, const bay_model_desc* d, bay_model** out) {
 int bay_model_release(bay_model* m) {
     return guarded([&] {
         if (!m) return;
-        if (m->lib) g_cu.LibraryUnload(m->lib);
-        delete m;
+        unload(m);
     });
 }
 
@@ -1593,6 +1700,7 @@ static int sampler_create(bay_model* m, uint32_t seed, uint64_t walkers, const f
                 s->params = p;
                 s->own_params = true;
             }
+            if (m->form == BAY_FORM_PLAIN) s->load_plain_kernels();
             if (s->streaming) {
                 const size_t Wn = walkers;
                 s->s_y = (float*)c->alloc(sizeof(float) * Wn * s->D);
@@ -1948,7 +2056,7 @@ void hist_count(bay_ctx* c, uint32_t flags, const float* x, uint32_t D, uint64_t
         const std::vector<std::string> opts = {"-arch=sm_103a", "-use_fast_math", "-default-device",
                                                "-std=c++17",
                                                "-DBAY_HIST_BINS=" + std::to_string(bins)};
-        std::vector<char> cubin = nvrtc_compile(src, opts);
+        std::vector<char> cubin = nvrtc_compile(src, opts, src);
         CUlibrary lib = nullptr;
         cu_check(g_cu.LibraryLoadData(&lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0),
                  "cuLibraryLoadData(histogram)");

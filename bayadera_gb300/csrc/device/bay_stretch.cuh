@@ -2304,9 +2304,9 @@ extern "C" __global__ void __launch_bounds__(1024, 1) bay_tcr_run_accu(bay_stret
 // One thread per walker of the moving half, the model's LOGFN evaluated per thread
 // (the reference's structure, with SoA coalesced loads and registers for Y).
 
-// The params staged in shared memory (STAGED: kernels of their own, named _s, launched with
-// dynamic shared memory for them; else they stay in global memory, always so where the source
-// may read them by global loads alone: BAY_ANY_SPACE 0).  One kernel for both, with
+// The params staged in shared memory (STAGED: a module with kernels of their own, named _s,
+// launched with dynamic shared memory for them; else they stay in global memory, always so where
+// the source may read them by global loads alone).  One kernel for both, with
 // the density twice in it, had ptxas schedule the loads from global memory worse: 8,192 walkers
 // x 65,536 rows of 65 floats 43.8 -> 62.4 ms an accu launch.  A density's loop reads them in order, all threads alike, a load
 // every few arithmetic instructions of one dependent sum: from global memory, L1 hits
@@ -2314,6 +2314,11 @@ extern "C" __global__ void __launch_bounds__(1024, 1) bay_tcr_run_accu(bay_stret
 // shared memory 8 (8,192 walkers x 1,000 rows: 18.8 us a launch, now 5.7).
 // One bulk copy, begun before the launch waits for its predecessor (the params never
 // change while a sampler runs), the last floats past its 16-byte multiple by plain loads.
+#if BAY_PLAIN_STAGED
+#define BAY_PLAIN(name) name##_s
+#else
+#define BAY_PLAIN(name) name
+#endif
 struct bay_plain_sync {
     unsigned long long bar;
 };
@@ -2437,18 +2442,12 @@ __device__ __forceinline__ void bay_stretch_plain(const bay_stretch_params& P) {
     }
 }
 
-extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_bare(bay_stretch_params P) {
-    bay_stretch_plain<false, false>(P);
+#if BAY_PLAIN_GROUP == 1
+extern "C" __global__ void __launch_bounds__(BAY_CTA) BAY_PLAIN(bay_stretch_bare)(bay_stretch_params P) {
+    bay_stretch_plain<false, BAY_PLAIN_STAGED>(P);
 }
-extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_accu(bay_stretch_params P) {
-    bay_stretch_plain<true, false>(P);
-}
-#if BAY_ANY_SPACE
-extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_bare_s(bay_stretch_params P) {
-    bay_stretch_plain<false, true>(P);
-}
-extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_stretch_accu_s(bay_stretch_params P) {
-    bay_stretch_plain<true, true>(P);
+extern "C" __global__ void __launch_bounds__(BAY_CTA) BAY_PLAIN(bay_stretch_accu)(bay_stretch_params P) {
+    bay_stretch_plain<true, BAY_PLAIN_STAGED>(P);
 }
 #endif
 
@@ -2465,12 +2464,9 @@ __device__ __forceinline__ void bay_logfn_plain(const bay_stretch_params& P) {
     for (int i = 0; i < DIM; ++i) x[i] = P.xs[(size_t)k * DIM + i];
     P.logfn[k] = bay_density<STAGED>((unsigned int)P.data_len, P.params_len, P.params, x);
 }
-extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_logfn_all(bay_stretch_params P) {
-    bay_logfn_plain<false>(P);
-}
-#if BAY_ANY_SPACE
-extern "C" __global__ void __launch_bounds__(BAY_CTA) bay_logfn_all_s(bay_stretch_params P) {
-    bay_logfn_plain<true>(P);
+#if BAY_PLAIN_GROUP == 0
+extern "C" __global__ void __launch_bounds__(BAY_CTA) BAY_PLAIN(bay_logfn_all)(bay_stretch_params P) {
+    bay_logfn_plain<BAY_PLAIN_STAGED>(P);
 }
 #endif
 
@@ -2493,16 +2489,11 @@ bay_points_density(unsigned long long n, unsigned int data_len, unsigned int par
         out[i] = exp_out ? expf(v) : v;
     }
 }
+#if BAY_PLAIN_GROUP == 2
 extern "C" __global__ void __launch_bounds__(BAY_CTA)
-bay_points_logfn(unsigned long long n, unsigned int data_len, unsigned int params_len,
-                 const float* params, const float* x, float* out, unsigned int exp_out) {
-    bay_points_density<false>(n, data_len, params_len, params, x, out, exp_out);
-}
-#if BAY_ANY_SPACE
-extern "C" __global__ void __launch_bounds__(BAY_CTA)
-bay_points_logfn_s(unsigned long long n, unsigned int data_len, unsigned int params_len,
-                   const float* params, const float* x, float* out, unsigned int exp_out) {
-    bay_points_density<true>(n, data_len, params_len, params, x, out, exp_out);
+BAY_PLAIN(bay_points_logfn)(unsigned long long n, unsigned int data_len, unsigned int params_len,
+                            const float* params, const float* x, float* out, unsigned int exp_out) {
+    bay_points_density<BAY_PLAIN_STAGED>(n, data_len, params_len, params, x, out, exp_out);
 }
 #endif
 
@@ -2534,16 +2525,11 @@ bay_points_sum(unsigned long long n, unsigned int data_len, unsigned int params_
     }
     if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
+#if BAY_PLAIN_GROUP == 2
 extern "C" __global__ void __launch_bounds__(BAY_CTA)
-bay_points_evidence(unsigned long long n, unsigned int data_len, unsigned int params_len,
-                    const float* params, const float* x, double* part) {
-    bay_points_sum<false>(n, data_len, params_len, params, x, part);
-}
-#if BAY_ANY_SPACE
-extern "C" __global__ void __launch_bounds__(BAY_CTA)
-bay_points_evidence_s(unsigned long long n, unsigned int data_len, unsigned int params_len,
-                      const float* params, const float* x, double* part) {
-    bay_points_sum<true>(n, data_len, params_len, params, x, part);
+BAY_PLAIN(bay_points_evidence)(unsigned long long n, unsigned int data_len, unsigned int params_len,
+                               const float* params, const float* x, double* part) {
+    bay_points_sum<BAY_PLAIN_STAGED>(n, data_len, params_len, params, x, part);
 }
 #endif
 
