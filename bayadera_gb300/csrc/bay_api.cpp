@@ -245,6 +245,10 @@ struct bay_ctx {
         est_ws = nullptr;
         est_ws_bytes = 0;
     }
+    // after a handle's memory has gone back: with no other handle's left, so does what is kept
+    void handle_released() {
+        if (allocated == sc_cap + est_ws_bytes) give_back();
+    }
     void release(void* p) {
         if (!p) return;
         auto it = sizes.find(p);
@@ -1835,6 +1839,7 @@ int bay_sampler_release(bay_sampler* s) {
         for (float* q : {s->s_y, s->s_b, s->s_prep, s->s_w, s->s_zu, s->s_part}) c->release(q);
         for (unsigned short* q : {s->tc_xh, s->tc_xl, s->s_bh, s->s_bl}) c->release(q);
         if (s->own_params) c->release((void*)s->params);
+        c->handle_released();
         delete s;
     });
 }

@@ -65,7 +65,8 @@ int bay_ctx_processing_elements(bay_ctx* ctx, uint64_t* out);
 int bay_ctx_stream(bay_ctx* ctx, void** stream);
 int bay_ctx_synchronize(bay_ctx* ctx);
 /* Bytes currently allocated by this context (with the workspaces it keeps between calls: at
- * most 64 MiB and the estimates' partial results, given back when an allocation needs room). */
+ * most 64 MiB and the estimates' partial results, given back when an allocation needs room and
+ * when the last sampler or batch is released). */
 int bay_ctx_allocated(bay_ctx* ctx, uint64_t* out);
 /* Kernels this library has enqueued in this process, all contexts (each replayed graph
  * counts its kernel nodes).  No reference counterpart: an instrumentation counter. */

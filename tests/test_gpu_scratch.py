@@ -65,3 +65,34 @@ def test_a_call_settles_what_is_kept_the_first_time():
             e.log_density(np.float32([0.0]), points(50))      # 75 MiB
             assert f.allocated() == held[1]
         e.release()
+
+
+def test_with_its_last_handle_a_context_gives_everything_back():
+    """A host's leak check: what is allocated after the handles' release is what was before."""
+    from bayadera_gb300 import models as M
+    from bayadera_gb300.engine import GB300BayaderaFactory
+    with GB300BayaderaFactory() as f:
+        before = f.allocated()
+        sf = f.mcmc_factory(M.mvn_precision_model(5), form="gemm")
+        a, b = (sf.create_sampler(i, 512, np.eye(5, dtype=np.float32).reshape(-1)) for i in (1, 2))
+        for s in (a, b):
+            s.init_position_normal(3, 0.0, 1.0)
+            s.run_sampler(60, 2.0)
+            s.sd()
+            s.histogram(1, 64)
+        f.acor(series(3))
+        held = f.allocated()
+        a.release()
+        assert 3 * MB < f.allocated() < held              # kept for the other one
+        b.release()
+        assert f.allocated() == before
+        sf.release()
+        sf = f.mcmc_factory(M.hierarchical_rows_batch_model(3), form="batch")
+        params, rows = M.hierarchical_rows_params([np.ones(9)] * 3, np.ones(3))
+        h = sf.create_batch([dict(dim=5, seed=1, walkers=64, params=params, rows=rows)])
+        h.init_position_normal([2], 0.0, 1.0)
+        h.burn_in(2, 2.0)
+        f.acor(series(1))
+        h.release()
+        assert f.allocated() == before
+        sf.release()
