@@ -2342,6 +2342,7 @@ int bay_histogram(bay_sampler* s, uint32_t cycles, uint32_t bins, uint32_t flags
             c->release(s->counts);
             s->hist = nullptr;
             s->counts = nullptr;
+            s->hist_bins = 0;   // an allocation that fails leaves none
             s->hist = (float*)c->alloc(sizeof(float) * (2 * (size_t)s->D + 2 * (size_t)bins * s->D));
             s->counts = (uint32_t*)c->alloc(sizeof(uint32_t) * (size_t)bins * s->D);
             s->hist_bins = bins;
