@@ -1048,6 +1048,7 @@ struct bay_sampler {
         if (means_cap >= n && means) return;
         ctx->release(means);
         means = nullptr;
+        g_accu_cap = ~0ull;   // a captured chunk holds the old address, even if no new one comes
         means_cap = 0;
         means = (float*)ctx->alloc(sizeof(float) * (size_t)D * (size_t)std::max<uint64_t>(n, 1));
         means_cap = n;
