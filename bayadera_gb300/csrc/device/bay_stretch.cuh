@@ -374,8 +374,8 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
     // ((step_off, 0) for half 1, (step_off - 1, 1) for half 0; the chunk's last half-step has
     // a launch of its own), beside the eight that move the walkers.  At the end of the moving
     // half's own launch the sums were a serial chain of 64 compensated additions that
-    // everything waited for: 12,290 walkers of 37 dimensions 8.3 -> 6.3 us a launch,
-    // 16,384 of 50 10.7 -> 7.4.
+    // everything waited for: 12,290 walkers of 37 dimensions 8.3 -> 5.9 us a launch,
+    // 16,384 of 50 10.7 -> 7.2.
     if (ACCU && tid >= 256u) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (P.means_cap != 0 && (P.half == 1u || P.step_off > 0u))
@@ -2415,11 +2415,19 @@ __device__ __forceinline__ void bay_stretch_plain(const bay_stretch_params& P) {
             const float s = bay_partner_coord(S, P.K, j, i);
             Y[i] = __fmaf_rn(z, __fsub_rn(X[(size_t)k * DIM + i], s), s);
         }
-        const float lx = P.logfn[(size_t)P.half * P.K + k];
-        const bool ok = bay_stage_wait<STAGED>(&sSync, &P.ctl->status);
         float ly = 0.0f;
-        if (ok) {   // else the params may be anything, lengths and offsets that it goes by too
+        if (STAGED) {
+            const float lx = P.logfn[(size_t)P.half * P.K + k];
+            if (bay_stage_wait<STAGED>(&sSync, &P.ctl->status)) {
+                // else the params may be anything, lengths and offsets that it goes by too
+                ly = bay_density<STAGED>((unsigned int)P.data_len, P.params_len, P.params, Y);
+                accepted = bay_accept(u2, z, ly, lx, beta);
+            }
+        } else {
+            // (the log density after the loop over the params: before it, that loop took 1,256 us
+            // of a bare launch of 4,096 walkers x 60,000 rows instead of 793)
             ly = bay_density<STAGED>((unsigned int)P.data_len, P.params_len, P.params, Y);
+            const float lx = P.logfn[(size_t)P.half * P.K + k];
             accepted = bay_accept(u2, z, ly, lx, beta);
         }
         if (accepted) {

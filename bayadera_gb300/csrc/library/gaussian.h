@@ -30,8 +30,8 @@ inline REAL gaussian_loglik(const uint32_t data_len, const REAL* data, const uin
     const REAL sigma = mu_sigma[1];
     if (!(0.0f < sigma)) return nanf("");
     REAL acc = gaussian_log_unscaled(mu, sigma, data[0]) + data_len * gaussian_log_scale(sigma);
-    // 16 terms side by side, added in order
     uint32_t i = 1;
+#if BAY_PLAIN_STAGED   // data in shared memory: 16 terms side by side, added in order
     for (; data_len - i >= 16 && i < data_len; i += 16) {
         const REAL* d = data + i;
         REAL t[16];
@@ -40,6 +40,7 @@ inline REAL gaussian_loglik(const uint32_t data_len, const REAL* data, const uin
 #pragma unroll
         for (int j = 0; j < 16; ++j) acc += t[j];
     }
+#endif
     for (; i < data_len; ++i) acc += gaussian_log_unscaled(mu, sigma, data[i]);
     return acc;
 }
