@@ -438,6 +438,21 @@ bool load_plain(bay_model* m, int group, size_t smem) {
     }
     return true;
 }
+// Whether programmatic dependent launch is a loss for launches of `ctas` CTAs one after another:
+// the device holds one launch and part of the next, which then starts some of its CTAs early, on
+// the SMs with room, and the others where this one's end first, so that some SMs get more than
+// their share.  37 dims x 40,000 walkers of the SIMT GEMM form (313 CTAs, room for 608): 10.6 us a
+// bare launch with it, 9.0 without; 400,000 walkers of the plain form (782 CTAs, 1,216) x 1,000
+// rows 37.1 and 29.0.  It is a gain where the next launch fits too, or next to nothing of it.
+bool pdl_late(CUkernel k, unsigned threads, size_t smem, uint64_t ctas, int sm_count) {
+    CUfunction f = nullptr;
+    cu_check(g_cu.KernelGetFunction(&f, k), "cuKernelGetFunction");
+    int per_sm = 0;
+    cu_check(g_cu.OccupancyMaxActiveBlocks(&per_sm, f, (int)threads, smem), "cuOccupancy");
+    const uint64_t most = (uint64_t)std::max(per_sm, 0) * (uint64_t)sm_count;
+    return ctas + ctas / 10 <= most && most < 2 * ctas;
+}
+
 // plain_smem of a launch whose module is loaded
 size_t plain_launch(bay_model* m, int group, const float* params, uint64_t n_params, uint64_t ctas) {
     const size_t smem = plain_smem(m, group, params, n_params, ctas);
@@ -487,9 +502,9 @@ uint64_t tr_group_bytes(uint32_t dim, uint32_t features) {
 // Tile groups of a move CTA when the model leaves them free: two where an SM holds no second
 // CTA of one group (113,664 bytes each, beside 2 KB of static and 1 KB of reserved shared
 // memory), two groups fit, and the tiles are more than the SMs -- 65,536 walkers of 98 and
-// 128 dims 27.8 -> 18.9 and 24.0 -> 17.7 us a launch.  Where two such CTAs fit they overlap
-// with the next launch's and stay (94 dims 16.1, 17.4 us with two groups); with a tile an SM
-// at most two groups would leave SMs idle (4,096 walkers of 98 dims 6.2, 8.5 us).
+// 128 dims 25.6 -> 18.2 and 23.7 -> 17.4 us a bare launch.  Where two such CTAs fit they overlap
+// with the next launch's and stay (94 dims 15.2, 16.6 us with two groups); with a tile an SM
+// at most two groups would leave SMs idle (4,096 walkers of 98 dims 5.5, 7.9 us).
 constexpr uint64_t kTrPairSmem = 113664;
 uint32_t tr_free_groups(uint64_t base, uint64_t greg, uint64_t tiles, uint64_t sms) {
     return base + greg > kTrPairSmem && base + 2 * greg <= kGemmMaxSmem && tiles > sms ? 2u : 1u;
@@ -705,14 +720,25 @@ struct bay_sampler {
     // Plain form: CTAs that share a group of model->cta walkers.  Below one group an SM the
     // default group of 256 is four CTAs of 64 threads, a cluster in the accu launch, which
     // combines the group's sums as one CTA does: 8,192 walkers x 1,000 rows are 128 CTAs then,
-    // 5.7 us a bare launch, and 8 with 32.
-    uint32_t plain_split() const {
-        if (model->form != BAY_FORM_PLAIN || model->cta != 256 || grid() >= (unsigned)ctx->sm_count) return 1u;
+    // 5.7 us a bare launch, and 8 with 32.  The cluster costs an accu launch 0.6 us: not where
+    // one CTA has all the walkers, or the density has next to nothing to read (4,096 walkers,
+    // 4, 14 and 34 params: 3.7, 3.8 and 3.9 us; one CTA a group 3.0, 3.2 and 4.0).
+    uint32_t plain_split(bool accu) const {
+        if (model->form != BAY_FORM_PLAIN || model->cta != 256 || grid() >= (unsigned)ctx->sm_count ||
+            K <= 64 || (accu && n_params <= 16))
+            return 1u;
         // (not where the params are staged by whole CTAs alone)
         return plain_smem(model, kPlainMove, params, n_params, 4ull * grid()) ||
                        !plain_smem(model, kPlainMove, params, n_params, grid())
                    ? 4u : 1u;
     }
+    // ... of the bare [0] and accu [1] launch: the split, the params staged (bytes or 0) and
+    // programmatic dependent launch (staged ones alone, as bay_stretch_plain waits)
+    struct {
+        uint32_t split = 1;
+        size_t smem = 0;
+        bool pdl = false;
+    } plain_move[2];
 
     // CTAs of the launch that writes the accu statistics (and so of the partials)
     unsigned grid() const { return (unsigned)((K + per_cta() - 1) / per_cta()); }
@@ -806,7 +832,7 @@ struct bay_sampler {
         // copies) and reads what the previous kernel of the stream does not write, then waits
         // (griddepcontrol.wait) for that kernel to complete, so all this overlaps its tail
         const bool tiled = model->form == BAY_FORM_TILED, plain = model->form == BAY_FORM_PLAIN;
-        const uint32_t split = plain_split();
+        const uint32_t split = plain ? plain_move[accu ? 1 : 0].split : 1u;
         CUlaunchAttribute at[2];
         at[0].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
         at[0].value.programmaticStreamSerializationAllowed = 1;
@@ -819,11 +845,11 @@ struct bay_sampler {
         cfg.blockDimY = 1;
         cfg.blockDimZ = 1;
         cfg.sharedMemBytes = (unsigned)(tcr || tiled ? smem_move
-                                        : plain ? plain_smem(model, kPlainMove, params, n_params, cfg.gridDimX)
+                                        : plain ? plain_move[accu ? 1 : 0].smem
                                                 : smem);
         cfg.hStream = (CUstream)st;
         cfg.attrs = at;
-        cfg.numAttrs = pdl && !(plain && !cfg.sharedMemBytes) ? 1 : 0;   // as bay_stretch_plain waits
+        cfg.numAttrs = pdl && !(plain && !plain_move[accu ? 1 : 0].pdl) ? 1 : 0;
         if (accu && split > 1) {
             CUlaunchAttribute& cl = at[cfg.numAttrs++];
             cl.id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
@@ -843,18 +869,27 @@ struct bay_sampler {
 
     // CTAs of the plain form's log-density launch
     uint64_t plain_logfn_grid() const {
-        const uint64_t per = model->cta / plain_split();
+        const uint64_t per = model->cta / plain_move[0].split;
         return (W + per - 1) / per;
     }
 
-    // the plain form's modules that this sampler's launches take (the moves' first: the split
-    // goes by what they may stage)
-    void load_plain_kernels() {
-        uint32_t split;
-        do {
-            split = plain_split();
-            plain_launch(model, kPlainMove, params, n_params, (uint64_t)grid() * split);
-        } while (split != plain_split());
+    // the plain form's launches and the modules they take
+    void plan_plain() {
+        for (int accu = 0; accu < 2; ++accu) {
+            auto& q = plain_move[accu];
+            do {   // (a refused amount of shared memory changes what may be staged, and the split)
+                q.split = plain_split(accu != 0);
+                q.smem = plain_launch(model, kPlainMove, params, n_params, (uint64_t)grid() * q.split);
+            } while (q.split != plain_split(accu != 0));
+            q.pdl = q.smem && !pdl_late(model->plain[kPlainMove][1].k[accu], model->cta / q.split, q.smem,
+                                        (uint64_t)grid() * q.split, ctx->sm_count);
+            // without it, a few params are read as fast from global memory as they are staged
+            // (400,000 walkers, 14 params: 4.1 and 5.7 us, staged 4.8 and 6.5)
+            if (q.smem && !q.pdl && n_params <= 64) {
+                q.smem = 0;
+                load_plain(model, kPlainMove, 0);
+            }
+        }
         plain_launch(model, kPlainLogfn, params, n_params, plain_logfn_grid());
     }
 
@@ -867,7 +902,7 @@ struct bay_sampler {
         bay_stretch_params p = make_params(0, 0);
         void* args[] = {&p};
         const bool plain = model->form == BAY_FORM_PLAIN;
-        const uint32_t block = tcr ? 256 : plain ? model->cta / plain_split() : model->cta;
+        const uint32_t block = tcr ? 256 : plain ? model->cta / plain_move[0].split : model->cta;
         const unsigned g = (unsigned)(plain ? plain_logfn_grid() : (W + per_cta() - 1) / per_cta());
         const size_t sm = plain ? plain_smem(model, kPlainLogfn, params, n_params, g) : smem;
         CUkernel k = tcr ? model->k_tr[2] : plain ? model->plain[kPlainLogfn][sm != 0].k[0] : model->k_logfn;
@@ -1705,7 +1740,7 @@ static int sampler_create(bay_model* m, uint32_t seed, uint64_t walkers, const f
                 s->params = p;
                 s->own_params = true;
             }
-            if (m->form == BAY_FORM_PLAIN) s->load_plain_kernels();
+            if (m->form == BAY_FORM_PLAIN) s->plan_plain();
             if (s->streaming) {
                 const size_t Wn = walkers;
                 s->s_y = (float*)c->alloc(sizeof(float) * Wn * s->D);
