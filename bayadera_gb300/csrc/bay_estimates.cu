@@ -3,10 +3,10 @@
 // its bitonic ranks.  Used on a sampler's walkers and on data matrices alike.
 //
 // Every kernel reads x where it lies, once a pass, in the flat order: a CTA owns a tile of
-// dt = at most 256 dimensions and rp = 256 / dt rows a pass, thread t working for dimension
-// t % dt on row t / dt, so a warp's loads are consecutive words and a thread's dimension
-// never changes.  gx CTAs share a dimension tile's rows (about 4 CTAs an SM over the grid,
-// at least 32 elements a thread); their partial results go to the context's workspace and
+// dt dimensions (at most 64 for the sums and limits) and rp = 256 / dt rows a pass, thread t
+// working for dimension t % dt on row t / dt, so a warp's loads are consecutive words and a
+// thread's dimension never changes.  gx CTAs share a dimension tile's rows (about 4 CTAs an SM over the grid,
+// at least 16 elements a thread); their partial results go to the context's workspace and
 // the tile's last CTA (a ticket, reset for the next launch) combines them in CTA order, so
 // the result does not depend on which CTA that is.
 // The earlier kernels took a dimension-major copy of the matrix (a transpose per call, as
@@ -153,15 +153,14 @@ struct fp_sum {
     }
 };
 
+// The CTA's sums of its share of dimension p.dl, in `total` of every thread of that dimension:
+// MODE 0 of x, MODE 1 of (x - c)^2 and x - c.
 template <int MODE>
-__global__ void __launch_bounds__(kThreads)
-moments_pass(const float* __restrict__ x, uint32_t D, uint64_t W, uint32_t gx, uint32_t tile,
-             double* mean, double* var, double* part, uint32_t* tickets) {
-    __shared__ double red[kThreads];
-    const Place p = place_of(D, gx, tile);
-    double acc[MODE + 1] = {};     // MODE 0: sum x; MODE 1: sum (x - c)^2, sum (x - c)
+__device__ __forceinline__ void moments_share(const Place& p, const float* __restrict__ x, uint32_t D,
+                                              uint64_t W, float c, double* red,
+                                              double (&total)[MODE + 1]) {
+    double acc[MODE + 1] = {};
     if (p.on) {
-        const float c = MODE == 1 ? (float)mean[p.d0 + p.dl] : 0.0f;
         const float* col = x + p.d0 + p.dl;
         fp_sum f;
         uint32_t held = 0;
@@ -193,7 +192,6 @@ moments_pass(const float* __restrict__ x, uint32_t D, uint64_t W, uint32_t gx, u
         }
         f.flush<MODE>(acc);
     }
-    double total[MODE + 1];
 #pragma unroll
     for (int q = 0; q <= MODE; ++q) {
         red[threadIdx.x] = acc[q];
@@ -201,6 +199,23 @@ moments_pass(const float* __restrict__ x, uint32_t D, uint64_t W, uint32_t gx, u
         total[q] = red[p.dl];
         __syncthreads();
     }
+}
+
+__device__ __forceinline__ double variance_of(const double (&total)[2], uint64_t W) {
+    const double m = total[0] / (double)W, u = total[1] / (double)W;
+    const double v = m - u * u;
+    return v < 0.0 ? 0.0 : v;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kThreads)
+moments_pass(const float* __restrict__ x, uint32_t D, uint64_t W, uint32_t gx, uint32_t tile,
+             double* mean, double* var, double* part, uint32_t* tickets) {
+    __shared__ double red[kThreads];
+    const Place p = place_of(D, gx, tile);
+    const float c = MODE == 1 && p.on ? (float)mean[p.d0 + p.dl] : 0.0f;
+    double total[MODE + 1];
+    moments_share<MODE>(p, x, D, W, c, red, total);
     if (gx > 1) {
         double* mine = part + ((uint64_t)p.d0 + p.dl) * gx * (MODE + 1);   // [dim][CTA][sum]
         if (p.on && p.rl == 0)
@@ -226,15 +241,23 @@ moments_pass(const float* __restrict__ x, uint32_t D, uint64_t W, uint32_t gx, u
         }
     }
     if (p.on && p.rl == 0) {
-        const uint32_t d = p.d0 + p.dl;
-        const double m = total[0] / (double)W;
-        if (MODE == 0) {
-            mean[d] = m;
-        } else {
-            const double u = total[MODE] / (double)W;
-            const double v = m - u * u;
-            var[d] = v < 0.0 ? 0.0 : v;
-        }
+        if constexpr (MODE == 0) mean[p.d0 + p.dl] = total[0] / (double)W;
+        else var[p.d0 + p.dl] = variance_of(total, W);
+    }
+}
+
+// Both passes where a CTA has all rows of its dimensions.
+__global__ void __launch_bounds__(kThreads)
+moments_both(const float* __restrict__ x, uint32_t D, uint64_t W, uint32_t tile, double* mean, double* var) {
+    __shared__ double red[kThreads];
+    const Place p = place_of(D, 1u, tile);
+    double sum[1], sq[2];
+    moments_share<0>(p, x, D, W, 0.0f, red, sum);
+    const double mu = sum[0] / (double)W;
+    moments_share<1>(p, x, D, W, (float)mu, red, sq);
+    if (p.on && p.rl == 0) {
+        mean[p.d0 + p.dl] = mu;
+        var[p.d0 + p.dl] = variance_of(sq, W);
     }
 }
 
@@ -243,12 +266,13 @@ moments_pass(const float* __restrict__ x, uint32_t D, uint64_t W, uint32_t gx, u
 __global__ void __launch_bounds__(kThreads)
 limits_pass(const float* __restrict__ x, uint32_t D, uint64_t W, uint32_t gx, uint32_t tile,
             int zero_fold, float* limits, float2* part, uint32_t* tickets, uint32_t* counts,
-            uint64_t n_counts, uint32_t start) {
+            uint64_t n_counts, uint32_t start, uint32_t n_limits) {
     __shared__ float2 red[kThreads];
-    const Place p = place_of(D, gx, tile);
     for (uint64_t i = blockIdx.x * (uint64_t)kThreads + threadIdx.x; i < n_counts;
          i += (uint64_t)gridDim.x * kThreads)
         counts[i] = start;
+    if (blockIdx.x >= n_limits) return;      // there for the counts alone
+    const Place p = place_of(D, gx, tile);
     const float nan = __int_as_float(0x7fc00000);
     float mn = nan, mx = nan;
     if (p.on) {
@@ -379,6 +403,7 @@ __global__ void hist_finish(const uint32_t* counts, const float* limits, uint32_
 
 namespace bay {
 
+// tiles of at most tile_max dimensions, shares of at least rows_min rows
 est_plan est_plan_of(uint32_t D, uint64_t W, uint32_t tile_max, uint64_t rows_min) {
     est_plan p;
     uint32_t tile = tile_max < kThreads ? tile_max : kThreads;
@@ -387,29 +412,50 @@ est_plan est_plan_of(uint32_t D, uint64_t W, uint32_t tile_max, uint64_t rows_mi
     p.tile = (uint32_t)(((uint64_t)D + gy - 1) / gy);      // equal tiles
     p.gy = (uint32_t)(((uint64_t)D + p.tile - 1) / p.tile);
     const uint64_t rp = kThreads / p.tile;
-    uint64_t per = rp * 2 * kBatch;                        // rows a CTA has at least
+    uint64_t per = rp * kBatch;                            // rows a CTA has at least
     if (per < rows_min) per = rows_min;
-    uint64_t gx = (W + per - 1) / per;
-    // 4 CTAs an SM, but no more partial results than its last CTA adds up in some us (FP64
-    // issue: 8,192 of them take 2 us) unless that leaves SMs without a CTA
-    uint64_t most = p.gy >= kEstCtas ? 1 : kEstCtas / p.gy;
-    const uint64_t sums = 8192 / p.tile, one = kEstCtas / 4 / p.gy;
-    if (most > sums) most = sums > one ? sums : one;
-    if (most < 1) most = 1;
+    const uint64_t gx = (W + per - 1) / per;
+    const uint64_t most = p.gy >= kEstCtas ? 1 : kEstCtas / p.gy;   // 4 CTAs an SM
     p.gx = (uint32_t)(gx < most ? (gx < 1 ? 1 : gx) : most);
     return p;
 }
 
+// The moments' and limits' plan.  A CTA's last one of a tile adds up gx partial results a
+// dimension (FP64 issue: 2,048 of them take 0.6 us, and it is alone then), so with many CTAs the
+// tiles are as narrow as keeps gx * tile below that (8 dimensions, a 32-byte sector, to 64); with
+// few, so narrow that one CTA has all rows of its dimensions and no others to wait for.  Moments
+// of 4,096 x 256, 65,536 x 100 and 1,000 x 20 values on the device, in tiles of up to 256
+// dimensions 100, 102 and 51 us a call, now 53, 77 and 38.
+est_plan sums_plan_of(uint32_t D, uint64_t W) {
+    // CTAs, of a batch a thread at least
+    uint64_t n = W > (uint64_t)kEstCtas * kThreads * kBatch ? kEstCtas : W * D / (kThreads * kBatch) + 1;
+    if (n > kEstCtas) n = kEstCtas;
+    uint64_t tile = 8;
+    if (n <= kEstCtas / 4) {
+        tile = (D + n - 1) / n;
+        if (tile < 4) tile = 4;
+    } else {
+        while (tile < 64 && n * (tile + 8) * (tile + 8) <= 2048ull * D) tile += 8;
+    }
+    if (tile > 64) tile = 64;
+    return est_plan_of(D, W, (uint32_t)tile, 0);
+}
+
 size_t est_workspace(uint32_t D, uint64_t W) {
-    const est_plan p = est_plan_of(D, W, kThreads, 0);
+    const est_plan p = sums_plan_of(D, W);
     return kEstTickets * sizeof(uint32_t) + 2 * sizeof(double) * (size_t)p.gx * D;
 }
 
 cudaError_t launch_moments(const float* x, uint32_t D, uint64_t W, double* mean, double* var,
                            void* ws, cudaStream_t s) {
-    const est_plan p = est_plan_of(D, W, kThreads, 0);
+    const est_plan p = sums_plan_of(D, W);
     uint32_t* tickets = static_cast<uint32_t*>(ws);
     double* part = reinterpret_cast<double*>(tickets + kEstTickets);
+    if (var && p.gx == 1) {
+        moments_both<<<p.gy, kThreads, 0, s>>>(x, D, W, p.tile, mean, var);
+        count_launches(1);
+        return cudaGetLastError();
+    }
     moments_pass<0><<<p.gx * p.gy, kThreads, 0, s>>>(x, D, W, p.gx, p.tile, mean, var, part, tickets);
     count_launches(1);
     if (var) {
@@ -422,11 +468,15 @@ cudaError_t launch_moments(const float* x, uint32_t D, uint64_t W, double* mean,
 cudaError_t launch_limits(const float* x, uint32_t D, uint64_t W, int zero_fold, float* limits,
                           uint32_t* counts, uint64_t n_counts, uint32_t start, void* ws,
                           cudaStream_t s) {
-    const est_plan p = est_plan_of(D, W, kThreads, 0);
+    const est_plan p = sums_plan_of(D, W);
     uint32_t* tickets = static_cast<uint32_t*>(ws);
-    limits_pass<<<p.gx * p.gy, kThreads, 0, s>>>(x, D, W, p.gx, p.tile, zero_fold, limits,
-                                                 reinterpret_cast<float2*>(tickets + kEstTickets),
-                                                 tickets, counts, n_counts, start);
+    // 16 counts a thread at least, by CTAs of their own where the limits' are too few
+    uint64_t ctas = (n_counts + kThreads * 16 - 1) / (kThreads * 16);
+    if (ctas > kEstCtas) ctas = kEstCtas;
+    if (ctas < (uint64_t)p.gx * p.gy) ctas = (uint64_t)p.gx * p.gy;
+    limits_pass<<<(uint32_t)ctas, kThreads, 0, s>>>(x, D, W, p.gx, p.tile, zero_fold, limits,
+                                                    reinterpret_cast<float2*>(tickets + kEstTickets),
+                                                    tickets, counts, n_counts, start, p.gx * p.gy);
     count_launches(1);
     return cudaGetLastError();
 }

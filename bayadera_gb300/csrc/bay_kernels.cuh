@@ -113,7 +113,7 @@ cudaError_t launch_init_normal(float* xs, uint32_t D, uint64_t W, uint32_t seed,
 // device).
 cudaError_t launch_init_normal_members(float* xs, const bay_init_member* mem, uint32_t n,
                                        uint64_t count_max, float mean, float sd, cudaStream_t s);
-// How an estimate kernel is spread: equal tiles of at most 256 dimensions, gx CTAs a tile
+// How an estimate kernel is spread: equal tiles of dimensions, gx CTAs a tile
 // (kEstCtas CTAs at most unless the tiles alone are more).
 constexpr uint32_t kEstCtas = 608;        // 4 CTAs of 256 threads an SM
 constexpr uint32_t kEstTickets = 1024;    // one a tile wherever gx > 1
@@ -121,7 +121,6 @@ constexpr uint32_t kHistCounts = 12288;   // shared-memory counts of a histogram
 struct est_plan {
     uint32_t tile = 1, gy = 1, gx = 1, copies = 1;
 };
-est_plan est_plan_of(uint32_t D, uint64_t W, uint32_t tile_max, uint64_t rows_min);
 est_plan hist_plan_of(uint32_t D, uint64_t W, uint32_t bins);
 // Bytes of the estimate kernels' workspace: kEstTickets words, zero before the first use
 // and after every launch, then the CTAs' partial results.
