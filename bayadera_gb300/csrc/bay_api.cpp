@@ -260,8 +260,8 @@ struct bay_ctx {
     }
     void use() { cuda_check(cudaSetDevice(device), "cudaSetDevice"); }
 
-    // Workspace of the estimate kernels, kept between calls (at most 2.5 MB up to
-    // 155,648 dimensions, 16 bytes a dimension past that).  Every user runs on this context's
+    // Workspace of the estimate kernels, kept between calls (at most 0.7 MB up to
+    // 38,912 dimensions, 16 bytes a dimension past that).  Every user runs on this context's
     // stream under its lock; growing frees the old one, which waits for the device.
     void* est_ws = nullptr;
     size_t est_ws_bytes = 0;
@@ -371,6 +371,7 @@ std::vector<char> nvrtc_compile(const std::string& src, const std::vector<std::s
 bool nvrtc_compiled(const std::vector<std::string>& opts, const std::string& id);
 
 constexpr uint32_t kGemmWalkers = 64;             // BAY_WT in device/bay_stretch.cuh
+constexpr unsigned kGemmAccuThreads = 320;        // an accu CTA's: two warps more, for the statistics
 constexpr size_t kGemmMaxSmem = 200 * 1024;       // dynamic shared memory cap per CTA
 
 // Dynamic shared memory of the GEMM-form kernels for `rows` rows (layout in
@@ -672,6 +673,7 @@ struct bay_sampler {
     uint64_t gemm_base = 0, gemm_rows = 0;  // GEMM form: A's row 0 and row count in params
     uint32_t gemm_np = 0;                   // rows padded to a multiple of 64
     float* gemm_lay = nullptr;              // the kernel's layout of A and the aux values
+    bool gemm_pdl[2] = {true, true};        // SIMT form, bare and accu: not a loss (pdl_late)
     size_t smem = 0;                        // dynamic shared memory per CTA
 
     // A device-detected failure (a bounded wait that gave up) sets ctl->status.
@@ -841,7 +843,7 @@ struct bay_sampler {
         cfg.gridDimY = 1;
         cfg.gridDimZ = 1;
         cfg.blockDimX = tcr ? 256 * tr_g : model->cta / split;
-        if (accu && !tcr && model->form == BAY_FORM_GEMM) cfg.blockDimX += 64;   // statistics
+        if (accu && !tcr && model->form == BAY_FORM_GEMM) cfg.blockDimX = kGemmAccuThreads;
         cfg.blockDimY = 1;
         cfg.blockDimZ = 1;
         cfg.sharedMemBytes = (unsigned)(tcr || tiled ? smem_move
@@ -849,7 +851,9 @@ struct bay_sampler {
                                                 : smem);
         cfg.hStream = (CUstream)st;
         cfg.attrs = at;
-        cfg.numAttrs = pdl && !(plain && !plain_move[accu ? 1 : 0].pdl) ? 1 : 0;
+        const bool simt = !tcr && model->form == BAY_FORM_GEMM;
+        cfg.numAttrs = pdl && !(plain && !plain_move[accu ? 1 : 0].pdl) && !(simt && !gemm_pdl[accu ? 1 : 0])
+                           ? 1 : 0;
         if (accu && split > 1) {
             CUlaunchAttribute& cl = at[cfg.numAttrs++];
             cl.id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
@@ -1798,6 +1802,9 @@ static int sampler_create(bay_model* m, uint32_t seed, uint64_t walkers, const f
                            "gemm_tc_image");
             } else if (m->form == BAY_FORM_GEMM) {
                 s->gemm_np = (uint32_t)((s->gemm_rows + 63) & ~63ull);
+                for (int accu = 0; accu < 2; ++accu)
+                    s->gemm_pdl[accu] = !pdl_late(accu ? m->k_accu : m->k_bare, accu ? kGemmAccuThreads : 256,
+                                                  s->smem, s->grid(), c->sm_count);
                 const uint32_t auxs = m->gemm_aux_len ? m->gemm_aux_len : 1u;
                 s->gemm_lay = (float*)c->alloc(
                     sizeof(float) * ((size_t)m->gemm_features * s->gemm_np + (size_t)s->gemm_np * auxs));

@@ -306,6 +306,25 @@ __device__ void bay_accu_epilogue(const bay_stretch_params& P, bool accepted, bo
 #define BAY_TERM16 0
 #endif
 
+// Unrolling of the feature loop, and the registers of the launches (by the CTAs an SM that they
+// are to allow).  Unrolled whole a small loop takes up to 127 registers, which costs nothing while
+// an SM has one CTA and is a loss with more: 40,000 walkers of 20 dims 7.8 us a bare launch and
+// 12.2 accu unrolled by 20, now 6.3 and 8.3; 65,536 of 10 dims 8.0 and 9.9, now 6.3 and 8.4.  With
+// four CTAs of a bare launch an SM the longer loops are scheduled better too (12,288 walkers of 77
+// dims 10.8, now 9.5 us; 8,192 of 120 14.8, now 12.4).  Without a bound the accu launch of 25 to 64
+// features is faster (12,290 walkers of 37 dims 5.9 us, 6.2 with three).  By 5, 8, 10, 16 and 20,
+// over 20 sizes from 2 to 120 dims, 20 was the fastest above 24 features or within 1 % of it but for
+// 40 dims (16: 5.6 against 6.1 us before the bound).
+#define BAY_G_UNROLL (BAY_GEMM_F > 24 ? 20 : BAY_GEMM_F > 10 ? 10 : 8)
+#define BAY_G_BOUNDS __launch_bounds__(256, 4)
+#if BAY_GEMM_F <= 24
+#define BAY_G_BOUNDS_ACCU __launch_bounds__(320, 4)
+#elif BAY_GEMM_F <= 64
+#define BAY_G_BOUNDS_ACCU __launch_bounds__(320)
+#else
+#define BAY_G_BOUNDS_ACCU __launch_bounds__(320, 3)
+#endif
+
 // barriers of the eight warps that move a tile (accu launches have two more)
 __device__ __forceinline__ void bay_g_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 __device__ __forceinline__ bool bay_g_or(bool p) {
@@ -511,12 +530,7 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
         for (int i = 0; i < BAY_RW; ++i)
 #pragma unroll
             for (int j = 0; j < BAY_RN; ++j) acc[i][j] = 0.0f;
-        // bare launches of 12,290 walkers of 37, 16,384 of 48, 50, 64 and 80, 12,288 of 77 and 8,192
-        // of 120 dims: 6.2, 7.0, 6.9, 7.8, 12.0, 12.7 and 15.9 us unrolled by 5; 5.8, 7.0, 7.0, 7.7,
-        // 11.2, 10.9 and 15.8 by 10; 5.8, 6.4, 6.4, 7.7, 11.1, 10.9 and 14.7 by 20, at no size from
-        // 2 to 120 dims more than 0.6 % behind those, accu launches included (by 16: 40 dims 5.6
-        // against 6.1, 48 dims 7.2 against 6.4); 5.9 and 14.9 (37, 77) in full
-#pragma unroll 20
+#pragma unroll BAY_G_UNROLL
         for (int f = 0; f < BAY_GEMM_F; ++f) {
             const float4 y = *reinterpret_cast<const float4*>(&Ys[f * BAY_WT + w0]);
             const float4 a = *reinterpret_cast<const float4*>(&As[(size_t)f * NP + n0]);
@@ -586,10 +600,10 @@ __device__ __forceinline__ void bay_stretch_gemm(const bay_stretch_params& P) {
     if (ACCU && tid == 0 && n_acc) atomicAdd(&P.ctl->accepted, (unsigned long long)n_acc);
 }
 
-extern "C" __global__ void __launch_bounds__(256) bay_stretch_bare(bay_stretch_params P) {
+extern "C" __global__ void BAY_G_BOUNDS bay_stretch_bare(bay_stretch_params P) {
     bay_stretch_gemm<false, false>(P);
 }
-extern "C" __global__ void __launch_bounds__(320) bay_stretch_accu(bay_stretch_params P) {
+extern "C" __global__ void BAY_G_BOUNDS_ACCU bay_stretch_accu(bay_stretch_params P) {
     bay_stretch_gemm<true, false>(P);
 }
 // the statistics of the last half-step of a chunk (half P.half, step P.step_off)
