@@ -522,7 +522,40 @@ __device__ __forceinline__ void bay_batch_accept_impl(const bay_batch_params& P,
     const unsigned int nt = nk - T.k0 < BAY_BT_W ? nk - T.k0 : BAY_BT_W;
     const unsigned int nd = dim - T.n < BAY_BT_D ? dim - T.n : BAY_BT_D;
     const bool stats = MODE == 1 && P.means_cap != 0;
-    {
+    if (dim <= BAY_BT_D) {
+        // one slice: the tile's rows are one block, moved element by element so that every lane
+        // has one (5 coordinates on the lanes of a warp a walker: 4.6 us a bare launch of 500
+        // members of 64 walkers, 3.0 so)
+        float* __restrict__ Xt = P.xs + M.xs + ((size_t)P.half * M.K + T.k0) * dim;
+        const float* __restrict__ Yt = P.y + M.xs + (size_t)T.k0 * dim;
+        const float inv_dim = __frcp_rn((float)dim);
+        const unsigned int ne = nt * dim;
+        for (unsigned int e0 = tid; e0 < ne; e0 += 8u * BAY_BT_W) {
+            float v[8];
+            bool a[8];
+            unsigned int at[8];
+#pragma unroll
+            for (unsigned int i = 0; i < 8u; ++i) {
+                const unsigned int e = e0 + i * BAY_BT_W;
+                a[i] = false;
+                v[i] = 0.0f;
+                at[i] = 0u;
+                if (e < ne) {
+                    const unsigned int w = bay_div_dim(e, dim, inv_dim);
+                    at[i] = w * 33u + e - w * dim;
+                    a[i] = sAcc[w];
+                    if (a[i]) v[i] = Yt[e];
+                    else if (stats) v[i] = Xt[e];
+                }
+            }
+#pragma unroll
+            for (unsigned int i = 0; i < 8u; ++i) {
+                const unsigned int e = e0 + i * BAY_BT_W;
+                if (a[i]) Xt[e] = v[i];
+                if (stats && e < ne) bay_bsm[at[i]] = v[i];
+            }
+        }
+    } else {
         // lane: coordinate, warp: every 8th walker, 8 loads in flight
         float* __restrict__ Xt = P.xs + M.xs + ((size_t)P.half * M.K + T.k0) * dim + T.n;
         const float* __restrict__ Yt = P.y + M.xs + (size_t)T.k0 * dim + T.n;
