@@ -420,10 +420,13 @@ est_plan est_plan_of(uint32_t D, uint64_t W, uint32_t tile_max, uint64_t rows_mi
     return p;
 }
 
+constexpr uint64_t kAlone = 64 * kThreads;     // values that a CTA takes alone: 64 a thread
+
 // The moments' and limits' plan.  A CTA's last one of a tile adds up gx partial results a
 // dimension (FP64 issue: 2,048 of them take 0.6 us, and it is alone then), so with many CTAs the
 // tiles are as narrow as keeps gx * tile below that (8 dimensions, a 32-byte sector, to 64); with
-// few, so narrow that one CTA has all rows of its dimensions and no others to wait for.  Moments
+// few, so narrow that one CTA has all rows of its dimensions and no others to wait for, at up to
+// 64 values a thread.  Moments
 // of 4,096 x 256, 65,536 x 100 and 1,000 x 20 values on the device, in tiles of up to 256
 // dimensions 100, 102 and 51 us a call, now 53, 77 and 38.
 est_plan sums_plan_of(uint32_t D, uint64_t W) {
@@ -433,11 +436,11 @@ est_plan sums_plan_of(uint32_t D, uint64_t W) {
     uint64_t tile = 8;
     if (n <= kEstCtas / 4) {
         tile = (D + n - 1) / n;
-        if (tile < 4) tile = 4;
-    } else {
-        while (tile < 64 && n * (tile + 8) * (tile + 8) <= 2048ull * D) tile += 8;
+        if (tile > 64) tile = 64;
+        while (tile > 1 && W * tile > kAlone) tile = (tile + 1) / 2;
+        return est_plan_of(D, W, (uint32_t)tile, W * tile <= kAlone ? W : 0);
     }
-    if (tile > 64) tile = 64;
+    while (tile < 64 && n * (tile + 8) * (tile + 8) <= 2048ull * D) tile += 8;
     return est_plan_of(D, W, (uint32_t)tile, 0);
 }
 
