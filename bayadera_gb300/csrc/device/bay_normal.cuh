@@ -4,8 +4,8 @@
 // The init is defined by an FP64 formula rounded to fp32: x = mean + sd r cos(t) and
 // mean + sd r sin(t), r = sqrt(-2 log u1), t = 6.283185307179586 u0.  FP64 issue is 1/64 of
 // fp32 on this part and the pair takes some 95 FP64 operations.  Here r, cos and sin are
-// evaluated as unevaluated sums of two floats (about 2^-44 accurate; series from the
-// functions' definitions, exact sums and products after Knuth and Dekker), and the rounding
+// evaluated as unevaluated sums of two floats (r to about 2^-41, cos and sin to 2^-44; series from
+// the functions' definitions, exact sums and products after Knuth and Dekker), and the rounding
 // to fp32 is accepted where every value within the error bound rounds alike (Ziv's test);
 // where not, some 2^-14 of the elements, the caller takes the FP64 formula.  The results are
 // the FP64 formula's, bit for bit.

@@ -107,7 +107,13 @@ int bay_launch_count(uint64_t* out);
  * tiled 64 per CTA in one launch per half-step; larger matrices are streamed (128-walker
  * x 128-row register tiles, per-row-block partial sums; row index 32-bit, element
  * offsets 64-bit; features <= 384).  With BAY_MODEL_GEMM_TENSOR the streamed eta runs
- * on the tensor cores (split bf16, see the flag).  Covers Gaussian targets (A =
+ * on the tensor cores (split bf16, see the flag).  Beside its row term f a source may give
+ * that form the sum of 16 rows' terms,
+ *   REAL f_16(const REAL* eta, const REAL* aux, uint64_t row, const REAL* x,
+ *             const REAL* prep, REAL* carry);       rows row .. row + 15
+ *   void f_16_init(REAL* carry);  REAL f_16_end(const REAL* carry, REAL* lo);
+ * the macro f_16_carry being the number (1 or more) of values carried over a thread's rows,
+ * whose part of the sum f_16_end gives as hi + lo.  Covers Gaussian targets (A =
  * precision matrix, term = -eta_r x_r/2) and regression likelihoods (A = design matrix,
  * aux = response). */
 /* BAY_FORM_BATCH compiles a model family for bay_batch (many independent models advanced
